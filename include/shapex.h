@@ -57,9 +57,9 @@ typedef struct se_options {
     float viewpoint[3];    /* orientation viewpoint, src/NormalEstimation.hpp:318-319 */
     float eigengap_fp64;   /* relative eigengap (l1-l0)/l2 below which the 3x3
                               eigensolve is redone in FP64 on the GPU */
-    int32_t leaf_bucket;   /* kNN bucket size: subtrees of <= this many points are
-                              scanned directly, 32 at a time (1..128; 0 or the
-                              default: 96) */
+    int32_t leaf_bucket;   /* kNN leaf size: Morton subtrees of <= this many points,
+                              but at most 32, are scanned directly (1..128; 0 or
+                              the default: 96) */
     int32_t device;        /* CUDA device ordinal */
     void* stream;          /* cudaStream_t to use; NULL: the context creates one */
     int32_t seed_halo;     /* kNN: points offered on each side of a warp's 32 queries
@@ -255,8 +255,8 @@ SE_API int se_tune_batch(se_ctx* ctx, const float* x, const float* y, const floa
 /* Work counters of the last se_normals/se_knn/se_knn_self call (diagnostics). */
 typedef struct se_stats {
     int64_t fp64_solves;     /* queries whose eigensolve took the FP64 path */
-    int64_t nodes_visited;   /* search-hierarchy nodes visited, summed over warps */
-    int64_t buckets_scanned; /* point buckets streamed, summed over warps */
+    int64_t nodes_visited;   /* search-hierarchy nodes whose (up to 32) children were tested, summed over warps */
+    int64_t buckets_scanned; /* leaves scanned, summed over warps */
     int64_t candidates;      /* points that reached a query's bound, summed over queries */
     int64_t merge_steps;     /* candidate-buffer merge steps, summed over warps */
     int64_t inserts;         /* insertions into the k-best lists, summed over queries */

@@ -425,8 +425,8 @@ __global__ void __launch_bounds__(kDedupThreads) k_dedup(const uint64_t* buf0, c
 // integer semantics as the reference, so topology is bit-exact. Node 0 is
 // computed twice: with the reference's root range l = N-1 (:128-130) for the
 // exported arrays when root_compat is set, and with the full range for the
-// search hierarchy. Also records each leaf's parent and each node's range end
-// for the search hierarchy.
+// features of the learned radius. Also records each leaf's parent and each
+// node's range end for them.
 // ---------------------------------------------------------------------------
 struct KNode {
     int64_t j;
@@ -491,17 +491,12 @@ __global__ void __launch_bounds__(256) k_karras(const uint64_t* __restrict__ cod
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= N) return;
     const KNode f = karras_node(codes, i, N, code_bits, false);
-    // search hierarchy (full root range)
+    // full root range
     range_end[i] = (int32_t)f.j;
     if (f.hl) leaf_parent[f.gamma] = (int32_t)i; else sparent[f.gamma] = (int32_t)i;
     if (f.hr) leaf_parent[f.gamma + 1] = (int32_t)i; else sparent[f.gamma + 1] = (int32_t)i;
     KNode e = f;
-    if (i == 0) {
-        st->sroot_gamma = (int32_t)f.gamma;
-        st->sroot_hl = f.hl;
-        st->sroot_hr = f.hr;
-        if (root_compat) e = karras_node(codes, 0, N, code_bits, true);
-    }
+    if (i == 0 && root_compat) e = karras_node(codes, 0, N, code_bits, true);
     left_child[i] = (int32_t)e.gamma;
     prefix_n[i] = (uint8_t)e.dnode;
     hll[i] = e.hl;
@@ -525,152 +520,205 @@ __global__ void k_root_parent(const int32_t* __restrict__ left_child, int32_t* _
 }
 
 // ---------------------------------------------------------------------------
-// Search boxes: bottom-up over the full-range radix tree (Karras 2012 sec. 4:
-// second arrival at a node merges). Only nodes the kNN traversal visits need
-// an SNode: the root and every node of more than `bucket` points. A subtree
-// of at most `bucket` points is a bucket, read as a point range, so its inner
-// nodes get nothing. Thread i looks at node i: a bucket root (at most
-// `bucket` points, parent the root or larger) has its contiguous points
-// reduced to a box by the whole warp (coalesced loads, shuffles), and its
-// thread enters the merge protocol at the parent. Thread i also looks at
-// leaf i: a leaf whose parent is the root or larger than a bucket is a bucket
-// of one point and enters the merge at that parent. (An earlier version had
-// every leaf climb to its bucket root and one thread read each bucket's
-// points serially: 0.91 ms against 0.52 ms for this one on 13M unique points.)
+// Search hierarchy. Its leaves are the maximal Morton subtrees of at most M
+// points, in Morton order; 32 consecutive nodes form a node of the next
+// level, up to a top level of at most 32 nodes.
+//
+// k_leaves finds the leaves from the sorted codes alone. Point i starts a leaf
+// when the subtree that joins it to point i - 1 holds more than M points: when
+// some run of M + 1 points [a, a + M] across the gap shares at least the
+// prefix that codes i - 1 and i share. So with w(a) = the common prefix of
+// codes a and a + M, point i starts a leaf when the largest w(a) over a in
+// [i - M, i - 1] is at least the common prefix of codes i - 1 and i: a sliding
+// maximum in shared memory (doubling windows), one ballot per 32 codes, and a
+// decoupled look-back over the tiles' leaf counts. With k_boxes it takes
+// 0.294 ms on 13M codes (20M precision mix), where merging the boxes of a
+// binary tree bottom-up took 0.530 ms; it reads no radix tree, so batched
+// builds make none. M is at most 32, one point per lane of the scan: of the
+// layouts simulated on 400k-point clouds (fixed runs of 16, 32 and 64 points,
+// runs cut at the best prefix, subtrees of at most 32 and 96) subtrees of at
+// most 32 let a warp scan the fewest points, 420 on a scene (96: 770; fixed
+// runs of 32: 920).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_boxes(const float4* __restrict__ pts, const int32_t* __restrict__ left_child,
-                                               const uint8_t* __restrict__ hll, const uint8_t* __restrict__ hlr,
-                                               const int32_t* __restrict__ sparent,
-                                               const int32_t* __restrict__ leaf_parent,
-                                               const int32_t* __restrict__ range_end, uint32_t* __restrict__ visit,
-                                               float4* __restrict__ node_box, SNode* __restrict__ snodes, int bucket,
-                                               DevState* st) {
+__global__ void __launch_bounds__(kLeafThreads) k_leaves(const uint64_t* __restrict__ codes, int M,
+                                                         int32_t* __restrict__ leaf_start,
+                                                         uint32_t* __restrict__ lookback, DevState* st,
+                                                         int spin_limit) {
+    constexpr int kHalo = kLeafMax, kSpan = kLeafTile + 2 * kHalo;
+    constexpr int kCells = kLeafIpt * kLeafThreads / 32;  // 32-code steps of a tile
+    static_assert(kCells == 32, "one warp scans the steps' counts");
+    constexpr unsigned kFull = 0xffffffffu;
+    __shared__ uint64_t s_code[kSpan];   // codes [t0 - kHalo, t0 + kLeafTile + kHalo)
+    __shared__ int8_t s_w[2][kSpan];     // window maxima of w, ping-pong
+    __shared__ uint32_t s_cnt[kCells];
+    __shared__ uint32_t s_tile;
     const int64_t u = (int64_t)st->u;
-    if (u < 2) return;
-    const int64_t N = u - 1;  // internal nodes
-    const int lane = threadIdx.x & 31;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // a node index and a leaf index
-    auto size_of = [&](int64_t c) {
-        const int64_t e = range_end[c];
-        return (c > e ? c - e : e - c) + 1;
-    };
-    // (a) thread i as internal node i: a bucket root is a node of at most
-    // `bucket` points below the root whose parent is the root or larger
-    int64_t f = 0, l = 0, par = -1;
-    bool root = false;
-    if (i > 0 && i < N) {
-        const int64_t e = range_end[i];
-        f = min(i, e);
-        l = max(i, e);
-        if (l - f + 1 <= bucket) {
-            par = sparent[i];
-            if (par < 0 || par >= N) {
-                set_err(&st->err, ERRBIT_BOUNDS);
-            } else {
-                root = par == 0 || size_of(par) > bucket;
-            }
-        }
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) s_tile = atomicAdd(&st->tile_counter[kSortPasses + 2], 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const int64_t t0 = (int64_t)tile * kLeafTile;
+    if (t0 >= u) return;
+    for (int j = tid; j < kSpan; j += kLeafThreads) {
+        const int64_t i = t0 - kHalo + j;
+        s_code[j] = i >= 0 && i < u ? codes[i] : 0ull;
     }
-    // the warp reduces each of its bucket roots' contiguous points together
-    uint32_t roots = __ballot_sync(0xffffffffu, root);
-    while (roots) {
-        const int r = __ffs(roots) - 1;
-        roots &= roots - 1;
-        const int64_t rf = __shfl_sync(0xffffffffu, f, r), rl = __shfl_sync(0xffffffffu, l, r);
-        float lx = INFINITY, ly = INFINITY, lz = INFINITY, hx = -INFINITY, hy = -INFINITY, hz = -INFINITY;
-        for (int64_t q = rf + lane; q <= rl; q += 32) {
-            const float4 v = __ldg(pts + q);
-            lx = fminf(lx, v.x); ly = fminf(ly, v.y); lz = fminf(lz, v.z);
-            hx = fmaxf(hx, v.x); hy = fmaxf(hy, v.y); hz = fmaxf(hz, v.z);
-        }
+    __syncthreads();
+    for (int j = tid; j < kSpan; j += kLeafThreads) {
+        const int64_t a = t0 - kHalo + j;
+        s_w[0][j] = a >= 0 && j + M < kSpan && a + M < u ? (int8_t)__clzll((long long)(s_code[j] ^ s_code[j + M])) : -1;
+    }
+    __syncthreads();
+    int p = 1, cur = 0;  // s_w[cur][j] = the largest w over [j, j + p)
+    for (; 2 * p <= M; p *= 2, cur ^= 1) {
+        for (int j = tid; j < kSpan; j += kLeafThreads)
+            s_w[cur ^ 1][j] = j + p < kSpan ? max(s_w[cur][j], s_w[cur][j + p]) : s_w[cur][j];
+        __syncthreads();
+    }
+    uint32_t flags[kLeafIpt];
 #pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) {
-            lx = fminf(lx, __shfl_xor_sync(0xffffffffu, lx, o));
-            ly = fminf(ly, __shfl_xor_sync(0xffffffffu, ly, o));
-            lz = fminf(lz, __shfl_xor_sync(0xffffffffu, lz, o));
-            hx = fmaxf(hx, __shfl_xor_sync(0xffffffffu, hx, o));
-            hy = fmaxf(hy, __shfl_xor_sync(0xffffffffu, hy, o));
-            hz = fmaxf(hz, __shfl_xor_sync(0xffffffffu, hz, o));
+    for (int r = 0; r < kLeafIpt; ++r) {
+        const int e = r * kLeafThreads + tid, j = kHalo + e;
+        const int64_t i = t0 + e;
+        bool f = i < u;
+        if (f && i > 0) {
+            const int d = __clzll((long long)(s_code[j - 1] ^ s_code[j]));
+            f = max(s_w[cur][j - M], s_w[cur][j - p]) >= d;
         }
-        if (lane == r) {
-            node_box[2 * i] = make_float4(lx, ly, lz, 0.f);
-            node_box[2 * i + 1] = make_float4(hx, hy, hz, 0.f);
-        }
+        flags[r] = __ballot_sync(kFull, f);
+        if (lane == 0) s_cnt[r * (kLeafThreads / 32) + warp] = __popc(flags[r]);
     }
-    // (b) thread i as leaf i: a leaf whose parent is the root or larger than a
-    // bucket is a bucket of one point and enters the merge at that parent
-    int64_t leaf_start = -1;
-    if (i < u) {
-        const int64_t lp = leaf_parent[i];
-        if (lp < 0 || lp >= N) {
-            set_err(&st->err, ERRBIT_BOUNDS);
-        } else if (lp == 0 || size_of(lp) > bucket) {
-            leaf_start = lp;
-        }
-    }
-    // Merge protocol over the nodes the traversal visits (Karras 2012 sec. 4):
-    // the second arrival at a node builds its SNode from both children and
-    // goes on to the parent. Arrivals come from bucket roots and one-point
-    // buckets; each thread runs at most two climbs.
-#pragma unroll 1
-    for (int climb = 0; climb < 2; ++climb) {
-        int64_t node = climb == 0 ? (root ? par : -1) : leaf_start;
-        if (node < 0) continue;
-        int it = 0;
-        for (; it < 130; ++it) {
-            if (node < 0 || node >= N) {
-                set_err(&st->err, ERRBIT_BOUNDS);
-                break;
-            }
-            __threadfence();
-            if (atomicAdd(&visit[node], 1u) == 0) break;
-            __threadfence();
-            int64_t g;
-            bool l_leaf, r_leaf;
-            if (node == 0) {
-                g = st->sroot_gamma;
-                l_leaf = st->sroot_hl;
-                r_leaf = st->sroot_hr;
-            } else {
-                g = left_child[node];
-                l_leaf = hll[node];
-                r_leaf = hlr[node];
-            }
-            float4 lo[2], hi[2];
-            int32_t ref[2], cnt[2];
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                const int64_t ch = g + side;
-                const bool leaf = side ? r_leaf : l_leaf;
-                if (leaf) {
-                    const float4 q = pts[ch];
-                    lo[side] = q;
-                    hi[side] = q;
-                    ref[side] = (int32_t)ch;
-                    cnt[side] = 1;
-                } else {
-                    lo[side] = __ldcg(node_box + 2 * ch);
-                    hi[side] = __ldcg(node_box + 2 * ch + 1);
-                    const int64_t e = range_end[ch];
-                    const int64_t cf = min(ch, e), cl = max(ch, e);
-                    cnt[side] = (int32_t)(cl - cf + 1);
-                    ref[side] = cnt[side] <= bucket ? (int32_t)cf : (int32_t)ch;
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t c = s_cnt[lane];
+        const uint32_t inc = warp_incl_scan(c);
+        const uint32_t tot = __shfl_sync(kFull, inc, 31);
+        // look-back, 32 predecessors per step (as k_dedup)
+        uint32_t excl = 0;
+        if (tile == 0) {
+            if (lane == 0) st_relaxed(lookback, LB_PRE | tot);
+        } else {
+            if (lane == 0) st_relaxed(lookback + tile, LB_AGG | tot);
+            int64_t q0 = (int64_t)tile - 1;
+            int spins = 0;
+            for (;;) {
+                const int64_t q = q0 - lane;
+                const uint32_t v = q >= 0 ? ld_relaxed(lookback + q) : LB_PRE;
+                const uint32_t fl = v >> 30;
+                const uint32_t pre = __ballot_sync(kFull, fl == 2);
+                const uint32_t need = pre ? (((pre & (0u - pre)) << 1) - 1u) : kFull;
+                if (__ballot_sync(kFull, fl == 0) & need) {
+                    if (++spins > spin_limit) {
+                        if (lane == 0) set_err(&st->err, ERRBIT_LOOKBACK);
+                        break;
+                    }
+                    continue;
                 }
+                excl += __reduce_add_sync(kFull, ((need >> lane) & 1u) ? (v & LB_VAL) : 0u);
+                if (pre) break;
+                q0 -= 32;
             }
-            SNode sn;
-            sn.lo_l = make_float4(lo[0].x, lo[0].y, lo[0].z, __int_as_float(ref[0]));
-            sn.hi_l = make_float4(hi[0].x, hi[0].y, hi[0].z, __int_as_float(cnt[0]));
-            sn.lo_r = make_float4(lo[1].x, lo[1].y, lo[1].z, __int_as_float(ref[1]));
-            sn.hi_r = make_float4(hi[1].x, hi[1].y, hi[1].z, __int_as_float(cnt[1]));
-            snodes[node] = sn;
-            node_box[2 * node] =
-                make_float4(fminf(lo[0].x, lo[1].x), fminf(lo[0].y, lo[1].y), fminf(lo[0].z, lo[1].z), 0.f);
-            node_box[2 * node + 1] =
-                make_float4(fmaxf(hi[0].x, hi[1].x), fmaxf(hi[0].y, hi[1].y), fmaxf(hi[0].z, hi[1].z), 0.f);
-            if (node == 0) break;
-            node = sparent[node];
+            if (lane == 0) st_relaxed(lookback + tile, LB_PRE | (excl + tot));
         }
-        if (it == 130) set_err(&st->err, ERRBIT_BOUNDS);
+        s_cnt[lane] = excl + inc - c;
+        if (lane == 0 && t0 + kLeafTile >= u) {
+            uint32_t n = excl + tot, off = 0;
+            int l = 0;
+            for (;; ++l) {
+                st->level_off[l] = off;
+                st->level_count[l] = n;
+                if (n <= kFan || l == kMaxLevels - 1) break;
+                off += n;
+                n = (n + kFan - 1) / kFan;
+            }
+            st->top_level = l;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kLeafIpt; ++r) {
+        if (!((flags[r] >> lane) & 1u)) continue;
+        const uint32_t pos = s_cnt[r * (kLeafThreads / 32) + warp] + __popc(flags[r] & lanemask_lt());
+        const int64_t i = t0 + r * kLeafThreads + tid;
+        if ((int64_t)pos < u) leaf_start[pos] = (int32_t)i;
+        else set_err(&st->err, ERRBIT_BOUNDS);
+    }
+}
+
+__device__ __forceinline__ float warp_min_f(float v) {
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max_f(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// Boxes of the hierarchy, bottom up: a warp takes 32 consecutive leaves (one
+// per lane, whose points follow one another, so the lanes' 16-byte loads share
+// cache lines) and reduces their boxes to the level-1 node's; the warp whose
+// node completes a group of 32 siblings (an arrival counter per parent) goes
+// on with the parent.
+__global__ void __launch_bounds__(128) k_boxes(const float4* __restrict__ pts, const int32_t* __restrict__ leaf_start,
+                                               uint32_t* __restrict__ arrivals, SNode* __restrict__ snodes,
+                                               DevState* st) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int64_t u = (int64_t)st->u;
+    const uint32_t nl = u > 0 && !(st->err & ERRBIT_LOOKBACK) ? st->level_count[0] : 0u;
+    const int lane = threadIdx.x & 31;
+    const int top = st->top_level;
+    const uint32_t groups = (nl + 31) / 32;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < groups; g += warps) {
+        const uint32_t leaf = g * 32 + lane;
+        float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+        if (leaf < nl) {
+            const int32_t f = leaf_start[leaf], e = leaf + 1 < nl ? leaf_start[leaf + 1] : (int32_t)u;
+            const int32_t cnt = e - f;
+            if (f < 0 || cnt < 1 || cnt > kLeafMax || e > u) {
+                set_err(&st->err, ERRBIT_BOUNDS);
+            } else {
+#pragma unroll 4
+                for (int32_t q = f; q < e; ++q) {
+                    const float4 v = __ldg(pts + q);
+                    lo.x = fminf(lo.x, v.x); lo.y = fminf(lo.y, v.y); lo.z = fminf(lo.z, v.z);
+                    hi.x = fmaxf(hi.x, v.x); hi.y = fmaxf(hi.y, v.y); hi.z = fmaxf(hi.z, v.z);
+                }
+                lo.w = __int_as_float(f);
+                hi.w = __int_as_float(cnt);
+                snodes[leaf].lo = lo;
+                snodes[leaf].hi = hi;
+            }
+        }
+        uint32_t node = g;
+        for (int l = 1; l <= top; ++l) {
+            lo = make_float4(warp_min_f(lo.x), warp_min_f(lo.y), warp_min_f(lo.z), 0.f);
+            hi = make_float4(warp_max_f(hi.x), warp_max_f(hi.y), warp_max_f(hi.z), 0.f);
+            SNode* mine = snodes + st->level_off[l] + node;
+            if (lane == 0) {
+                mine->lo = lo;
+                mine->hi = hi;
+            }
+            if (l == top) break;
+            // the parent's other children may be other warps': the last to arrive reduces them all
+            const uint32_t parent = node / kFan, first = parent * kFan;
+            const uint32_t kids = min((uint32_t)kFan, st->level_count[l] - first);
+            uint32_t seen = 0;
+            __threadfence();
+            if (lane == 0) seen = atomicAdd(arrivals + (st->level_off[l + 1] - st->level_off[2]) + parent, 1u);
+            seen = __shfl_sync(kFull, seen, 0);
+            if (seen + 1 != kids) break;
+            __threadfence();
+            lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+            hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+            if (lane < kids) {
+                lo = __ldcg(&snodes[st->level_off[l] + first + lane].lo);
+                hi = __ldcg(&snodes[st->level_off[l] + first + lane].hi);
+            }
+            node = parent;
+        }
     }
 }
 
@@ -1010,23 +1058,27 @@ cudaError_t enqueue_build(const BuildBufs& b, const BuildParams& p, cudaStream_t
                                                          b.lookback, b.st, p.spin_limit);
     ++nl;
     mark(4);
-    cudaMemsetAsync(b.parent, 0, sizeof(int32_t) * n, s);
-    cudaMemsetAsync(b.visit, 0, sizeof(uint32_t) * n, s);
-    cudaMemsetAsync(b.sparent, 0xff, sizeof(int32_t) * n, s);
-    cudaMemsetAsync(b.leaf_parent, 0xff, sizeof(int32_t) * n, s);
-    k_karras<<<grid_for(n, 256, 0), 256, 0, s>>>(b.codes, p.code_bits, p.root_compat, b.left_child, b.parent,
-                                                 b.prefix_n, b.has_leaf_left, b.has_leaf_right, b.sparent,
-                                                 b.leaf_parent, b.range_end, b.st);
-    ++nl;
-    if (p.root_compat) {
-        k_root_parent<<<1, 1, 0, s>>>(b.left_child, b.parent, b.has_leaf_left, b.has_leaf_right, b.st);
+    if (p.build_radix) {
+        cudaMemsetAsync(b.parent, 0, sizeof(int32_t) * n, s);
+        cudaMemsetAsync(b.sparent, 0xff, sizeof(int32_t) * n, s);
+        cudaMemsetAsync(b.leaf_parent, 0xff, sizeof(int32_t) * n, s);
+        k_karras<<<grid_for(n, 256, 0), 256, 0, s>>>(b.codes, p.code_bits, p.root_compat, b.left_child, b.parent,
+                                                     b.prefix_n, b.has_leaf_left, b.has_leaf_right, b.sparent,
+                                                     b.leaf_parent, b.range_end, b.st);
         ++nl;
+        if (p.root_compat) {
+            k_root_parent<<<1, 1, 0, s>>>(b.left_child, b.parent, b.has_leaf_left, b.has_leaf_right, b.st);
+            ++nl;
+        }
     }
     mark(5);
-    k_boxes<<<grid_for(n, 256, 0), 256, 0, s>>>(b.pts4, b.left_child, b.has_leaf_left, b.has_leaf_right, b.sparent,
-                                                b.leaf_parent, b.range_end, b.visit, b.node_box, b.snodes, p.bucket,
-                                                b.st);
-    ++nl;
+    const int64_t leaf_tiles = (n + kLeafTile - 1) / kLeafTile;
+    cudaMemsetAsync(b.lookback, 0, sizeof(uint32_t) * leaf_tiles, s);
+    cudaMemsetAsync(b.arrivals, 0, sizeof(uint32_t) * arrival_words(n), s);
+    k_leaves<<<(unsigned)leaf_tiles, kLeafThreads, 0, s>>>(b.codes, p.bucket < kLeafMax ? p.bucket : kLeafMax,
+                                                           b.leaf_start, b.lookback, b.st, p.spin_limit);
+    k_boxes<<<grid_for(n, 32 * 128, num_sms * 8), 128, 0, s>>>(b.pts4, b.leaf_start, b.arrivals, b.snodes, b.st);
+    nl += 2;
     mark(6);
     if (p.build_octree) {
         cudaError_t e = enqueue_octree(b, p, s, num_sms, &nl);

@@ -66,7 +66,7 @@ void free_build(se_ctx* c) {
     BuildBufs& b = c->b;
     void* ptrs[] = {b.keys0,     b.keys1,     b.lookback,    b.lookback64, b.codes,     b.pts4,
                     b.pts3,      b.left_child, b.parent,     b.prefix_n,   b.has_leaf_left, b.has_leaf_right,
-                    b.sparent,   b.leaf_parent, b.range_end, b.visit,      b.node_box,  b.snodes,
+                    b.sparent,   b.leaf_parent, b.range_end, b.leaf_start, b.arrivals,  b.snodes,
                     b.oct_counts, b.oct_offsets, c->in_xyz};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -106,9 +106,9 @@ int ensure_build_capacity(se_ctx* c, int64_t n) {
     SE_CUDA(c, regrow(b.sparent, cap), "alloc search");
     SE_CUDA(c, regrow(b.leaf_parent, cap), "alloc search");
     SE_CUDA(c, regrow(b.range_end, cap), "alloc search");
-    SE_CUDA(c, regrow(b.visit, cap), "alloc search");
-    SE_CUDA(c, regrow(b.node_box, 2 * cap), "alloc search");
-    SE_CUDA(c, regrow(b.snodes, cap), "alloc search");
+    SE_CUDA(c, regrow(b.leaf_start, cap), "alloc search");
+    SE_CUDA(c, regrow(b.arrivals, arrival_words(cap)), "alloc search");
+    SE_CUDA(c, regrow(b.snodes, hierarchy_nodes(cap)), "alloc search");
     SE_CUDA(c, regrow(b.oct_counts, cap), "alloc octree");
     SE_CUDA(c, regrow(b.oct_offsets, cap + 1), "alloc octree");
     SE_CUDA(c, regrow(c->in_xyz, 3 * cap), "alloc staging");
@@ -161,7 +161,6 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
     q.vz = c->opt.viewpoint[2];
     q.eigengap_fp64 = c->opt.eigengap_fp64;
     q.code_bits = c->opt.code_bits;
-    q.bucket = c->opt.leaf_bucket;
     q.seed_halo = seed_halo_for(c, k);
     q.compat = c->opt.search_compat ? 1 : 0;
     q.n_octree = c->info.n_octree;
@@ -409,9 +408,8 @@ int se_destroy(se_ctx* c) {
     if (c->lut_buf) cudaFree(c->lut_buf);
     for (BatchLane& l : c->lanes) {
         if (l.stream) cudaStreamSynchronize(l.stream);
-        void* ptrs[] = {l.b.keys0, l.b.keys1, l.b.lookback, l.b.lookback64, l.b.codes, l.b.pts4, l.b.pts3,
-                        l.b.left_child, l.b.parent, l.b.prefix_n, l.b.has_leaf_left, l.b.has_leaf_right, l.b.sparent,
-                        l.b.leaf_parent, l.b.range_end, l.b.visit, l.b.node_box, l.b.snodes, l.b.st};
+        void* ptrs[] = {l.b.keys0, l.b.keys1,      l.b.lookback, l.b.codes,
+                        l.b.pts3,  l.b.leaf_start, l.b.arrivals, l.b.st};
         for (void* p : ptrs)
             if (p) cudaFree(p);
         if (l.done) cudaEventDestroy(l.done);

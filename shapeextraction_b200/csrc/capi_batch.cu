@@ -34,23 +34,13 @@ int lane_capacity(se_ctx* c, BatchLane& l, int64_t n) {
     BuildBufs& b = l.b;
     const int64_t cap = n < 1024 ? 1024 : n;
     const int64_t sort_tiles = (cap + kSortTile - 1) / kSortTile;
-    const int64_t scan_tiles = (cap + kScanTile - 1) / kScanTile;
     SE_CUDA(c, regrow(b.keys0, cap), "alloc lane");
     SE_CUDA(c, regrow(b.keys1, cap), "alloc lane");
     SE_CUDA(c, regrow(b.lookback, sort_tiles * kSortBins + 64), "alloc lane");
-    SE_CUDA(c, regrow(b.lookback64, scan_tiles + 64), "alloc lane");
     SE_CUDA(c, regrow(b.codes, cap), "alloc lane");
     SE_CUDA(c, regrow(b.pts3, 3 * cap), "alloc lane");
-    SE_CUDA(c, regrow(b.left_child, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.parent, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.prefix_n, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.has_leaf_left, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.has_leaf_right, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.sparent, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.leaf_parent, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.range_end, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.visit, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.node_box, 2 * cap), "alloc lane");
+    SE_CUDA(c, regrow(b.leaf_start, cap), "alloc lane");
+    SE_CUDA(c, regrow(b.arrivals, arrival_words(cap)), "alloc lane");
     b.cap = cap;
     l.cap = cap;
     return SE_OK;
@@ -63,6 +53,7 @@ namespace {
 // What one se_normals_batch call enqueues: per-lane build queues, k groups.
 struct BatchPlan {
     int n_lanes = 0;
+    std::vector<int64_t> node_off;  // each cloud's slice of the search hierarchies (+ end)
     std::vector<std::vector<int>> queue;  // clouds per lane: group by group, largest first in each
     std::vector<std::vector<int>> group_end;  // per lane: end of each group's run in `queue`
     std::vector<char> lane_query;         // per cloud: queried on its lane right after its build
@@ -132,9 +123,9 @@ int enqueue_batch(se_ctx* c, const BatchPlan& plan, const BatchCloud* d_desc, co
             b.y = by + off;
             b.z = bz + off;
             b.pts4 = c->batch_pts4 + off;
-            b.snodes = c->batch_snodes + off;
+            b.snodes = c->batch_snodes + plan.node_off[ci];
             b.st = c->batch_st + ci;
-            BuildParams p{n, c->opt.code_bits, 0, 0, c->opt.leaf_bucket};
+            BuildParams p{n, c->opt.code_bits, 0, 0, c->opt.leaf_bucket, 0};
             int nl = 0;
             SE_CUDA(c, enqueue_build(b, p, lane.stream, c->num_sms, nullptr, &nl), "launch batch build");
             launches += nl;
@@ -150,7 +141,6 @@ int enqueue_batch(se_ctx* c, const BatchPlan& plan, const BatchCloud* d_desc, co
                 q.vz = c->opt.viewpoint[2];
                 q.eigengap_fp64 = c->opt.eigengap_fp64;
                 q.code_bits = c->opt.code_bits;
-                q.bucket = c->opt.leaf_bucket;
                 q.seed_halo = seed_halo_for(c, q.k);
                 SE_CUDA(c, enqueue_query(b, q, lane.stream, c->num_sms), "launch batch query");
                 ++launches;
@@ -169,7 +159,6 @@ int enqueue_batch(se_ctx* c, const BatchPlan& plan, const BatchCloud* d_desc, co
         q.vz = c->opt.viewpoint[2];
         q.eigengap_fp64 = c->opt.eigengap_fp64;
         q.code_bits = c->opt.code_bits;
-        q.bucket = c->opt.leaf_bucket;
         q.seed_halo = seed_halo_for(c, q.k);
         q.batch_blocks_per_sm = c->opt.batch_blocks_per_sm;
         q.batch_warps_per_block = c->opt.batch_warps_per_block;
@@ -246,10 +235,17 @@ int se_normals_batch(se_ctx* c, const float* x, const float* y, const float* z, 
     if (!c->batch_ev_in) SE_CUDA(c, cudaEventCreateWithFlags(&c->batch_ev_in, cudaEventDisableTiming), "event");
     if (!c->batch_ev_out) SE_CUDA(c, cudaEventCreateWithFlags(&c->batch_ev_out, cudaEventDisableTiming), "event");
     if (!c->graph_stream) SE_CUDA(c, cudaStreamCreateWithFlags(&c->graph_stream, cudaStreamNonBlocking), "stream");
+    BatchPlan plan;
+    plan.node_off.assign(n_clouds + 1, 0);
+    for (int i = 0; i < n_clouds; ++i)
+        plan.node_off[i + 1] = plan.node_off[i] + hierarchy_nodes(offsets[i + 1] - offsets[i]);
     if (c->batch_pts_cap < total) {
         if (int rc = grow_batch(c, c->batch_pts4, total, "alloc batch points")) return rc;
-        if (int rc = grow_batch(c, c->batch_snodes, total, "alloc batch hierarchy")) return rc;
         c->batch_pts_cap = total;
+    }
+    if (c->batch_nodes_cap < plan.node_off[n_clouds]) {
+        if (int rc = grow_batch(c, c->batch_snodes, plan.node_off[n_clouds], "alloc batch hierarchy")) return rc;
+        c->batch_nodes_cap = plan.node_off[n_clouds];
     }
     if (host && total > 0 && c->batch_cap < total) {
         if (int rc = grow_batch(c, c->batch_in, 3 * total, "alloc batch staging")) return rc;
@@ -266,7 +262,6 @@ int se_normals_batch(se_ctx* c, const float* x, const float* y, const float* z, 
     // the small ones group by group; largest cloud first, each to the lane
     // with the least queued work.
     const int64_t kLaneQueryMin = batch_lane_min(c);
-    BatchPlan plan;
     plan.lane_query.assign(n_clouds, 0);
     plan.n_lanes = std::min(n_clouds, batch_lanes(c));
     if ((int)c->lanes.size() < plan.n_lanes) c->lanes.resize(plan.n_lanes);
@@ -335,7 +330,7 @@ int se_normals_batch(se_ctx* c, const float* x, const float* y, const float* z, 
         for (int ci : order) {
             const int64_t off = offsets[ci], n = offsets[ci + 1] - offsets[ci];
             if (n == 0 || ks[ci] != k || plan.lane_query[ci]) continue;
-            desc.push_back(BatchCloud{c->batch_pts4 + off, c->batch_snodes + off, c->batch_st + ci, bout + 3 * off, items});
+            desc.push_back(BatchCloud{c->batch_pts4 + off, c->batch_snodes + plan.node_off[ci], c->batch_st + ci, bout + 3 * off, items});
             items += (n + 31) / 32;
         }
         plan.group_items.push_back(items);

@@ -99,6 +99,7 @@ struct se_ctx {
     float4* batch_pts4 = nullptr;
     SNode* batch_snodes = nullptr;
     int64_t batch_pts_cap = 0;
+    int64_t batch_nodes_cap = 0;
     DevState* batch_st = nullptr;
     BatchCloud* batch_desc = nullptr;    // per k group, clouds largest first
     BatchCloud* h_batch_desc = nullptr;  // pinned host copy

@@ -12,9 +12,9 @@
 // coherent); lane i owns query i. Each lane keeps its k best (squared
 // distance, index) keys as a sorted list in registers, whose last entry is
 // the lane's pruning bound. The warp first offers the Morton window around its
-// queries, then walks the search hierarchy depth first with a shared stack: a
-// child is entered when any lane's bound reaches its box, nearer child first
-// by lane vote. Bucket points (contiguous runs of at most `bucket` points) are
+// queries, then walks the search hierarchy: 32 nodes are tested at once
+// against the box of the warp's queries, nearest first, and each that passes
+// by all 32 queries. Leaf points (contiguous runs of at most 32 points) are
 // staged in shared memory and read by broadcast. A point that reaches a lane's
 // bound goes to that lane's candidate buffer; buffers are merged into the
 // lists in batches, so that the warp pays for one list update per buffered
@@ -33,7 +33,6 @@ namespace shapex {
 
 namespace {
 
-constexpr int kStackDepth = 96;
 // Per-k tile shape, measured on B200 (2M scene and 5M mixture clouds): small
 // lists leave registers for more resident warps, which pays for itself up to
 // k = 16. The 24- and 32-key lists need more registers, so they keep the
@@ -188,14 +187,20 @@ struct TopK {
     }
 };
 
-// Per-warp shared scratch: traversal stack, staged points, candidate buffers
-// ([slot][lane] so that a warp's accesses to one slot fall in distinct banks).
+// Per-warp shared scratch: staged points (the seed window, then one leaf in
+// its first 32 entries), candidate buffers ([slot][lane] so that a warp's
+// accesses to one slot fall in distinct banks). While the warp walks the
+// hierarchy, entries [64, 104) of pts hold the order keys of the levels above
+// the current one.
 template <int B>
 struct WarpSmem {
-    int32_t stack[kStackDepth];
     float4 pts[kWindowMax];
     int32_t buf[B][32];
+    __device__ __forceinline__ uint32_t* level_keys(int l) {  // l >= 1
+        return reinterpret_cast<uint32_t*>(&pts[64]) + 32 * (l - 1);
+    }
 };
+static_assert(64 + (kMaxLevels - 1) * 8 <= kWindowMax, "order keys fit behind the staged leaf");
 
 // Ordered widest first so that the struct packs into 128 bytes: one more
 // padded word (144 bytes) made ptxas give the k = 32 kernels 161-163
@@ -212,7 +217,6 @@ struct QArgs {
     float gap;
     int k;
     int code_bits;
-    int bucket;
     int seed_halo;
     int learned_skip_seed;
     int device_count;  // 1: u = count = the build's unique-point count, read on the device (start 0)
@@ -221,7 +225,7 @@ struct QArgs {
     int cell_pmax;     // cell scan: most points per warp before it falls back to the walk
     int cell_span;     // cell scan: most cells per axis covering one lane's ball (2..4)
 };
-static_assert(sizeof(QArgs) == 128, "QArgs grew past 128 bytes");
+static_assert(sizeof(QArgs) <= 128, "QArgs grew past 128 bytes");
 
 struct Counters {
     int cand = 0, ins = 0, merge = 0, buckets = 0, lmiss = 0, cells = 0, cell_fallback = 0, cell_lookups = 0,
@@ -406,7 +410,7 @@ __device__ __forceinline__ void ball_box(uint64_t code, float r2, uint32_t M, fl
     }
 }
 
-constexpr int kCellBits = 1024;   // cells of a warp's union grid: one bit each, in stack[0, 32)
+constexpr int kCellBits = 1024;   // cells of a warp's union grid: one bit each, in pts[112, 120)
 constexpr int kCellRanges = 64;   // nonempty cells a warp scans: listed in pts[32, 96), order keys after
 
 // Learned attempt as a direct scan of Morton cells, with no tree walk.
@@ -470,7 +474,7 @@ __device__ __forceinline__ bool cell_scan(TopK<K, EXACT>& tk, int& bc, WS& W, in
         ++s;
     }
     // mark the union of the lanes' cells
-    uint32_t* bits = reinterpret_cast<uint32_t*>(W.stack);  // words [0, 32); inclusive prefixes at [32, 64)
+    uint32_t* bits = reinterpret_cast<uint32_t*>(&W.pts[112]);  // words [0, 32); inclusive prefixes at [32, 64)
     __syncwarp();
     bits[lane] = 0u;
     __syncwarp();
@@ -705,6 +709,131 @@ __device__ __forceinline__ void estimate_normal(const int32_t* nbr, int k, const
     out[2] = nz;
 }
 
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// Walk of the search hierarchy for the warp's active lanes, depth first,
+// nearest node first. The 32 children of a node are tested at once, one per
+// lane, against the box of the warp's queries (its distance to a child's box
+// never exceeds that of any query in it, by the same rounding chain); a child
+// within the largest bound of the warp is then tested by every lane against
+// its own query and bound. The first test is one pass for 32 nodes where a
+// binary tree took a visit for every two; the second keeps warps whose queries
+// lie far apart (their box covers what is between) from descending everywhere.
+// A lane's order key is its child's distance with the lane in the low 5 bits
+// (rounded down, so still a lower bound); keys of the levels above wait in
+// shared memory.
+template <int K, bool EXACT, class WS>
+__device__ __forceinline__ void walk(TopK<K, EXACT>& tk, int& bc, WS& W, int lane, Counters& ct,
+                                     const float4* __restrict__ pts, const SNode* __restrict__ snodes, const QArgs& a,
+                                     DevState* st, bool act, float qx, float qy, float qz, float cap, int64_t u,
+                                     int64_t sw0, int64_t sw1, uint32_t& steps) {
+    constexpr int kBuf = KnnCfg<K>::buf;
+    constexpr uint32_t kNone = 0xffffffffu;
+    // Siblings that pass the first test before each is tested by all 32 queries
+    // at once. Most warps pass a few of 32; a warp across a Morton jump passes
+    // nearly all, and a visit for each makes it the last to end: the 100k-point
+    // k = 8 search took 237 us without this test, 168 us with it (24), 176 us at
+    // 12. Large clouds, where other warps fill in, pay for it sooner: the 20M
+    // precision mix 17.89 ms without, 18.04 at 24, 18.52 at 12.
+    constexpr int kMaxLoose = 24;
+    // the box of the active queries
+    const float lx = warp_min(act ? qx : INFINITY), hx = warp_max(act ? qx : -INFINITY);
+    const float ly = warp_min(act ? qy : INFINITY), hy = warp_max(act ? qy : -INFINITY);
+    const float lz = warp_min(act ? qz : INFINITY), hz = warp_max(act ? qz : -INFINITY);
+    const uint32_t step_cap = a.step_limit > 0 ? (uint32_t)a.step_limit : (uint32_t)min64(4 * u + 64, 0x7fffffff);
+    float tau = act ? fminf(tk.tau(), cap) : -1.0f;
+    float tau_max = warp_max(tau);
+    int l = __ldg(&st->top_level);
+    const int top = l;
+    uint32_t first = 0;                                       // the current siblings: [first, first + 32) of level l,
+    const SNode* group = snodes + __ldg(&st->level_off[l]);   // from here on
+    // order key of the lane's sibling
+    auto order_key = [&]() -> uint32_t {
+        const bool valid = first + lane < __ldg(&st->level_count[l]);
+        const SNode* n = group + (valid ? lane : 0);
+        const float4 lo = __ldg(&n->lo), hi = __ldg(&n->hi);
+        const float gx = fmaxf(fmaxf(__fsub_rn(lo.x, hx), __fsub_rn(lx, hi.x)), 0.0f);
+        const float gy = fmaxf(fmaxf(__fsub_rn(lo.y, hy), __fsub_rn(ly, hi.y)), 0.0f);
+        const float gz = fmaxf(fmaxf(__fsub_rn(lo.z, hz), __fsub_rn(lz, hi.z)), 0.0f);
+        float d = __fmaf_rn(gx, gx, __fmaf_rn(gy, gy, __fmul_rn(gz, gz)));
+        bool reach = valid && d <= tau_max;
+        if (__popc(__ballot_sync(FULL, reach)) > kMaxLoose) {
+            // the box of the queries may hold much that no query is near:
+            // take the distance of the nearest query that reaches the child
+            d = INFINITY;
+            reach = false;
+#pragma unroll 1
+            for (int i = 0; i < 32; ++i) {
+                const float xi = __shfl_sync(FULL, qx, i), yi = __shfl_sync(FULL, qy, i), zi = __shfl_sync(FULL, qz, i);
+                const float ti = __shfl_sync(FULL, tau, i);
+                const float di = box_dist2(xi, yi, zi, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z);
+                if (di <= ti) {
+                    d = fminf(d, di);
+                    reach = valid;
+                }
+            }
+        }
+        return reach ? (__float_as_uint(d) & ~31u) | (uint32_t)lane : kNone;
+    };
+    uint32_t key = order_key();
+    ++steps;
+    for (;;) {
+        const uint32_t m = __reduce_min_sync(FULL, key);
+        if (m == kNone || __uint_as_float(m & ~31u) > tau_max) {  // nothing left here: up a level
+            if (l == top) break;
+            ++l;
+            first = (first / kFan) & ~31u;
+            group = snodes + __ldg(&st->level_off[l]) + first;
+            key = W.level_keys(l)[lane];
+            continue;
+        }
+        if (key == m) key = kNone;
+        const float4 lo = __ldg(&group[m & 31u].lo), hi = __ldg(&group[m & 31u].hi);
+        const float d = box_dist2(qx, qy, qz, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z);
+        const bool need = d <= tau;
+        const uint32_t needm = __ballot_sync(FULL, need);
+        if (!needm) continue;
+        if (l > 0) {
+            if (++steps > step_cap) {
+                if (lane == 0) set_err(&st->err, ERRBIT_SEARCH_LIMIT);
+                break;
+            }
+            W.level_keys(l)[lane] = key;
+            --l;
+            first = (first + (m & 31u)) * kFan;
+            group = snodes + __ldg(&st->level_off[l]) + first;
+            key = order_key();
+            continue;
+        }
+        const int32_t f = __float_as_int(lo.w), cnt = __float_as_int(hi.w);
+        if (cnt < 1 || cnt > kLeafMax || (uint32_t)f > (uint32_t)u - (uint32_t)cnt) {
+            if (lane == 0) set_err(&st->err, ERRBIT_BOUNDS);
+            break;
+        }
+        if (f >= sw0 && f + cnt <= sw1) continue;  // all of it was in the seed window
+        ++ct.buckets;
+        if (__any_sync(FULL, bc + cnt > kBuf)) {
+            flush(tk, bc, W, lane, ct, pts, qx, qy, qz);
+            tau = act ? fminf(tk.tau(), cap) : -1.0f;
+            tau_max = warp_max(tau);
+        }
+        if (3 * __popc(needm) < 2 * cnt)
+            scan_sparse(f, cnt, needm, qx, qy, qz, tau, bc, W, pts, (int32_t)sw0, (int32_t)sw1, lane);
+        else
+            scan_chunk(f, cnt, need, qx, qy, qz, tau, bc, W, pts, (int32_t)sw0, (int32_t)sw1, lane);
+    }
+    __syncwarp();
+}
+
 // The 32 queries [q0, q0 + 32) of one warp: search, then the outputs.
 // CELLS: the learned attempt may run the cell scan (a separate instantiation,
 // launched only when the caller turned the cell scan on: compiled into the
@@ -818,84 +947,8 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
             } while (t < nsteps);
         }
 
-        if (!scanned && u >= 2 && (sw0 > 0 || sw1 < u)) {
-            int sp = 1;
-            if (lane == 0) W.stack[0] = 0;
-            __syncwarp();
-            const uint32_t step_cap =
-                a.step_limit > 0 ? (uint32_t)a.step_limit : (uint32_t)min64(2 * u + 64, 0x7fffffff);
-            while (sp > 0) {
-                --sp;
-                const int32_t node = W.stack[sp];
-                __syncwarp();
-                if (++steps > step_cap || node < 0 || node >= u - 1) {
-                    if (lane == 0) set_err(&st->err, steps > step_cap ? ERRBIT_SEARCH_LIMIT : ERRBIT_BOUNDS);
-                    break;
-                }
-                const SNode* sn = snodes + node;
-                const float4 lo_l = __ldg(&sn->lo_l), hi_l = __ldg(&sn->hi_l);
-                const float4 lo_r = __ldg(&sn->lo_r), hi_r = __ldg(&sn->hi_r);
-                const int32_t refl = __float_as_int(lo_l.w), refr = __float_as_int(lo_r.w);
-                const int32_t cntl = __float_as_int(hi_l.w), cntr = __float_as_int(hi_r.w);
-                const uint32_t u32 = (uint32_t)u;
-                const bool okl = cntl <= a.bucket ? (cntl >= 1 && (uint32_t)refl <= u32 - (uint32_t)cntl)
-                                                  : (uint32_t)refl < u32 - 1;
-                const bool okr = cntr <= a.bucket ? (cntr >= 1 && (uint32_t)refr <= u32 - (uint32_t)cntr)
-                                                  : (uint32_t)refr < u32 - 1;
-                if (!(okl && okr)) {
-                    if (lane == 0) set_err(&st->err, ERRBIT_BOUNDS);
-                    break;
-                }
-                const float tau = fminf(tk.tau(), cap);
-                const float dl = box_dist2(qx, qy, qz, lo_l.x, lo_l.y, lo_l.z, hi_l.x, hi_l.y, hi_l.z);
-                const float dr = box_dist2(qx, qy, qz, lo_r.x, lo_r.y, lo_r.z, hi_r.x, hi_r.y, hi_r.z);
-                const uint32_t bl = __ballot_sync(FULL, act && dl <= tau);
-                const uint32_t br = __ballot_sync(FULL, act && dr <= tau);
-                if (!(bl | br)) continue;
-                const uint32_t vote = __ballot_sync(FULL, act && dl <= dr);
-                const int nact = __popc(__ballot_sync(FULL, act));
-                const bool leftFirst = 2 * __popc(vote) >= nact;
-                // rolled: one copy of the scan and merge code serves both
-                // children (a copy per child cost 4-8% in instruction fetch)
-#pragma unroll 1
-                for (int o = 0; o < 2; ++o) {
-                    const bool left = (o == 0) == leftFirst;
-                    const int32_t cnt = left ? cntl : cntr;
-                    if (cnt > a.bucket) continue;
-                    const int32_t first = left ? refl : refr;
-                    if (first >= sw0 && first + cnt <= sw1) continue;  // all of it was in the seed window
-                    const float bnd = fminf(tk.tau(), cap);
-                    const bool need = act && (left ? dl : dr) <= bnd;
-                    const uint32_t needm = __ballot_sync(FULL, need);
-                    if (!needm) continue;
-                    ++ct.buckets;
-                    // buckets of more than 32 points go in 32-point chunks
-                    for (int c0 = 0; c0 < cnt; c0 += 32) {
-                        const int32_t f = first + c0;
-                        const int n = min(32, cnt - c0);
-                        if (f >= sw0 && f + n <= sw1) continue;  // this chunk was in the seed window
-                        if (__any_sync(FULL, bc + n > kBuf)) flush(tk, bc, W, lane, ct, pts, qx, qy, qz);
-                        const float b2 = fminf(tk.tau(), cap);
-                        if (3 * __popc(needm) < 2 * n)
-                            scan_sparse(f, n, needm, qx, qy, qz, b2, bc, W, pts, (int32_t)sw0, (int32_t)sw1, lane);
-                        else
-                            scan_chunk(f, n, need, qx, qy, qz, b2, bc, W, pts, (int32_t)sw0, (int32_t)sw1, lane);
-                    }
-                }
-#pragma unroll
-                for (int o = 1; o >= 0; --o) {
-                    const bool left = (o == 0) == leftFirst;
-                    if ((left ? cntl : cntr) <= a.bucket || !(left ? bl : br)) continue;
-                    if (sp >= kStackDepth) {
-                        if (lane == 0) set_err(&st->err, ERRBIT_STACK);
-                        continue;
-                    }
-                    if (lane == 0) W.stack[sp] = left ? refl : refr;
-                    ++sp;
-                }
-                __syncwarp();
-            }
-        }
+        if (!scanned && (sw0 > 0 || sw1 < u))
+            walk<K, EXACT>(tk, bc, W, lane, ct, pts, snodes, a, st, act, qx, qy, qz, cap, u, sw0, sw1, steps);
         flush(tk, bc, W, lane, ct, pts, qx, qy, qz);
         if (attempt == 0) {
             // a lane the cell scan could not serve (its cap is +inf or not a
@@ -1116,7 +1169,6 @@ cudaError_t enqueue_query_batch(const BatchCloud* clouds, int n_clouds, int64_t 
     a.vz = q.vz;
     a.gap = q.eigengap_fp64;
     a.code_bits = q.code_bits;
-    a.bucket = q.bucket;
     a.seed_halo = q.seed_halo < 0 ? 0 : (q.seed_halo > kMaxHalo ? kMaxHalo : q.seed_halo);
     a.device_count = 1;
     const int bps = q.batch_blocks_per_sm, wpb = q.batch_warps_per_block;
@@ -1153,7 +1205,6 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     a.vz = q.vz;
     a.gap = q.eigengap_fp64;
     a.code_bits = q.code_bits;
-    a.bucket = q.bucket;
     a.seed_halo = q.seed_halo;
     a.learned_r2 = q.learned_r2;
     a.learned_skip_seed = q.learned_skip_seed;

@@ -22,6 +22,14 @@ constexpr int kDedupTile = kDedupThreads * kDedupIpt;
 constexpr int kScanThreads = 256;
 constexpr int kScanIpt = 16;
 constexpr int kScanTile = kScanThreads * kScanIpt;
+constexpr int kLeafThreads = 256;
+constexpr int kLeafIpt = 4;
+constexpr int kLeafTile = kLeafThreads * kLeafIpt;
+// Search hierarchy: leaves of at most kLeafMax points, kFan nodes under each
+// inner node, at most kMaxLevels levels (32^6 leaves).
+constexpr int kLeafMax = 32;
+constexpr int kFan = 32;
+constexpr int kMaxLevels = 6;
 
 // Query counters: fp64 solves, nodes visited, buckets scanned, candidates,
 // merge steps, inserts.
@@ -44,9 +52,11 @@ struct DevState {
     unsigned long long u;                   // unique codes
     unsigned long long n_oct;               // octree nodes
     int32_t root_level;
-    // fixed-root description used by the search hierarchy (node 0)
-    int32_t sroot_gamma;
-    int32_t sroot_hl, sroot_hr;
+    // search hierarchy: level l holds level_count[l] nodes from level_off[l] on;
+    // the top level is the first of at most kFan nodes
+    int32_t top_level;
+    uint32_t level_off[kMaxLevels];
+    uint32_t level_count[kMaxLevels];
     // query counters, in the order of se_stats
     unsigned long long counters[kQueryCounters];
 };
@@ -61,16 +71,25 @@ struct OtNode {
 };
 static_assert(sizeof(OtNode) == 56, "OTNode layout");
 
-// Search hierarchy node: internal node of the binary radix tree (root range
-// always [0, u-1]) holding both children's tight point boxes. A child with at
-// most `bucket` points is a bucket: ref = first point index, points
-// [ref, ref + cnt) are contiguous in Morton order. Otherwise ref = node index.
+// Search hierarchy node: the box of its points. A leaf (level 0) is a maximal
+// Morton subtree of at most min(leaf_bucket, 32) points: lo.w holds its first
+// point and hi.w its point count (int bits). Node i of level l covers nodes
+// [32 i, 32 i + 32) of level l - 1.
 struct __align__(16) SNode {
-    float4 lo_l;  // .w: ref of the left child (int bits)
-    float4 hi_l;  // .w: point count of the left child (int bits)
-    float4 lo_r;
-    float4 hi_r;
+    float4 lo;
+    float4 hi;
 };
+// Nodes of the hierarchy over n points, at most (every leaf holds a point).
+__host__ __device__ constexpr int64_t hierarchy_nodes(int64_t n) {
+    int64_t total = n;
+    for (int64_t c = n; c > kFan;) {
+        c = (c + kFan - 1) / kFan;
+        total += c;
+    }
+    return total;
+}
+// Words of the arrival counters that its build needs (one per node of level 2 and up).
+__host__ __device__ constexpr int64_t arrival_words(int64_t n) { return n / 512 + 16; }
 
 struct BuildBufs {
     int64_t cap;  // capacity in points
@@ -90,13 +109,14 @@ struct BuildBufs {
     uint8_t* prefix_n;
     uint8_t* has_leaf_left;
     uint8_t* has_leaf_right;
-    // search hierarchy
+    // radix tree with the full root range, for the learned radius features
     int32_t* sparent;
     int32_t* leaf_parent;
     int32_t* range_end;
-    uint32_t* visit;
-    float4* node_box;  // 2 per node: lo, hi
-    SNode* snodes;
+    // search hierarchy
+    int32_t* leaf_start;  // first point of each leaf
+    uint32_t* arrivals;   // arrival counters of the hierarchy build
+    SNode* snodes;        // hierarchy_nodes(cap) entries
     // octree
     int32_t* oct_counts;
     int32_t* oct_offsets;  // cap + 1
@@ -111,6 +131,7 @@ struct BuildParams {
     int root_compat;
     int build_octree;
     int bucket;
+    int build_radix = 1;  // 0: no radix tree (the search does not need it)
     int spin_limit = kSpinLimit;  // polls before a look-back wait gives up
     int stall_first_tile = 0;     // test hook: the first sort tile never publishes its prefix
 };
@@ -179,7 +200,6 @@ struct QueryParams {
     float vx, vy, vz;
     float eigengap_fp64;
     int code_bits;
-    int bucket;
     int seed_halo;
     const float* learned_r2;  // per query: starting bound from the learned radius, or nullptr
     int learned_skip_seed;    // with learned_r2: skip the Morton-window seed
@@ -223,7 +243,7 @@ struct BatchCloud {
 // Normals of many clouds that share q.k in one persistent launch (grid = the
 // kernel's resident blocks on every SM). `clouds` is a device array of
 // n_clouds entries, `counter` a device word this call resets. q supplies k,
-// viewpoint, eigengap threshold, bucket and seed halo.
+// viewpoint, eigengap threshold and seed halo.
 // u and the error word of every cloud of a batch (states st[0..n)) into
 // u_out / err_out.
 cudaError_t enqueue_batch_collect(const DevState* st, int n, unsigned long long* u_out, uint32_t* err_out,
