@@ -109,7 +109,7 @@ typedef struct se_options {
     int32_t batch_blocks_per_sm;   /* resident blocks per SM of the persistent launches
                                       (default: as many as fit) */
     int32_t batch_warps_per_block; /* warps per block of the persistent launches: 2 or 4
-                                      (default: 4 up to k = 16, 2 above) */
+                                      (default: 2) */
 } se_options;
 
 /* se_options.debug_inject bits. */
@@ -257,9 +257,12 @@ typedef struct se_stats {
     int64_t fp64_solves;     /* queries whose eigensolve took the FP64 path */
     int64_t nodes_visited;   /* search-hierarchy nodes whose (up to 32) children were tested, summed over warps */
     int64_t buckets_scanned; /* leaves scanned, summed over warps */
-    int64_t candidates;      /* points that reached a query's bound, summed over queries */
-    int64_t merge_steps;     /* candidate-buffer merge steps, summed over warps */
-    int64_t inserts;         /* insertions into the k-best lists, summed over queries */
+    int64_t candidates;      /* points that reached a query's bound (the first k of a seeded
+                                list among them), summed over queries */
+    int64_t merge_steps;     /* candidates merged into the k-best lists by the lane with the
+                                most of them, summed over merges and warps */
+    int64_t inserts;         /* candidates still within their bound when a warp dropped the
+                                others, summed over queries and drops */
     int64_t learned_misses;  /* queries whose learned radius was too small (searched again) */
     int64_t cell_warps;      /* warps whose learned attempt scanned Morton cells (no tree walk) */
     int64_t cell_fallbacks;  /* warps whose cells were too many: the learned attempt walked the tree */

@@ -4,6 +4,7 @@
 // point replaces are in include/shapex.h.
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <numeric>
@@ -258,7 +259,7 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
     }
     // clear the error word and counters of the previous call
     SE_CUDA(c, cudaMemsetAsync(&c->b.st->err, 0, sizeof(uint32_t), c->stream), "reset");
-    SE_CUDA(c, cudaMemsetAsync(c->b.st->counters, 0, sizeof(c->b.st->counters), c->stream), "reset");
+    SE_CUDA(c, cudaMemsetAsync(c->b.st->counters, 0, sizeof(DevState) - offsetof(DevState, counters), c->stream), "reset");
     c->have_query_times = false;
     SE_CUDA(c, cudaEventRecord(c->query_ev[0], c->stream), "event");
     if (use_learned)

@@ -8,23 +8,34 @@
 //   cusolverDnSsyevjBatched             src/NormalEstimation.hpp:235-301
 //   normalsFromEigenVectors             src/NormalEstimation.hpp:158-192
 //
-// One warp serves 32 consecutive queries (Morton-ordered, so spatially
-// coherent); lane i owns query i. Each lane keeps its k best (squared
-// distance, index) keys as a sorted list in registers, whose last entry is
-// the lane's pruning bound. The warp first offers the Morton window around its
-// queries, then walks the search hierarchy: 32 nodes are tested at once
-// against the box of the warp's queries, nearest first, and each that passes
-// by all 32 queries. Leaf points (contiguous runs of at most 32 points) are
-// staged in shared memory and read by broadcast. A point that reaches a lane's
-// bound goes to that lane's candidate buffer; buffers are merged into the
-// lists in batches, so that the warp pays for one list update per buffered
-// slot rather than one per point any lane accepts. Pruning uses the box
-// distance with the same rounding chain as the point distance, so the result
-// is exact, ties broken by point index.
+// One warp serves up to 32 consecutive queries (Morton-ordered, so spatially
+// coherent); lane i owns query i. Each lane keeps the k smallest squared
+// distances offered to it as a sorted list in registers, whose last entry is
+// its pruning bound, and the (distance, index) candidates within the bound in
+// shared memory. The warp first offers the Morton window around its queries,
+// then walks the search hierarchy: 32 nodes are tested at once against the box
+// of the warp's queries, nearest first, and each that passes by all 32
+// queries. Points come in runs of at most 32, staged in shared memory; each
+// lane's hits are a bit mask, from which they are appended to its candidates.
+// When a lane's slots are full, all lanes merge their fresh distances into
+// their lists and drop the candidates beyond their bounds. The k nearest are
+// the candidates left at the end, sorted by (distance, index). Pruning uses the
+// box distance with the same rounding chain as the point distance, so the
+// result is exact, ties broken by point index.
+//
+// Before, the lists held (distance, index) keys and took one insertion per
+// buffered candidate. Distances alone merge eight at a time through min/max
+// networks in half the registers, and nothing is gathered twice: 2M scene,
+// k = 16, ALU instructions 0.81 G -> 0.52 G, search 2.69 -> 2.29 ms; 20M
+// precision mix 18.0 -> 15.5 ms; 1M lists of 32 3.14 -> 2.05 ms. What holds it
+// now is latency: issue slots 54% busy, fixed-latency waits 2.4 per issue,
+// shared and global loads 0.9 each.
 
 #include <cfloat>
 #include <climits>
 #include <cstdint>
+#include <type_traits>
+#include <utility>
 
 #include "pipeline.cuh"
 #include "eig3.cuh"
@@ -33,27 +44,23 @@ namespace shapex {
 
 namespace {
 
-// Per-k tile shape, measured on B200 (2M scene and 5M mixture clouds): small
-// lists leave registers for more resident warps, which pays for itself up to
-// k = 16. The 24- and 32-key lists need more registers, so they keep the
-// larger buffer and run in 2-warp blocks: 7 resident blocks (14 warps) where
-// 4-warp blocks fit only 3 (12 warps); k = 32 ran 2.7% faster. k = 24 fits
-// 128 registers without spills and is asked for 8 blocks (16 warps): at 130
-// registers (7 blocks) it ran 11% slower on the 2M scene. k = 32 asks for 6
-// so that ptxas does not cap its registers (a cap of 7 x 64 threads forced
-// 128 registers and spills). Registers, not shared
-// memory, hold k <= 16 at 5 blocks, so its buffer grew from 48 to 56 slots
-// (fewer flushes; the learned search ran 3% faster). 64 slots shrank the L1
-// cache enough to cost 3-4%.
+// Per-k tile shape, measured on B200 (2M scene): candidate slots (8 bytes per
+// lane and slot, shared memory) against resident warps. Fewer slots mean more
+// merges and prunes, fewer warps leave the fixed-latency stalls uncovered, and
+// registers beyond the budget spill. k = 16: 28 slots x 24 warps 2281 us, 32 x
+// 22 2288 (20M precision mix 15.47 ms; kept), 36 x 20 2328, 24 x 28 2787;
+// k = 8: 22 x 28 1434 us, 22 x 24 1477, 18 x 24 1480, 20 x 20 1578; k = 32
+// (1M): 48 x 16 2049 us, 56 x 14 2105, 52 x 14 2177, 44 x 18 2230. Blocks of
+// two warps: with four, 22 warps do not divide; one each costs 1 KB of reserved
+// shared memory per warp (2371 us).
 template <int K>
 struct KnnCfg {
-    static constexpr int buf = K <= 8 ? 40 : (K <= 16 ? 56 : 64);  // candidate buffer slots per lane
-    static constexpr int threads = K <= 16 ? 128 : 64;              // block size
+    static constexpr int buf = K <= 8 ? 22 : (K <= 16 ? 32 : (K <= 24 ? 40 : 48));  // candidate slots per lane
+    static constexpr int threads = 64;                                                // block size
     static constexpr int warps = threads / 32;
-    static constexpr int min_blocks = K <= 8 ? 6 : (K <= 16 ? 5 : (K <= 24 ? 8 : 6));  // resident blocks per SM asked of ptxas
+    static constexpr int min_blocks = K <= 8 ? 14 : (K <= 16 ? 11 : (K <= 24 ? 9 : 8));  // resident blocks per SM asked of ptxas
 };
 constexpr int kMaxHalo = 48;            // seed points on each side of a warp's queries
-constexpr int kWindowMax = 32 + 2 * kMaxHalo;
 constexpr unsigned FULL = 0xffffffffu;
 
 // (squared distance, index) packed so that one unsigned compare orders by
@@ -65,142 +72,129 @@ constexpr unsigned long long kEmptyKey = (0x7f800000ull << 32) | 0xffffffffull; 
 __device__ __forceinline__ int32_t key_idx(unsigned long long k) { return (int32_t)(uint32_t)k; }
 __device__ __forceinline__ float key_d(unsigned long long k) { return __uint_as_float((uint32_t)(k >> 32)); }
 
-// key[i] for a run-time i, as a masked OR over all entries, so that the list
-// stays in registers (a direct key[i] would move it to local memory).
+// v[i] for a run-time i, as a masked OR over all entries, so that the list
+// stays in registers (a direct v[i] would move it to local memory).
 template <int K>
-__device__ __forceinline__ unsigned long long pick(const unsigned long long (&key)[K], int i) {
-    unsigned long long acc = 0;
+__device__ __forceinline__ float pick(const float (&v)[K], int i) {
+    uint32_t acc = 0;
 #pragma unroll
-    for (int j = 0; j < K; ++j) acc |= key[j] & (0ull - (unsigned long long)(j == i));
-    return acc;
+    for (int j = 0; j < K; ++j) acc |= j == i ? __float_as_uint(v[j]) : 0u;
+    return __uint_as_float(acc);
 }
 
-// The k best keys of one query, ascending, in registers. Insertion compares
-// the new key with every entry independently and shifts in one step (no
-// serial chain). With EXACT = false the list is longer than k and the bound
-// is entry k-1.
-template <int K, bool EXACT>
-struct TopK {
-    static_assert(K % 2 == 0, "list sizes are even");
-    unsigned long long key[K];
-    unsigned long long bk;  // entry k-1: the pruning bound
-    int kk;
-    __device__ __forceinline__ void init(int k) {
-#pragma unroll
-        for (int j = 0; j < K; ++j) key[j] = kEmptyKey;
-        bk = kEmptyKey;
-        kk = k;
-    }
-    __device__ __forceinline__ float tau() const { return key_d(bk); }
-    // After key[0..K) was filled with arbitrary keys: sort ascending with an
-    // odd-even transposition network (K passes of independent
-    // compare-exchanges) and set the bound.
-    __device__ __forceinline__ void sort_filled() {
-        if constexpr (K == 4 || K == 8 || K == 16) {
-            // power-of-two lists: a bitonic network, fully unrolled (80
-            // compare-exchanges at K = 16 against 120 for the transposition
-            // network below, in about as much code)
-#pragma unroll
-            for (int k = 2; k <= K; k <<= 1)
-#pragma unroll
-                for (int j = k >> 1; j > 0; j >>= 1)
-#pragma unroll
-                    for (int i = 0; i < K; ++i) {
-                        const int l = i ^ j;
-                        if (l > i) {
-                            const unsigned long long a = key[i], b = key[l];
-                            const bool up = (i & k) == 0;
-                            const bool sw = up ? (b < a) : (a < b);
-                            key[i] = sw ? b : a;
-                            key[l] = sw ? a : b;
+__device__ __forceinline__ void exchange(float& a, float& b) {  // a <= b afterwards
+    const float t = fminf(a, b);
+    b = fmaxf(a, b);
+    a = t;
+}
+__device__ __forceinline__ void exchange(unsigned long long& a, unsigned long long& b) {
+    const bool sw = b < a;
+    const unsigned long long t = sw ? b : a;
+    b = sw ? a : b;
+    a = t;
+}
+
+// Ascending sort of N values in registers: Batcher's odd-even merge exchange
+// (Knuth, TAOCP vol. 3, Algorithm 5.2.2M): 19 exchanges for 8 values, 63 for
+// 16, 191 for 32. The network is a compile-time list of wire pairs.
+template <int N>
+struct SortNet {
+    int n = 0;
+    int lo[N * N / 2] = {}, hi[N * N / 2] = {};
+    __host__ __device__ constexpr SortNet() {
+        for (int p = 1; p < N; p <<= 1)
+            for (int k = p; k >= 1; k >>= 1)
+                for (int j = k % p; j + k < N; j += 2 * k)
+                    for (int i = j; i < j + k && i + k < N; ++i)
+                        if (i / (2 * p) == (i + k) / (2 * p)) {
+                            lo[n] = i;
+                            hi[n++] = i + k;
                         }
-                    }
-        } else {
-            // K passes as K/2 rolled (even, odd) pairs: the same exchanges as
-            // a fully unrolled network in K instead of K*K/2 instructions'
-            // worth of code, which keeps large-k kernels inside the
-            // instruction cache
-#pragma unroll 1
-            for (int pass = 0; pass < K; pass += 2) {
-#pragma unroll
-                for (int j = 0; j + 1 < K; j += 2) {
-                    const unsigned long long a = key[j], b = key[j + 1];
-                    key[j] = a < b ? a : b;
-                    key[j + 1] = a < b ? b : a;
+    }
+};
+// A bitonic merge of N wires, N not necessarily a power of two: the network
+// of the next power of two with its lowest wires held at minus infinity, so
+// that their exchanges fall away.
+template <int N>
+struct MergeNet {
+    int n = 0;
+    int lo[N * 5] = {}, hi[N * 5] = {};
+    __host__ __device__ constexpr MergeNet() {
+        int P = 1;
+        while (P < N) P <<= 1;
+        for (int h = P / 2; h >= 1; h >>= 1)
+            for (int i = P - N; i + h < P; ++i)
+                if ((i & h) == 0) {
+                    lo[n] = i - (P - N);
+                    hi[n++] = i + h - (P - N);
                 }
-#pragma unroll
-                for (int j = 1; j + 1 < K; j += 2) {
-                    const unsigned long long a = key[j], b = key[j + 1];
-                    key[j] = a < b ? a : b;
-                    key[j + 1] = a < b ? b : a;
-                }
-            }
-        }
-        if (EXACT) {
-            bk = key[K - 1];
-        } else {
-            bk = pick(key, kk - 1);
-        }
     }
-    // insert() for a key that lands in the last K - H entries (nk > key[H - 1]):
-    // the first H stay, so only the rest is compared and shifted.
-    template <int H>
-    __device__ __forceinline__ void insert_upper(unsigned long long nk) {  // requires key[H-1] < nk < bk
-        bool lt[K];
+};
+template <class Net, class T, int N, size_t... I>
+__device__ __forceinline__ void run_net(T (&v)[N], std::index_sequence<I...>) {
+    constexpr Net net;
+    (exchange(v[std::integral_constant<int, net.lo[I]>::value], v[std::integral_constant<int, net.hi[I]>::value]), ...);
+}
+template <class T, int N>
+__device__ __forceinline__ void sort_values(T (&v)[N]) {
+    run_net<SortNet<N>>(v, std::make_index_sequence<SortNet<N>().n>());
+}
+
+constexpr int kBatch = 8;  // candidates merged into a list at once
+
+// The k smallest squared distances offered to one query so far, ascending, in
+// registers; their last is the pruning bound. The points they belong to are
+// not carried along: the lane's buffer of candidate indices keeps every point
+// within the bound, and the k nearest are taken from it at the end. With
+// EXACT = false the list is longer than k and the bound is entry k-1.
+//
+// Distances alone are 32 bits, so an exchange of the merge network is a min
+// and a max, where (distance, index) keys took six instructions on the
+// half-rate ALU pipe, and the list takes half the registers.
+template <int K, bool EXACT>
+struct Nearest {
+    float d[K];
+    float tau;  // d[k - 1]
+    __device__ __forceinline__ void init() {
 #pragma unroll
-        for (int j = H; j < K; ++j) lt[j] = key[j] < nk;
-#pragma unroll
-        for (int j = K - 1; j >= H + 1; --j) key[j] = lt[j] ? key[j] : (lt[j - 1] ? nk : key[j - 1]);
-        key[H] = lt[H] ? key[H] : nk;
-        if (EXACT) {
-            bk = key[K - 1];
-        } else {
-            bk = pick(key, kk - 1);
-        }
+        for (int j = 0; j < K; ++j) d[j] = INFINITY;
+        tau = INFINITY;
     }
-    // One merge step of the warp (lists of up to 16 keys): lanes with `ins`
-    // insert nk; when every inserting lane's key lands in the upper half of
-    // its list (most late insertions), the warp takes the half-width
-    // insertion. Plain kNN 1.5-3.7% faster at k = 16. Lists of 24 and 32 keys
-    // keep the full insertion: the second one's registers cost them
-    // occupancy (k = 32 1-4% slower).
-    __device__ __forceinline__ void merge_step(unsigned long long nk, bool ins) {
-        if (!__any_sync(0xffffffffu, ins)) return;
-        if (__all_sync(0xffffffffu, !ins || nk > key[K / 2 - 1])) {
-            if (ins) insert_upper<K / 2>(nk);
-        } else {
-            if (ins) insert(nk);
-        }
+    __device__ __forceinline__ void set_bound(int k) { tau = EXACT ? d[K - 1] : pick(d, k - 1); }
+    __device__ __forceinline__ void sort_filled(int k) {
+        sort_values(d);
+        set_bound(k);
     }
-    __device__ __forceinline__ void insert(unsigned long long nk) {  // requires nk < bk
-        bool lt[K];
+    // The K lowest of the list and the batch c: the list's tail against the
+    // sorted batch reversed leaves the K lowest as a sequence that rises and
+    // then falls (Batcher 1968), which a bitonic merge sorts.
+    __device__ __forceinline__ void merge(float (&c)[kBatch], int k) {
+        sort_values(c);
 #pragma unroll
-        for (int j = 0; j < K; ++j) lt[j] = key[j] < nk;
-#pragma unroll
-        for (int j = K - 1; j >= 1; --j) key[j] = lt[j] ? key[j] : (lt[j - 1] ? nk : key[j - 1]);
-        key[0] = lt[0] ? key[0] : nk;
-        if (EXACT) {
-            bk = key[K - 1];
-        } else {
-            bk = pick(key, kk - 1);
-        }
+        for (int t = 0; t < kBatch && t < K; ++t) d[K - 1 - t] = fminf(d[K - 1 - t], c[t]);
+        run_net<MergeNet<K>>(d, std::make_index_sequence<MergeNet<K>().n>());
+        set_bound(k);
     }
 };
 
-// Per-warp shared scratch: staged points (the seed window, then one leaf in
-// its first 32 entries), candidate buffers ([slot][lane] so that a warp's
-// accesses to one slot fall in distinct banks). While the warp walks the
-// hierarchy, entries [64, 104) of pts hold the order keys of the levels above
-// the current one.
-template <int B>
+// Per-warp shared scratch. pts[0, 24): a staged run of 32 points; pts[24, 64):
+// while the warp walks the hierarchy, the order keys of the levels above the
+// current one; pts[64, 96): the lanes' queries and bounds. The cell scan uses
+// a larger pts in its own way. d and idx: each lane's candidates, [slot][lane]
+// so that a warp's accesses to one slot fall in distinct banks.
+template <int B, bool CELLS = false>
 struct WarpSmem {
-    float4 pts[kWindowMax];
-    int32_t buf[B][32];
+    float4 pts[CELLS ? 128 : 96];
+    float d[B][32];
+    int32_t idx[B][32];
+    uint32_t count[kQueryCounters];  // the warp's work counters, added to the build state's when it ends
+    float4 box_lo, box_hi;           // the box of the warp's active queries
     __device__ __forceinline__ uint32_t* level_keys(int l) {  // l >= 1
-        return reinterpret_cast<uint32_t*>(&pts[64]) + 32 * (l - 1);
+        return reinterpret_cast<uint32_t*>(&pts[24]) + 32 * (l - 1);
     }
+    __device__ __forceinline__ float4* query() { return pts + 64; }  // x, y, z, bound (-1: idle lane)
 };
-static_assert(64 + (kMaxLevels - 1) * 8 <= kWindowMax, "order keys fit behind the staged leaf");
+static_assert(24 + (kMaxLevels - 1) * 8 <= 64, "order keys fit behind the staged run");
 
 // Ordered widest first so that the struct packs into 128 bytes: one more
 // padded word (144 bytes) made ptxas give the k = 32 kernels 161-163
@@ -224,6 +218,7 @@ struct QArgs {
     int lut_shift;     // per-axis shift of the table's level (bits per axis - level)
     int cell_pmax;     // cell scan: most points per warp before it falls back to the walk
     int cell_span;     // cell scan: most cells per axis covering one lane's ball (2..4)
+    int warp_queries;  // queries per warp, 1..32
 };
 static_assert(sizeof(QArgs) <= 128, "QArgs grew past 128 bytes");
 
@@ -232,121 +227,166 @@ struct Counters {
         cell_points = 0;
 };
 
-// Merge every lane's buffered candidates into its list; the warp steps
-// through max-over-lanes slots together.
+// One query: its candidates are slots [0, n) of the lane's columns W.d and
+// W.idx, every point offered so far that may be among its k nearest; the
+// distances of the first `merged` of them are in the list.
+struct Query {
+    float x, y, z;
+    int k;
+    int n, merged;
+};
+
+// Merge the distances of every lane's fresh candidates into its list; the warp
+// steps through max-over-lanes batches together.
 template <int K, bool EXACT, class WS>
-__device__ __forceinline__ void flush(TopK<K, EXACT>& tk, int& bc, WS& W, int lane, Counters& ct,
-                                      const float4* __restrict__ pts, float qx, float qy, float qz) {
-    const int maxc = (int)__reduce_max_sync(FULL, (unsigned)bc);
-    ct.merge += maxc;
-    ct.cand += bc;
-    if (K > 8) {
-        // the next candidate's point is loaded before this one's insertion,
-        // hiding its latency behind the list update (about 1% at k >= 16;
-        // slower at k = 8, whose insertions are too short to hide it)
-        int32_t idx_n = bc > 0 ? W.buf[0][lane] : 0;
-        float4 p_n = bc > 0 ? __ldg(pts + idx_n) : make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int j = 0; j < maxc; ++j) {
-            const int32_t idx = idx_n;
-            const float4 p = p_n;
-            if (j + 1 < bc) {
-                idx_n = W.buf[j + 1][lane];
-                p_n = __ldg(pts + idx_n);
+__device__ __forceinline__ void merge_fresh(Nearest<K, EXACT>& nn, Query& q, WS& W, int lane, Counters& ct) {
+    const int fresh = q.n - q.merged;
+    const int most = (int)__reduce_max_sync(FULL, (unsigned)fresh);
+    ct.merge += most;
+    ct.cand += fresh;
+#pragma unroll 1
+    for (int j = 0; j < most; j += kBatch) {
+        float c[kBatch];
+#pragma unroll
+        for (int t = 0; t < kBatch; ++t) c[t] = j + t < fresh ? W.d[q.merged + j + t][lane] : INFINITY;
+        nn.merge(c, q.k);
+    }
+    q.merged = q.n;
+}
+
+// Drop the candidates beyond every lane's bound (all must be merged). At most
+// `room` stay: equal distances can leave more than k, and of those at the
+// bound the lowest indices go first, as in the lists.
+template <class WS>
+__device__ __forceinline__ void prune(Query& q, float tau, int room, WS& W, int lane, Counters& ct) {
+    const int most = (int)__reduce_max_sync(FULL, (unsigned)q.n);
+    int w = 0;
+#pragma unroll 4
+    for (int j = 0; j < most; ++j) {
+        const float d = W.d[j][lane];
+        if (j < q.n && d <= tau) {
+            const int32_t i = W.idx[j][lane];
+            W.d[w][lane] = d;
+            W.idx[w][lane] = i;
+            ++w;
+        }
+    }
+    ct.ins += w;
+    if (w > room) {  // ties at the bound: keep k candidates
+        int ties = q.k;
+        for (int j = 0; j < w; ++j) ties -= W.d[j][lane] < tau;
+        int32_t last = -1;  // the ties-th lowest index at the bound
+        for (int i = 0; i < ties; ++i) {
+            int32_t next = INT_MAX;
+            for (int j = 0; j < w; ++j) {
+                const int32_t at = W.idx[j][lane];
+                if (at > last && at < next && W.d[j][lane] == tau) next = at;
             }
-            if constexpr (K <= 16) {
-                const unsigned long long nk = pack_key(dist2(qx, qy, qz, p.x, p.y, p.z), idx);
-                const bool ins = j < bc && nk < tk.bk;
-                tk.merge_step(nk, ins);
-                ct.ins += ins;
-            } else {
-                if (j < bc) {
-                    const unsigned long long nk = pack_key(dist2(qx, qy, qz, p.x, p.y, p.z), idx);
-                    if (nk < tk.bk) {
-                        tk.insert(nk);
-                        ++ct.ins;
-                    }
+            last = next;
+        }
+        int v = 0;
+        for (int j = 0; j < w; ++j) {
+            const float d = W.d[j][lane];
+            const int32_t at = W.idx[j][lane];
+            if (d < tau || at <= last) {
+                W.d[v][lane] = d;
+                W.idx[v][lane] = at;
+                ++v;
+            }
+        }
+        w = v;
+    }
+    q.n = q.merged = w;
+}
+
+// Append every lane's hits among a run of points (bit i of `hits`: point
+// `first` + i, at(i) its coordinates) to its candidates, making room on the
+// way; a hit that a bound tightened meanwhile excludes is passed over. With
+// `settle` all candidates are merged in any case.
+template <int K, bool EXACT, class WS, class At>
+__device__ __forceinline__ void take_hits(uint32_t hits, bool settle, At at, Nearest<K, EXACT>& nn, Query& q, float& tau,
+                                          float cap, WS& W, int lane, Counters& ct) {
+    constexpr int kBuf = KnnCfg<K>::buf;
+    for (;;) {
+        const int mine = __popc(hits);
+        int rounds = (int)__reduce_max_sync(FULL, (unsigned)mine);
+        if (rounds == 0 && !settle) return;
+        if (settle || __any_sync(FULL, q.n + mine > kBuf)) {
+            settle = false;
+            merge_fresh(nn, q, W, lane, ct);
+            prune(q, nn.tau, kBuf - 8, W, lane, ct);
+            if (tau >= 0.0f) tau = fminf(nn.tau, cap);
+            rounds = min(rounds, (int)__reduce_min_sync(FULL, (unsigned)(kBuf - q.n)));
+        }
+#pragma unroll 1
+        for (; rounds > 0; --rounds) {
+            if (hits) {
+                const int i = __ffs(hits) - 1;
+                hits &= hits - 1;
+                int32_t idx;
+                const float3 p = at(i, idx);
+                const float d = dist2(q.x, q.y, q.z, p.x, p.y, p.z);
+                if (d <= tau) {
+                    W.d[q.n][lane] = d;
+                    W.idx[q.n][lane] = idx;
+                    ++q.n;
                 }
             }
         }
-    } else {
-        for (int j = 0; j < maxc; ++j) {
-            const bool in = j < bc;
-            const int32_t idx = in ? W.buf[j][lane] : 0;
-            const float4 p = __ldg(pts + idx);
-            const unsigned long long nk = pack_key(dist2(qx, qy, qz, p.x, p.y, p.z), idx);
-            const bool ins = in && nk < tk.bk;
-            tk.merge_step(nk, ins);
-            ct.ins += ins;
-        }
     }
-    bc = 0;
 }
 
-// Stage points [first, first + cnt) (cnt <= 32) in shared memory and append
-// every one whose distance reaches the lane's bound to the lane's buffer.
-// Points of the seed window [w0, w1) are skipped (they were already offered).
-// The caller guarantees that bc + cnt fits the buffer.
-// The points are staged in pairs for dist2_pair: floats [4j, 4j + 4) hold
-// x and y of points 2j and 2j + 1, floats [64 + 2j, 64 + 2j + 2) their z; a
-// slot past cnt holds a NaN x, whose distance passes no bound.
+// The lanes' hits among points [first, first + cnt) (cnt <= 32) except those in
+// [w0, w1) (already offered): bit i of a lane's mask for point first + i within
+// its bound. The points are staged in pairs for dist2_pair: floats [4j, 4j + 4)
+// hold x and y of points 2j and 2j + 1, floats [64 + 2j, 64 + 2j + 2) their z;
+// a slot past cnt holds a NaN x, whose distance passes no bound. Either every
+// lane tests all points (two at a time), or, when few lanes need them (`needm`),
+// each lane holds one point and the warp steps over those queries, so that the
+// cost follows their number.
 template <class WS>
-__device__ __forceinline__ void scan_chunk(int32_t first, int cnt, bool need, float qx, float qy, float qz,
-                                           float tau, int& bc, WS& W, const float4* __restrict__ pts,
-                                           int32_t w0, int32_t w1, int lane) {
+__device__ __forceinline__ uint32_t scan_run(int32_t first, int cnt, uint32_t needm, int32_t w0, int32_t w1,
+                                             const Query& q, float tau, WS& W, int lane,
+                                             const float4* __restrict__ pts) {
     float* f = reinterpret_cast<float*>(W.pts);
+    const float4 p = lane < cnt ? __ldg(pts + first + lane) : make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
     {
-        const float4 p = lane < cnt ? __ldg(pts + first + lane) : make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
         const int o = 4 * (lane >> 1) + (lane & 1);
         f[o] = p.x;
         f[o + 2] = p.y;
         f[64 + lane] = p.z;
     }
     __syncwarp();
-    if (need) {
-        const uint64_t qqx = twice(qx), qqy = twice(qy), qqz = twice(qz);
-        if (first < w1 && first + cnt > w0) {  // overlaps the seed window: skip its points
-            for (int t = 0; t < cnt; t += 2) {
-                const ulonglong2 xy = *reinterpret_cast<const ulonglong2*>(f + 2 * t);
-                const uint64_t d = dist2_pair(qqx, qqy, qqz, xy.x, xy.y, *reinterpret_cast<const uint64_t*>(f + 64 + t));
-                const int32_t idx = first + t;
-                if (lo_half(d) <= tau && (idx < w0 || idx >= w1)) W.buf[bc++][lane] = idx;
-                if (hi_half(d) <= tau && (idx + 1 < w0 || idx + 1 >= w1)) W.buf[bc++][lane] = idx + 1;
+    uint32_t hits = 0;
+    if (2 * __popc(needm) < cnt) {
+        while (needm) {
+            const int i = __ffs(needm) - 1;
+            needm &= needm - 1;
+            const float4 o = W.query()[i];
+            const uint32_t h = __ballot_sync(FULL, dist2(o.x, o.y, o.z, p.x, p.y, p.z) <= o.w);
+            if (lane == i) hits = h;
+        }
+    } else {
+        const uint64_t qqx = twice(q.x), qqy = twice(q.y), qqz = twice(q.z);
+#pragma unroll 1
+        for (int t = 0; t < cnt; t += 8) {
+            uint32_t h = 0;
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                const ulonglong2 xy = *reinterpret_cast<const ulonglong2*>(f + 2 * (t + e));
+                const uint64_t d =
+                    dist2_pair(qqx, qqy, qqz, xy.x, xy.y, *reinterpret_cast<const uint64_t*>(f + 64 + t + e));
+                if (lo_half(d) <= tau) h |= 1u << e;
+                if (hi_half(d) <= tau) h |= 2u << e;
             }
-        } else {
-            for (int t = 0; t < cnt; t += 2) {
-                const ulonglong2 xy = *reinterpret_cast<const ulonglong2*>(f + 2 * t);
-                const uint64_t d = dist2_pair(qqx, qqy, qqz, xy.x, xy.y, *reinterpret_cast<const uint64_t*>(f + 64 + t));
-                if (lo_half(d) <= tau) W.buf[bc++][lane] = first + t;
-                if (hi_half(d) <= tau) W.buf[bc++][lane] = first + t + 1;
-            }
+            hits |= h << t;
         }
     }
-    __syncwarp();
-}
-
-// Same as scan_chunk when few lanes need the bucket (`mask`): each lane holds
-// one point of the bucket and the warp steps over the needing queries, so the
-// cost follows the number of needing lanes rather than the bucket size. Hits
-// are appended to the needing lane's buffer in ballot order.
-template <class WS>
-__device__ __forceinline__ void scan_sparse(int32_t first, int cnt, uint32_t mask, float qx, float qy, float qz,
-                                            float tau, int& bc, WS& W, const float4* __restrict__ pts,
-                                            int32_t w0, int32_t w1, int lane) {
-    const int32_t idx = first + lane;
-    const bool has = lane < cnt && (idx < w0 || idx >= w1);
-    const float4 p = lane < cnt ? __ldg(pts + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
-    while (mask) {
-        const int i = __ffs(mask) - 1;
-        mask &= mask - 1;
-        const float xi = __shfl_sync(FULL, qx, i), yi = __shfl_sync(FULL, qy, i), zi = __shfl_sync(FULL, qz, i);
-        const float ti = __shfl_sync(FULL, tau, i);
-        const int base = __shfl_sync(FULL, bc, i);
-        const bool pass = has && dist2(xi, yi, zi, p.x, p.y, p.z) <= ti;
-        const uint32_t pm = __ballot_sync(FULL, pass);
-        if (pass) W.buf[base + __popc(pm & lanemask_lt())][i] = idx;
-        if (lane == i) bc += __popc(pm);
+    if (first < w1 && first + cnt > w0) {  // some were already offered
+        const int lo = max(w0 - first, 0), hi = min(w1 - first, 32);
+        hits &= ~((0xffffffffu >> (32 - (hi - lo))) << lo);
     }
-    __syncwarp();
+    return hits;
 }
 
 // Position of set bit number n (from 0) of w; w has more than n set bits.
@@ -432,11 +472,10 @@ constexpr int kCellRanges = 64;   // nonempty cells a warp scans: listed in pts[
 // cells are too many (queries spread across distant regions) or hold more
 // than cell_pmax points; the caller then walks the tree with the cap.
 template <int K, bool EXACT, class WS>
-__device__ __forceinline__ bool cell_scan(TopK<K, EXACT>& tk, int& bc, WS& W, int lane, Counters& ct,
+__device__ __forceinline__ bool cell_scan(Nearest<K, EXACT>& nn, Query& q, WS& W, int lane, Counters& ct,
                                           const float4* __restrict__ pts, const uint64_t* __restrict__ codes,
-                                          const QArgs& a, const DevState* st, bool act, int64_t qi, float qx,
-                                          float qy, float qz, float cap) {
-    constexpr int kBuf = KnnCfg<K>::buf;
+                                          const QArgs& a, const DevState* st, bool act, int64_t qi, float cap) {
+    const float qx = q.x, qy = q.y, qz = q.z;
     const int bpa = a.code_bits / 3;
     const uint32_t M = bitscale_of(a.code_bits);
     const float fbs = (float)M;
@@ -575,19 +614,22 @@ __device__ __forceinline__ bool cell_scan(TopK<K, EXACT>& tk, int& bc, WS& W, in
     bool merged = false;
     auto test_chunk = [&](int n) {
         __syncwarp();
-        if (__any_sync(FULL, bc + n > kBuf)) flush(tk, bc, W, lane, ct, pts, qx, qy, qz);
-        if (ok) {
-            const float b2 = fminf(tk.tau(), cap);
-            for (int t = 0; t < n; ++t) {
-                const float4 p = W.pts[t];
-                if (dist2(qx, qy, qz, p.x, p.y, p.z) <= b2) W.buf[bc++][lane] = __float_as_int(p.w);
-            }
+        float b2 = ok ? fminf(nn.tau, cap) : -1.0f;
+        uint32_t hits = 0;
+        for (int t = 0; t < n; ++t) {
+            const float4 p = W.pts[t];
+            if (dist2(qx, qy, qz, p.x, p.y, p.z) <= b2) hits |= 1u << t;
         }
+        take_hits<K, EXACT>(
+            hits, !merged,
+            [&](int i, int32_t& idx) {
+                const float4 p = W.pts[i];
+                idx = __float_as_int(p.w);
+                return make_float3(p.x, p.y, p.z);
+            },
+            nn, q, b2, cap, W, lane, ct);
         __syncwarp();
-        if (!merged) {  // the nearest points usually hold most of each list: merge them at once
-            merged = true;
-            flush(tk, bc, W, lane, ct, pts, qx, qy, qz);
-        }
+        merged = true;
     };
     for (int it = 0; it < nr; ++it) {
         const uint32_t m = __reduce_min_sync(FULL, min(ok0, ok1));
@@ -602,7 +644,7 @@ __device__ __forceinline__ bool cell_scan(TopK<K, EXACT>& tk, int& bc, WS& W, in
             axis_bounds(Cax << s, (uint32_t)min64((int64_t)M, ((int64_t)(Cax + 1) << s) - 1), inv_m, mn, range, pad,
                         bl[ax], bh[ax]);
         }
-        const bool need = ok && box_dist2(qx, qy, qz, bl[0], bl[1], bl[2], bh[0], bh[1], bh[2]) <= fminf(tk.tau(), cap);
+        const bool need = ok && box_dist2(qx, qy, qz, bl[0], bl[1], bl[2], bh[0], bh[1], bh[2]) <= fminf(nn.tau, cap);
         if (!__any_sync(FULL, need)) continue;
         ++ct.buckets;
         for (int off = 0; off < r.y;) {
@@ -633,7 +675,7 @@ __device__ __forceinline__ void neu_add(float& s, float& c, float x) {
 }
 
 // Normal of one query from its k neighbours, ascending, whose indices are in
-// nbr[0], nbr[32], ... (the lane's column of the candidate buffer, free once
+// nbr[0], nbr[32], ... (the lane's column of the candidate indices, free once
 // the search is done; rolled loops keep the code small for large k):
 // centred covariance with compensated FP32 sums, FP32 Jacobi, FP64 redo when
 // the relative eigengap (l1 - l0) / l2 is below `gap`, orientation towards
@@ -725,18 +767,29 @@ __device__ __forceinline__ float warp_max(float v) {
 // lane, against the box of the warp's queries (its distance to a child's box
 // never exceeds that of any query in it, by the same rounding chain); a child
 // within the largest bound of the warp is then tested by every lane against
-// its own query and bound. The first test is one pass for 32 nodes where a
-// binary tree took a visit for every two; the second keeps warps whose queries
-// lie far apart (their box covers what is between) from descending everywhere.
+// its own query and bound. The first test is one pass for 32 nodes where the
+// binary tree before it took a visit for every two (2M scene, k = 16: 43 tree
+// visits and 12 buckets of about 60 points per warp became 19 visits of 32
+// nodes and 21 leaves of about 20 points; warp instructions 2.10 G -> 1.71 G,
+// search 3.08 -> 2.69 ms; 20M precision mix 20.8 -> 18.0 ms, both with the
+// earlier lists). The second keeps warps whose queries lie far apart (their
+// box covers what is between) from descending everywhere. Fetching the next
+// sibling's box one step ahead was slower (3.01 ms): its registers and moves
+// cost more than the load, which mostly hits L1.
 // A lane's order key is its child's distance with the lane in the low 5 bits
 // (rounded down, so still a lower bound); keys of the levels above wait in
 // shared memory.
+// Before the walk the warp offers the Morton window [w0, w1) around its
+// queries to all of them, except the points [e0, e1) that a lane's list was
+// filled with (w0 = w1: no seed). Window runs and leaves go through one copy
+// of the scan and merge code: with a copy each, instruction fetch stalls
+// doubled.
 template <int K, bool EXACT, class WS>
-__device__ __forceinline__ void walk(TopK<K, EXACT>& tk, int& bc, WS& W, int lane, Counters& ct,
-                                     const float4* __restrict__ pts, const SNode* __restrict__ snodes, const QArgs& a,
-                                     DevState* st, bool act, float qx, float qy, float qz, float cap, int64_t u,
-                                     int64_t sw0, int64_t sw1, uint32_t& steps) {
-    constexpr int kBuf = KnnCfg<K>::buf;
+__device__ __forceinline__ void search(Nearest<K, EXACT>& nn, Query& q, WS& W, int lane, Counters& ct,
+                                       const float4* __restrict__ pts, const SNode* __restrict__ snodes,
+                                       const QArgs& a, DevState* st, bool act, float cap, int32_t u, int32_t w0,
+                                       int32_t w1, int32_t e0, int32_t e1, uint32_t& steps) {
+    const float qx = q.x, qy = q.y, qz = q.z;
     constexpr uint32_t kNone = 0xffffffffu;
     // Siblings that pass the first test before each is tested by all 32 queries
     // at once. Most warps pass a few of 32; a warp across a Morton jump passes
@@ -745,13 +798,12 @@ __device__ __forceinline__ void walk(TopK<K, EXACT>& tk, int& bc, WS& W, int lan
     // 12. Large clouds, where other warps fill in, pay for it sooner: the 20M
     // precision mix 17.89 ms without, 18.04 at 24, 18.52 at 12.
     constexpr int kMaxLoose = 24;
-    // the box of the active queries
-    const float lx = warp_min(act ? qx : INFINITY), hx = warp_max(act ? qx : -INFINITY);
-    const float ly = warp_min(act ? qy : INFINITY), hy = warp_max(act ? qy : -INFINITY);
-    const float lz = warp_min(act ? qz : INFINITY), hz = warp_max(act ? qz : -INFINITY);
-    const uint32_t step_cap = a.step_limit > 0 ? (uint32_t)a.step_limit : (uint32_t)min64(4 * u + 64, 0x7fffffff);
-    float tau = act ? fminf(tk.tau(), cap) : -1.0f;
-    float tau_max = warp_max(tau);
+    W.box_lo = make_float4(warp_min(act ? qx : INFINITY), warp_min(act ? qy : INFINITY), warp_min(act ? qz : INFINITY), 0.f);
+    W.box_hi = make_float4(warp_max(act ? qx : -INFINITY), warp_max(act ? qy : -INFINITY), warp_max(act ? qz : -INFINITY), 0.f);
+    const uint32_t step_cap = a.step_limit > 0 ? (uint32_t)a.step_limit : (uint32_t)min64(4 * (int64_t)u + 64, 0x7fffffff);
+    float tau = act ? fminf(nn.tau, cap) : -1.0f;
+    float tau_max = INFINITY;
+    W.query()[lane] = make_float4(qx, qy, qz, tau);
     int l = __ldg(&st->top_level);
     const int top = l;
     uint32_t first = 0;                                       // the current siblings: [first, first + 32) of level l,
@@ -761,9 +813,10 @@ __device__ __forceinline__ void walk(TopK<K, EXACT>& tk, int& bc, WS& W, int lan
         const bool valid = first + lane < __ldg(&st->level_count[l]);
         const SNode* n = group + (valid ? lane : 0);
         const float4 lo = __ldg(&n->lo), hi = __ldg(&n->hi);
-        const float gx = fmaxf(fmaxf(__fsub_rn(lo.x, hx), __fsub_rn(lx, hi.x)), 0.0f);
-        const float gy = fmaxf(fmaxf(__fsub_rn(lo.y, hy), __fsub_rn(ly, hi.y)), 0.0f);
-        const float gz = fmaxf(fmaxf(__fsub_rn(lo.z, hz), __fsub_rn(lz, hi.z)), 0.0f);
+        const float4 ql = W.box_lo, qh = W.box_hi;
+        const float gx = fmaxf(fmaxf(__fsub_rn(lo.x, qh.x), __fsub_rn(ql.x, hi.x)), 0.0f);
+        const float gy = fmaxf(fmaxf(__fsub_rn(lo.y, qh.y), __fsub_rn(ql.y, hi.y)), 0.0f);
+        const float gz = fmaxf(fmaxf(__fsub_rn(lo.z, qh.z), __fsub_rn(ql.z, hi.z)), 0.0f);
         float d = __fmaf_rn(gx, gx, __fmaf_rn(gy, gy, __fmul_rn(gz, gz)));
         bool reach = valid && d <= tau_max;
         if (__popc(__ballot_sync(FULL, reach)) > kMaxLoose) {
@@ -773,10 +826,9 @@ __device__ __forceinline__ void walk(TopK<K, EXACT>& tk, int& bc, WS& W, int lan
             reach = false;
 #pragma unroll 1
             for (int i = 0; i < 32; ++i) {
-                const float xi = __shfl_sync(FULL, qx, i), yi = __shfl_sync(FULL, qy, i), zi = __shfl_sync(FULL, qz, i);
-                const float ti = __shfl_sync(FULL, tau, i);
-                const float di = box_dist2(xi, yi, zi, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z);
-                if (di <= ti) {
+                const float4 o = W.query()[i];
+                const float di = box_dist2(o.x, o.y, o.z, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z);
+                if (di <= o.w) {
                     d = fminf(d, di);
                     reach = valid;
                 }
@@ -784,71 +836,107 @@ __device__ __forceinline__ void walk(TopK<K, EXACT>& tk, int& bc, WS& W, int lan
         }
         return reach ? (__float_as_uint(d) & ~31u) | (uint32_t)lane : kNone;
     };
-    uint32_t key = order_key();
-    ++steps;
+    uint32_t key = kNone;
+    int32_t next = w0;        // the window's next run
+    bool started = false;     // the root's children are in `key`
     for (;;) {
-        const uint32_t m = __reduce_min_sync(FULL, key);
-        if (m == kNone || __uint_as_float(m & ~31u) > tau_max) {  // nothing left here: up a level
-            if (l == top) break;
-            ++l;
-            first = (first / kFan) & ~31u;
-            group = snodes + __ldg(&st->level_off[l]) + first;
-            key = W.level_keys(l)[lane];
-            continue;
-        }
-        if (key == m) key = kNone;
-        const float4 lo = __ldg(&group[m & 31u].lo), hi = __ldg(&group[m & 31u].hi);
-        const float d = box_dist2(qx, qy, qz, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z);
-        const bool need = d <= tau;
-        const uint32_t needm = __ballot_sync(FULL, need);
-        if (!needm) continue;
-        if (l > 0) {
-            if (++steps > step_cap) {
-                if (lane == 0) set_err(&st->err, ERRBIT_SEARCH_LIMIT);
+        int32_t f = 0, cnt = 0;
+        uint32_t needm = FULL;
+        const bool window = next < w1;
+        if (window) {
+            f = next;
+            cnt = min(32, w1 - f);
+            next += 32;
+        } else {
+            if (!started) {
+                started = true;
+                // nothing beyond the window: the tree has no more to offer
+                if (w0 > 0 || w1 < u) {
+                    tau_max = warp_max(tau);
+                    W.query()[lane].w = tau;
+                    __syncwarp();
+                    key = order_key();
+                    ++steps;
+                }
+            }
+            // the next leaf that some lane needs
+            for (;;) {
+                const uint32_t m = __reduce_min_sync(FULL, key);
+                if (m == kNone || __uint_as_float(m & ~31u) > tau_max) {  // nothing left here: up a level
+                    if (l == top) break;
+                    ++l;
+                    first = (first / kFan) & ~31u;
+                    group = snodes + __ldg(&st->level_off[l]) + first;
+                    key = W.level_keys(l)[lane];
+                    continue;
+                }
+                if (key == m) key = kNone;
+                const float4 lo = __ldg(&group[m & 31u].lo), hi = __ldg(&group[m & 31u].hi);
+                const float d = box_dist2(qx, qy, qz, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z);
+                needm = __ballot_sync(FULL, d <= tau);
+                if (!needm) continue;
+                if (l > 0) {
+                    if (++steps > step_cap) {
+                        if (lane == 0) set_err(&st->err, ERRBIT_SEARCH_LIMIT);
+                        break;
+                    }
+                    W.level_keys(l)[lane] = key;
+                    --l;
+                    first = (first + (m & 31u)) * kFan;
+                    group = snodes + __ldg(&st->level_off[l]) + first;
+                    key = order_key();
+                    continue;
+                }
+                f = __float_as_int(lo.w);
+                if (f >= w0 && f + __float_as_int(hi.w) <= w1) continue;  // all of it was in the window
+                cnt = __float_as_int(hi.w);
+                if (cnt < 1 || cnt > kLeafMax || (uint32_t)f > (uint32_t)u - (uint32_t)cnt) {
+                    if (lane == 0) set_err(&st->err, ERRBIT_BOUNDS);
+                    cnt = 0;
+                }
                 break;
             }
-            W.level_keys(l)[lane] = key;
-            --l;
-            first = (first + (m & 31u)) * kFan;
-            group = snodes + __ldg(&st->level_off[l]) + first;
-            key = order_key();
-            continue;
+            ct.buckets += cnt > 0;
         }
-        const int32_t f = __float_as_int(lo.w), cnt = __float_as_int(hi.w);
-        if (cnt < 1 || cnt > kLeafMax || (uint32_t)f > (uint32_t)u - (uint32_t)cnt) {
-            if (lane == 0) set_err(&st->err, ERRBIT_BOUNDS);
-            break;
-        }
-        if (f >= sw0 && f + cnt <= sw1) continue;  // all of it was in the seed window
-        ++ct.buckets;
-        if (__any_sync(FULL, bc + cnt > kBuf)) {
-            flush(tk, bc, W, lane, ct, pts, qx, qy, qz);
-            tau = act ? fminf(tk.tau(), cap) : -1.0f;
+        const bool done = cnt == 0;
+        const float before = tau;
+        uint32_t hits = 0;
+        if (!done)
+            hits = scan_run(f, cnt, needm, window ? e0 : w0, window ? e1 : w1, q, tau, W, lane, pts);
+        take_hits<K, EXACT>(
+            hits, done || (window && next >= w1),
+            [&](int i, int32_t& idx) {
+                const float* c = reinterpret_cast<const float*>(W.pts);
+                const int o = 4 * (i >> 1) + (i & 1);
+                idx = f + i;
+                return make_float3(c[o], c[o + 2], c[64 + i]);
+            },
+            nn, q, tau, cap, W, lane, ct);
+        __syncwarp();
+        if (done) break;
+        if (__any_sync(FULL, tau != before)) {
             tau_max = warp_max(tau);
+            W.query()[lane].w = tau;
+            __syncwarp();
         }
-        if (3 * __popc(needm) < 2 * cnt)
-            scan_sparse(f, cnt, needm, qx, qy, qz, tau, bc, W, pts, (int32_t)sw0, (int32_t)sw1, lane);
-        else
-            scan_chunk(f, cnt, need, qx, qy, qz, tau, bc, W, pts, (int32_t)sw0, (int32_t)sw1, lane);
     }
-    __syncwarp();
 }
 
-// The 32 queries [q0, q0 + 32) of one warp: search, then the outputs.
+// The queries [q0, q0 + warp_queries) of one warp: search, then the outputs.
 // CELLS: the learned attempt may run the cell scan (a separate instantiation,
 // launched only when the caller turned the cell scan on: compiled into the
 // default kernels, its code alone slowed them by about 8%).
 template <int K, bool EXACT, bool EXT, bool NORMALS, bool CELLS>
 __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const SNode* __restrict__ snodes,
                                          const uint64_t* __restrict__ codes, const QArgs& a, DevState* st,
-                                         int64_t q0, WarpSmem<KnnCfg<K>::buf>& W, int lane) {
+                                         int64_t q0, WarpSmem<KnnCfg<K>::buf, CELLS>& W, int lane) {
     constexpr int kBuf = KnnCfg<K>::buf;
-    static_assert(K <= kBuf, "the neighbour list is staged in the candidate buffer");
+    static_assert(K + 8 <= kBuf, "k candidates and room for hits");
     const int64_t u = a.device_count ? (int64_t)st->u : a.u;
     const int64_t count = a.device_count ? u : a.count;
     if (q0 >= count) return;  // whole warp
     const int64_t qo = q0 + lane;
-    const bool active = qo < count;
+    const bool active = lane < a.warp_queries && qo < count;
     float qx, qy, qz;
     int64_t center;  // tree index of the warp's first query (or its code position)
     if (EXT) {
@@ -879,11 +967,10 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
         center = a.start + q0;
     }
     const int64_t w0 = max64(0, center - a.seed_halo);
-    const int64_t w1 = min64(u, center + 32 + a.seed_halo);
-    const int S = (int)(w1 - w0);
+    const int64_t w1 = min64(u, center + (EXT ? 32 : a.warp_queries) + a.seed_halo);
 
-    TopK<K, EXACT> tk;
-    tk.init(a.k);
+    Nearest<K, EXACT> nn;
+    Query q{qx, qy, qz, a.k, 0, 0};
     Counters ct;
     uint32_t steps = 0;
     // With a learned radius, attempt 0 searches with the predicted bound as a
@@ -892,99 +979,105 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
     const bool learned = a.learned_r2 != nullptr;
     const float cap0 = (learned && active) ? __ldg(a.learned_r2 + qo) : INFINITY;
     bool act = active;
+    nn.init();
     for (int attempt = learned ? 0 : 1; attempt < 2; ++attempt) {
         const float cap = attempt == 0 ? cap0 : INFINITY;
         const bool seed = attempt == 1 || !a.learned_skip_seed;
         const int64_t sw0 = seed ? w0 : 0, sw1 = seed ? w1 : 0;  // points offered by the seed
-        if (act) tk.init(a.k);
-        int bc = 0;  // buffered candidates of this lane
-        // learned attempt as a cell scan (falls back to the capped tree walk)
-        const bool scanned = CELLS && attempt == 0 && a.cell_lut != nullptr &&
-                             cell_scan<K, EXACT>(tk, bc, W, lane, ct, pts, codes, a, st, act,
-                                                 a.start + (active ? qo : q0), qx, qy, qz, cap);
-        __syncwarp();
-        if (seed) {
-            // Seed: each lane walks the Morton window outwards from its own
-            // position (0, +1, -1, +2, ...), so its first candidates are its
-            // index neighbours.
-            __syncwarp();
-            for (int i = lane; i < S; i += 32) W.pts[i] = __ldg(pts + w0 + i);
-            __syncwarp();
-            const int p = EXT ? (int)(center + 16 - w0) : (int)(center + lane - w0);
-            const int reach = max(p, S - 1 - p);
-            const int nsteps = 2 * (int)__reduce_max_sync(FULL, (unsigned)(act ? reach : 0)) + 1;
-            // the first K spiral candidates fill the list directly, then one sort
-            if (act) {
-#pragma unroll
-                for (int t = 0; t < K; ++t) {
-                    const int off = (t & 1) ? (t + 1) >> 1 : -(t >> 1);
-                    const int iw = p + off;
-                    unsigned long long kv = kEmptyKey;
-                    if (iw >= 0 && iw < S) {
-                        const float4 q = W.pts[iw];
-                        kv = pack_key(dist2(qx, qy, qz, q.x, q.y, q.z), w0 + iw);
-                    }
-                    tk.key[t] = kv;
-                }
-                tk.sort_filled();
-            }
-            // the rest of the window in runs of at most kBuf steps (a step
-            // buffers at most one point per lane), one merge after each run
-            float tau = fminf(tk.tau(), cap);
-            int t = K;
-            do {
-                const int lim = min(nsteps, t + kBuf);
-                for (; t < lim; ++t) {
-                    const int off = (t & 1) ? (t + 1) >> 1 : -(t >> 1);
-                    const int iw = p + off;
-                    if (act && iw >= 0 && iw < S) {
-                        const float4 q = W.pts[iw];
-                        if (dist2(qx, qy, qz, q.x, q.y, q.z) <= tau) W.buf[bc++][lane] = (int32_t)(w0 + iw);
-                    }
-                }
-                flush(tk, bc, W, lane, ct, pts, qx, qy, qz);
-                tau = fminf(tk.tau(), cap);
-            } while (t < nsteps);
+        if (act) {
+            nn.init();
+            q.n = q.merged = 0;
         }
-
-        if (!scanned && (sw0 > 0 || sw1 < u))
-            walk<K, EXACT>(tk, bc, W, lane, ct, pts, snodes, a, st, act, qx, qy, qz, cap, u, sw0, sw1, steps);
-        flush(tk, bc, W, lane, ct, pts, qx, qy, qz);
+        // learned attempt as a cell scan (falls back to the capped tree walk)
+        bool scanned = false;
+        if constexpr (CELLS)
+            scanned = attempt == 0 && a.cell_lut != nullptr &&
+                      cell_scan<K, EXACT>(nn, q, W, lane, ct, pts, codes, a, st, act, a.start + (active ? qo : q0),
+                                          cap);
+        __syncwarp();
+        int32_t e0 = 0, e1 = 0;
+        if (seed && act) {
+            // Seed: K points of the Morton window around the lane's own
+            // position fill its list; the search offers the rest of the window.
+            const int64_t at = EXT ? center + 16 : center + lane;
+            e0 = (int32_t)max64(w0, min64(at - (K / 2 - 1), w1 - K));
+            e1 = (int32_t)min64(w1, e0 + K);
+#pragma unroll
+            for (int t = 0; t < K; ++t) {
+                nn.d[t] = INFINITY;
+                if (e0 + t < e1) {
+                    const float4 p = __ldg(pts + e0 + t);
+                    nn.d[t] = dist2(qx, qy, qz, p.x, p.y, p.z);
+                    W.d[t][lane] = nn.d[t];
+                    W.idx[t][lane] = e0 + t;
+                }
+            }
+            nn.sort_filled(a.k);
+            q.n = q.merged = e1 - e0;
+            ct.cand += q.n;
+            if (cap < INFINITY) {  // those beyond a learned cap do not count
+#pragma unroll
+                for (int t = 0; t < K; ++t) ct.cand -= nn.d[t] > cap && nn.d[t] < INFINITY;
+            }
+        }
+        if (!scanned)
+            search<K, EXACT>(nn, q, W, lane, ct, pts, snodes, a, st, act, cap, (int32_t)u, (int32_t)sw0, (int32_t)sw1, e0,
+                             e1, steps);
+        else
+            merge_fresh(nn, q, W, lane, ct);
         if (attempt == 0) {
             // a lane the cell scan could not serve (its cap is +inf or not a
             // number) was offered nothing: search it again as a miss
             const bool unserved = scanned && !(cap >= 0.0f && cap < INFINITY);
-            const bool miss = act && (unserved || !(tk.tau() <= cap));
+            const bool miss = act && (unserved || !(nn.tau <= cap));
             ct.lmiss += miss;
             act = miss;
             if (!__any_sync(FULL, act)) break;
         }
     }
+    if (__any_sync(FULL, q.n > K)) prune(q, nn.tau, K, W, lane, ct);
     {
         const unsigned cand = __reduce_add_sync(FULL, (unsigned)ct.cand);
         const unsigned ins = __reduce_add_sync(FULL, (unsigned)ct.ins);
         const unsigned lmiss = __reduce_add_sync(FULL, (unsigned)ct.lmiss);
         if (lane == 0) {
-            if (ct.cells) atomicAdd(&st->counters[CNT_CELL_WARPS], (unsigned long long)ct.cells);
-            if (ct.cell_fallback) atomicAdd(&st->counters[CNT_CELL_FALLBACK], (unsigned long long)ct.cell_fallback);
-            if (ct.cell_lookups) atomicAdd(&st->counters[CNT_CELL_LOOKUPS], (unsigned long long)ct.cell_lookups);
-            if (ct.cell_points) atomicAdd(&st->counters[CNT_CELL_POINTS], (unsigned long long)ct.cell_points);
-            atomicAdd(&st->counters[CNT_NODES], (unsigned long long)steps);
-            atomicAdd(&st->counters[CNT_BUCKETS], (unsigned long long)ct.buckets);
-            atomicAdd(&st->counters[CNT_MERGE], (unsigned long long)ct.merge);
-            atomicAdd(&st->counters[CNT_CANDIDATES], (unsigned long long)cand);
-            atomicAdd(&st->counters[CNT_INSERTS], (unsigned long long)ins);
-            if (lmiss) atomicAdd(&st->counters[CNT_LEARNED_MISS], (unsigned long long)lmiss);
+            W.count[CNT_NODES] += steps;
+            W.count[CNT_BUCKETS] += ct.buckets;
+            W.count[CNT_MERGE] += ct.merge;
+            W.count[CNT_CANDIDATES] += cand;
+            W.count[CNT_INSERTS] += ins;
+            W.count[CNT_LEARNED_MISS] += lmiss;
+            if constexpr (CELLS) {
+                W.count[CNT_CELL_WARPS] += ct.cells;
+                W.count[CNT_CELL_FALLBACK] += ct.cell_fallback;
+                W.count[CNT_CELL_LOOKUPS] += ct.cell_lookups;
+                W.count[CNT_CELL_POINTS] += ct.cell_points;
+            }
         }
     }
     if (!active) return;
 
+    // A query with a NaN coordinate is near nothing: it gets points of its
+    // window, at distance NaN.
+    const bool lost = q.n == 0;
+    if (lost)
+        for (; q.n < K && w0 + q.n < w1; ++q.n) {
+            W.d[q.n][lane] = INFINITY;
+            W.idx[q.n][lane] = (int32_t)(w0 + q.n);
+        }
+    // the k nearest in the lists' order: by distance, then by index
+    unsigned long long key[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        key[j] = j < q.n ? pack_key(W.d[j][lane], W.idx[j][lane]) : kEmptyKey;
+    }
+    sort_values(key);
     // fewer than k points in the tree: repeat entry 0 (src/Octree.hpp:181-191)
     int32_t nbr[K];
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-        if (j > 0 && tk.key[j] == kEmptyKey) tk.key[j] = tk.key[0];
-        nbr[j] = key_idx(tk.key[j]);
+        if (j > 0 && key[j] == kEmptyKey) key[j] = key[0];
+        nbr[j] = key_idx(key[j]);
     }
     if (a.out_idx) {
         int32_t* o = a.out_idx + qo * a.k;
@@ -996,25 +1089,40 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
         float* o = a.out_d2 + qo * a.k;
 #pragma unroll
         for (int j = 0; j < K; ++j)
-            if (j < a.k) o[j] = key_d(tk.key[j]);
+            if (j < a.k) o[j] = lost ? __int_as_float(0x7fc00000) : key_d(key[j]);
     }
     if (NORMALS) {
 #pragma unroll
-        for (int j = 0; j < K; ++j) W.buf[j][lane] = nbr[j];  // this lane's column only
-        estimate_normal(&W.buf[0][lane], a.k, pts, qx, qy, qz, a, a.out_normals + 3 * qo, st);
+        for (int j = 0; j < K; ++j) W.idx[j][lane] = nbr[j];  // this lane's column only
+        estimate_normal(&W.idx[0][lane], a.k, pts, qx, qy, qz, a, a.out_normals + 3 * qo, st);
     }
 }
 
+// Persistent: the grid is the resident blocks and each warp takes its next
+// queries from a counter. With a block per four warps' queries a block kept its
+// registers and shared memory until its slowest warp ended, and 15 of 20
+// resident warps were active on average: the 2M scene's k = 16 search took
+// 2.68 ms, 2.35 ms persistent.
 template <int K, bool EXACT, bool EXT, bool NORMALS, bool CELLS>
 __global__ void __launch_bounds__(KnnCfg<K>::threads, KnnCfg<K>::min_blocks)
     k_knn(const float4* __restrict__ pts, const SNode* __restrict__ snodes,
                                                      const uint64_t* __restrict__ codes, QArgs a, DevState* st) {
     extern __shared__ __align__(16) unsigned char knn_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    using WS = WarpSmem<KnnCfg<K>::buf>;
+    using WS = WarpSmem<KnnCfg<K>::buf, CELLS>;
     WS& W = reinterpret_cast<WS*>(knn_smem)[warp];
-    const int64_t q0 = ((int64_t)blockIdx.x * KnnCfg<K>::warps + warp) * 32;
-    knn_warp<K, EXACT, EXT, NORMALS, CELLS>(pts, snodes, codes, a, st, q0, W, lane);
+    if (lane < kQueryCounters) W.count[lane] = 0;
+    __syncwarp();
+    const int64_t n = a.device_count ? (int64_t)st->u : a.count;
+    const uint32_t items = (uint32_t)((n + a.warp_queries - 1) / a.warp_queries);
+    uint32_t item = blockIdx.x * KnnCfg<K>::warps + warp;
+    while (item < items) {
+        knn_warp<K, EXACT, EXT, NORMALS, CELLS>(pts, snodes, codes, a, st, (int64_t)item * a.warp_queries, W, lane);
+        __syncwarp();
+        if (lane == 0) item = gridDim.x * KnnCfg<K>::warps + atomicAdd(&st->work, 1u);
+        item = __shfl_sync(FULL, item, 0);
+    }
+    if (lane < kQueryCounters && W.count[lane]) atomicAdd(&st->counters[lane], (unsigned long long)W.count[lane]);
 }
 
 // Persistent kernel over many clouds that share k: each warp takes the next
@@ -1040,6 +1148,8 @@ __global__ void __launch_bounds__(BatchCfg<K, NW>::threads, BatchCfg<K, NW>::min
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     using WS = WarpSmem<KnnCfg<K>::buf>;
     WS& W = reinterpret_cast<WS*>(knn_smem)[warp];
+    if (lane < kQueryCounters) W.count[lane] = 0;
+    __syncwarp();
     for (;;) {
         unsigned long long item = 0;
         if (lane == 0) item = atomicAdd(counter, 1ull);
@@ -1059,31 +1169,41 @@ __global__ void __launch_bounds__(BatchCfg<K, NW>::threads, BatchCfg<K, NW>::min
         knn_warp<K, EXACT, false, true, false>(d.pts, d.snodes, nullptr, ca, d.st, ((int64_t)item - d.item0) * 32,
                                                W, lane);
         __syncwarp();
+        if (lane < kQueryCounters && W.count[lane]) {
+            atomicAdd(&d.st->counters[lane], (unsigned long long)W.count[lane]);
+            W.count[lane] = 0;
+        }
+        __syncwarp();
     }
 }
 
 template <int K, bool EXACT, bool EXT, bool NORMALS, bool CELLS = false>
-cudaError_t launch_one(const BuildBufs& b, const QArgs& a, unsigned blocks, cudaStream_t s) {
-    constexpr int smem = (int)sizeof(WarpSmem<KnnCfg<K>::buf>) * KnnCfg<K>::warps;
+cudaError_t launch_one(const BuildBufs& b, const QArgs& a, unsigned blocks, cudaStream_t s, int num_sms) {
+    constexpr int smem = (int)sizeof(WarpSmem<KnnCfg<K>::buf, CELLS>) * KnnCfg<K>::warps;
     cudaError_t e = cudaFuncSetAttribute(k_knn<K, EXACT, EXT, NORMALS, CELLS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_knn<K, EXACT, EXT, NORMALS, CELLS>, KnnCfg<K>::threads, smem);
+    if (e != cudaSuccess) return e;
+    const unsigned resident = (unsigned)(per_sm > 0 ? per_sm : 1) * (unsigned)num_sms;
+    if (blocks > resident) blocks = resident;
     k_knn<K, EXACT, EXT, NORMALS, CELLS><<<blocks, KnnCfg<K>::threads, smem, s>>>(b.pts4, b.snodes, b.codes, a,
                                                                                    b.st);
     return cudaGetLastError();
 }
 
 template <int K, bool EXACT>
-cudaError_t launch_k(const BuildBufs& b, const QArgs& a, bool ext, bool normals, cudaStream_t s) {
-    const int64_t warps = (a.count + 31) / 32;
+cudaError_t launch_k(const BuildBufs& b, const QArgs& a, bool ext, bool normals, cudaStream_t s, int num_sms) {
+    const int64_t warps = (a.count + a.warp_queries - 1) / a.warp_queries;
     const unsigned blocks = (unsigned)((warps + KnnCfg<K>::warps - 1) / KnnCfg<K>::warps);
-    if (ext) return launch_one<K, EXACT, true, false>(b, a, blocks, s);
+    if (ext) return launch_one<K, EXACT, true, false>(b, a, blocks, s, num_sms);
     if (a.cell_lut) {
-        if (normals) return launch_one<K, EXACT, false, true, true>(b, a, blocks, s);
-        return launch_one<K, EXACT, false, false, true>(b, a, blocks, s);
+        if (normals) return launch_one<K, EXACT, false, true, true>(b, a, blocks, s, num_sms);
+        return launch_one<K, EXACT, false, false, true>(b, a, blocks, s, num_sms);
     }
-    if (normals) return launch_one<K, EXACT, false, true>(b, a, blocks, s);
-    return launch_one<K, EXACT, false, false>(b, a, blocks, s);
+    if (normals) return launch_one<K, EXACT, false, true>(b, a, blocks, s, num_sms);
+    return launch_one<K, EXACT, false, false>(b, a, blocks, s, num_sms);
 }
 
 template <int K, bool EXACT, int NW>
@@ -1171,6 +1291,7 @@ cudaError_t enqueue_query_batch(const BatchCloud* clouds, int n_clouds, int64_t 
     a.code_bits = q.code_bits;
     a.seed_halo = q.seed_halo < 0 ? 0 : (q.seed_halo > kMaxHalo ? kMaxHalo : q.seed_halo);
     a.device_count = 1;
+    a.warp_queries = 32;
     const int bps = q.batch_blocks_per_sm, wpb = q.batch_warps_per_block;
     switch (q.k) {
         case 8: return launch_batch<8, true>(clouds, n_clouds, n_items, counter, a, s, num_sms, bps, wpb);
@@ -1187,7 +1308,7 @@ cudaError_t enqueue_query_batch(const BatchCloud* clouds, int n_clouds, int64_t 
     return launch_batch<32, false>(clouds, n_clouds, n_items, counter, a, s, num_sms, bps, wpb);
 }
 
-cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t s, int /*num_sms*/) {
+cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t s, int num_sms) {
     if (q.count <= 0) return cudaSuccess;
     if (q.k < 1 || q.k > 32) return cudaErrorInvalidValue;
     if (q.compat) return enqueue_query_compat(b, q, s);
@@ -1216,21 +1337,32 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     a.cell_span = q.cell_span < 2 ? 2 : (q.cell_span > 4 ? 4 : q.cell_span);
     if (a.seed_halo > kMaxHalo) a.seed_halo = kMaxHalo;
     if (a.seed_halo < 0) a.seed_halo = 0;
+    // Few queries: fewer per warp, down to one, until there are ten warps per
+    // SM. 32 queries of one warp mostly wait for one another (the union of
+    // their nodes, the longest of their lists), and a small call lasts as long
+    // as one warp: 2k points, k = 8, 74 us with 32 queries per warp and 39 us
+    // with one; 10k points, k = 16, 162 and 115 us (eight per warp). With 20
+    // warps per SM as the aim the wider spread costs more than it shortens
+    // (10k points 141 us, 40k points 230 against 197 us); from 48k points on
+    // every choice is 32.
+    a.warp_queries = 32;
+    while (a.warp_queries > 1 && (q.count + a.warp_queries - 1) / a.warp_queries < (int64_t)10 * num_sms)
+        a.warp_queries /= 2;
     const bool ext = q.ext_queries != nullptr;
     const bool nrm = q.out_normals != nullptr && !ext;
     switch (q.k) {
-        case 8: return launch_k<8, true>(b, a, ext, nrm, s);
-        case 10: return launch_k<10, true>(b, a, ext, nrm, s);
-        case 16: return launch_k<16, true>(b, a, ext, nrm, s);
-        case 32: return launch_k<32, true>(b, a, ext, nrm, s);
+        case 8: return launch_k<8, true>(b, a, ext, nrm, s, num_sms);
+        case 10: return launch_k<10, true>(b, a, ext, nrm, s, num_sms);
+        case 16: return launch_k<16, true>(b, a, ext, nrm, s, num_sms);
+        case 32: return launch_k<32, true>(b, a, ext, nrm, s, num_sms);
         default: break;
     }
-    if (q.k <= 4) return launch_k<4, false>(b, a, ext, nrm, s);
-    if (q.k <= 8) return launch_k<8, false>(b, a, ext, nrm, s);
-    if (q.k <= 12) return launch_k<12, false>(b, a, ext, nrm, s);
-    if (q.k <= 16) return launch_k<16, false>(b, a, ext, nrm, s);
-    if (q.k <= 24) return launch_k<24, false>(b, a, ext, nrm, s);
-    return launch_k<32, false>(b, a, ext, nrm, s);
+    if (q.k <= 4) return launch_k<4, false>(b, a, ext, nrm, s, num_sms);
+    if (q.k <= 8) return launch_k<8, false>(b, a, ext, nrm, s, num_sms);
+    if (q.k <= 12) return launch_k<12, false>(b, a, ext, nrm, s, num_sms);
+    if (q.k <= 16) return launch_k<16, false>(b, a, ext, nrm, s, num_sms);
+    if (q.k <= 24) return launch_k<24, false>(b, a, ext, nrm, s, num_sms);
+    return launch_k<32, false>(b, a, ext, nrm, s, num_sms);
 }
 
 }  // namespace shapex

@@ -59,6 +59,7 @@ struct DevState {
     uint32_t level_count[kMaxLevels];
     // query counters, in the order of se_stats
     unsigned long long counters[kQueryCounters];
+    uint32_t work;  // next work item of a persistent search launch
 };
 
 // Byte layout of OT::OTNode (reference src/Octree.hpp:19-36), 56 bytes.

@@ -48,3 +48,64 @@ def test_lists_exact_on_every_level_count(native, oracle, shape, bucket):
             ei, ed = oracle.knn_exact(p, p, k)
             assert np.array_equal(idx, ei), (shape, bucket, n)
             assert np.array_equal(d2, ed), (shape, bucket, n)
+
+
+def _shell(scale=2097151):
+    """Integer points at one exact distance from a centre, as many as there
+    are, and a few nearer ones: coordinates that the 21-bit code round trip
+    keeps, corner points that pin the range."""
+    f = np.float32
+    v = np.arange(0, 400).astype(f)
+    code = np.floor(f(scale) * (v / f(scale))).astype(np.int64)
+    back = (code.astype(f) / f(scale)).astype(np.float64) * scale
+    kept = set(np.flatnonzero(back.astype(f) == v).tolist())
+    c = np.array([200, 200, 200])
+    r = np.arange(-40, 41)
+    o = np.stack(np.meshgrid(r, r, r), -1).reshape(-1, 3)
+    o = o[np.array([all(int(t) in kept for t in p) for p in c + o])]
+    n2 = (o**2).sum(1)
+    best = np.bincount(n2[(n2 > 500) & (n2 < 1500)]).argmax()
+    pts = np.concatenate([c + o[n2 == best], c + o[(n2 > 0) & (n2 <= 3)], [c], [[0, 0, 0]], [[scale] * 3]])
+    return pts.astype(np.float32), int((n2 == best).sum())
+
+
+@pytest.mark.parametrize("k", [1, 8, 10, 16, 24, 30, 32])
+def test_more_ties_at_the_bound_than_slots(native, oracle, k):
+    pts, ties = _shell()
+    assert ties > 60  # more than any list keeps slots for
+    x, y, z = (np.ascontiguousarray(a) for a in pts.T)
+    with native.Context() as c:
+        c.build(x, y, z)
+        p = c.points()
+        idx, d2 = c.knn_self(k, with_d2=True)
+        ei, ed = oracle.knn_exact(p, p, k)
+        assert np.array_equal(d2, ed)
+        assert np.array_equal(idx, ei)
+
+
+def test_nan_queries_get_points_of_the_tree(native, oracle):
+    rng = np.random.default_rng(3)
+    x, y, z = rng.random((3, 5_000)).astype(np.float32)
+    q = rng.random((100, 3)).astype(np.float32)
+    q[::7, 1] = np.nan
+    with native.Context() as c:
+        c.build(x, y, z)
+        idx, d2 = c.knn(q, 9, with_d2=True)
+        p = c.points()
+    assert idx.min() >= 0 and idx.max() < len(p)
+    ok = np.isfinite(q).all(1)
+    assert np.isnan(d2[~ok]).all()
+    ei, ed = oracle.knn_exact(p, q[ok], 9)
+    assert np.array_equal(idx[ok], ei) and np.array_equal(d2[ok], ed)
+
+
+@pytest.mark.parametrize("n", [319, 740, 1_481, 2_959, 3_001, 11_840, 11_841, 23_681])
+def test_few_queries_per_warp(native, oracle, n):
+    """Counts on both sides of each halving of the queries per warp."""
+    rng = np.random.default_rng(n)
+    x, y, z = rng.random((3, n)).astype(np.float32)
+    with native.Context(build_octree=False) as c:
+        c.build(x, y, z)
+        p = c.points()
+        assert np.array_equal(c.knn_self(16), oracle.knn_exact(p, p, 16)[0])
+        assert np.array_equal(c.knn_self(16, 5, 301), oracle.knn_exact(p, p[5:306], 16)[0])
