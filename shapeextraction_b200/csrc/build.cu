@@ -150,7 +150,8 @@ __global__ void __launch_bounds__(256) k_encode(const float* __restrict__ x, con
 }
 
 // Digit offsets, trivial-pass detection and ping-pong parity, on one block.
-__global__ void __launch_bounds__(kSortBins) k_sort_prep(int64_t n, DevState* st) {
+// With first < last only passes [first, last) run, all of them.
+__global__ void __launch_bounds__(kSortBins) k_sort_prep(int64_t n, DevState* st, int first = 0, int last = 0) {
     __shared__ uint32_t s_w[kSortBins / 32 + 1];
     __shared__ int s_triv[kSortPasses];
     const int d = threadIdx.x;
@@ -167,9 +168,10 @@ __global__ void __launch_bounds__(kSortBins) k_sort_prep(int64_t n, DevState* st
     if (d == 0) {
         int act = 0;
         for (int p = 0; p < kSortPasses; ++p) {
-            st->pass_active[p] = !s_triv[p];
+            const bool run = first < last ? p >= first && p < last : !s_triv[p];
+            st->pass_active[p] = run;
             st->pass_parity[p] = act & 1;
-            act += !s_triv[p];
+            act += run;
         }
         st->n_active = act;
     }
@@ -957,6 +959,30 @@ __global__ void __launch_bounds__(256) k_copy_if_odd(const uint64_t* __restrict_
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = src[i];
 }
 
+// Order keys of foreign queries (their places by binary search over the
+// tree's codes) and the digit histograms of the passes that sort them.
+__global__ void __launch_bounds__(256) k_query_keys(const float* __restrict__ q, int64_t n,
+                                                    const uint64_t* __restrict__ codes, int64_t u, int code_bits,
+                                                    int shift, int first, uint64_t* __restrict__ keys,
+                                                    const DevState* tree, DevState* st) {
+    __shared__ uint32_t s_h[kSortPasses][kSortBins];
+    for (int i = threadIdx.x; i < kSortPasses * kSortBins; i += blockDim.x) (&s_h[0][0])[i] = 0;
+    __syncthreads();
+    const float mn = tree->min_coord, range = tree->range;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
+        const uint64_t code = query_to_code(q[3 * i], q[3 * i + 1], q[3 * i + 2], mn, range, code_bits);
+        const uint64_t k = ((uint64_t)code_position(codes, u, code) << (shift + kOrderShift)) | (uint64_t)i;
+        keys[i] = k;
+        for (int p = first; p < kSortPasses - 1; ++p) atomicAdd(&s_h[p][(k >> (kSortBits * p)) & (kSortBins - 1)], 1u);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kSortPasses * kSortBins; i += blockDim.x) {
+        const uint32_t v = (&s_h[0][0])[i];
+        if (v) atomicAdd(&(&st->hist[0][0])[i], v);
+    }
+}
+
 inline unsigned grid_for(int64_t work, int threads, int64_t cap_blocks) {
     int64_t b = (work + threads - 1) / threads;
     if (b < 1) b = 1;
@@ -992,6 +1018,33 @@ cudaError_t enqueue_sort_keys(uint64_t* keys, uint64_t* tmp, int64_t n, uint32_t
                                                                                  kSpinLimit, 0);
     }
     k_copy_if_odd<<<grid_for(n, 256, num_sms * 4), 256, 0, s>>>(tmp, keys, n, st);
+    return cudaGetLastError();
+}
+
+cudaError_t enqueue_query_order(const BuildBufs& b, const QueryOrder& o, const float* queries, int64_t n, int64_t u,
+                                int code_bits, const uint64_t** order, int* shift, cudaStream_t s, int num_sms,
+                                int* launches) {
+    cudaError_t e = set_onesweep_attributes();
+    if (e != cudaSuccess) return e;
+    int bits = 1;  // places are in [0, u]
+    while (((int64_t)1 << bits) <= u) ++bits;
+    *shift = bits < 30 ? 30 - bits : 0;
+    // A warp takes 32 queries, so a place need only be right to a few queries:
+    // the top 18 bits up to 2M queries, 27 above (bits 45..62, 36..62).
+    const int passes = n <= ((int64_t)1 << 21) ? 2 : 3;
+    const int first = kSortPasses - 1 - passes;
+    cudaMemsetAsync(o.st, 0, sizeof(DevState), s);
+    k_query_keys<<<grid_for(n, 256, num_sms * 4), 256, 0, s>>>(queries, n, b.codes, u, code_bits, *shift, first, o.keys0,
+                                                               b.st, o.st);
+    k_sort_prep<<<1, kSortBins, 0, s>>>(n, o.st, first, kSortPasses - 1);
+    const int64_t tiles = (n + kSortTile - 1) / kSortTile;
+    for (int pass = first; pass < kSortPasses - 1; ++pass) {
+        cudaMemsetAsync(o.lookback, 0, sizeof(uint32_t) * kSortBins * tiles, s);
+        k_onesweep<<<(unsigned)tiles, kSortThreads, sizeof(SortSmem), s>>>(o.keys0, o.keys1, n, pass, o.lookback, o.st,
+                                                                            kSpinLimit, 0);
+    }
+    *order = passes & 1 ? o.keys1 : o.keys0;
+    *launches += 2 + passes;
     return cudaGetLastError();
 }
 

@@ -217,6 +217,21 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
             q.ext_queries = ext;
         }
     }
+    // Foreign queries come in any order; a warp's 32 share a walk only if they
+    // lie close together, so they are taken in the order of their places in the
+    // tree. With one query per warp there is nothing to share. (250k queries
+    // near a 2M-point scene, k = 8, in random order: 21.0 ms as given, 0.93 ms
+    // with the sort, which takes about 70 us of it.)
+    const bool sorted = ext && !q.compat && queries_per_warp(count, c->num_sms, true) > 1;
+    if (sorted && c->q_order_cap < count) {
+        QueryOrder& o = c->q_order;
+        c->q_order_cap = 0;
+        if (!o.st) SE_CUDA(c, cudaMalloc(&o.st, sizeof(DevState)), "alloc query order");
+        SE_CUDA(c, regrow(o.keys0, count), "alloc query order");
+        SE_CUDA(c, regrow(o.keys1, count), "alloc query order");
+        SE_CUDA(c, regrow(o.lookback, (count + kSortTile - 1) / kSortTile * kSortBins), "alloc query order");
+        c->q_order_cap = count;
+    }
     // Pinned host outputs are written by the kernel itself (mapped host
     // memory), so the results cross PCIe while the kernel runs instead of in
     // a copy after it. Other host outputs go through device staging.
@@ -266,6 +281,11 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
         SE_CUDA(c, enqueue_predict_radius(c->b, c->mlp, c->mlp_margin, u, c->opt.code_bits, start, count, c->r2_buf,
                                           nullptr, c->stream),
                 "launch radius prediction");
+    int order_launches = 0;
+    if (sorted)
+        SE_CUDA(c, enqueue_query_order(c->b, c->q_order, q.ext_queries, count, u, c->opt.code_bits, &q.order,
+                                       &q.order_shift, c->stream, c->num_sms, &order_launches),
+                "order queries");
     SE_CUDA(c, enqueue_query(c->b, q, c->stream, c->num_sms), "launch query");
     SE_CUDA(c, cudaEventRecord(c->query_ev[1], c->stream), "event");
     if (host) {
@@ -280,16 +300,21 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
                                        c->stream),
                     "copy normals");
     }
-    c->query_launches = (use_learned ? 2 : 1) + (lut_launched ? 1 : 0);
+    c->query_launches = (use_learned ? 2 : 1) + (lut_launched ? 1 : 0) + order_launches;
     c->have_query_times = true;
     SE_CUDA(c, cudaMemcpyAsync(&c->h_st->err, &c->b.st->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
             "read state");
+    c->h_st->pad0 = 0;
+    if (sorted)  // the error word of the queries' sort
+        SE_CUDA(c, cudaMemcpyAsync(&c->h_st->pad0, &c->q_order.st->err, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                   c->stream),
+                "read state");
     SE_CUDA(c, cudaMemcpyAsync(c->h_st->counters, c->b.st->counters, sizeof(c->b.st->counters),
                                cudaMemcpyDeviceToHost, c->stream),
             "read state");
     SE_CUDA(c, cudaStreamSynchronize(c->stream), "synchronize");
     for (int i = 0; i < kQueryCounters; ++i) c->last_counters[i] = (int64_t)c->h_st->counters[i];
-    return check_err_bits(c, c->h_st->err);
+    return check_err_bits(c, c->h_st->err | c->h_st->pad0);
 }
 
 }  // namespace
@@ -402,6 +427,9 @@ int se_destroy(se_ctx* c) {
     if (c->idx_buf) cudaFree(c->idx_buf);
     if (c->d2_buf) cudaFree(c->d2_buf);
     if (c->q_buf) cudaFree(c->q_buf);
+    void* obufs[] = {c->q_order.keys0, c->q_order.keys1, c->q_order.lookback, c->q_order.st};
+    for (void* p : obufs)
+        if (p) cudaFree(p);
     float* mlp_bufs[] = {c->mlp, c->mlp_m, c->mlp_v, c->mlp_g, c->mlp_loss, c->r2_buf, c->xs_buf,
                          c->mw.yhat, c->mw.h1, c->mw.h2, c->mw.dy, c->mw.dh1, c->mw.dh2};
     for (float* p : mlp_bufs)

@@ -68,6 +68,27 @@ __device__ __forceinline__ uint64_t point_to_code(float x, float y, float z, flo
     return spread3(xc & bs) | (spread3(yc & bs) << 1) | (spread3(zc & bs) << 2);
 }
 
+// Morton code of a foreign query: pointToCode with the coordinates clamped to
+// the tree's cube (a NaN goes to its low corner).
+__device__ __forceinline__ uint64_t query_to_code(float x, float y, float z, float mn, float range, int code_bits) {
+    const float fbs = (float)bitscale_of(code_bits);
+    auto cell = [&](float v) {
+        const float f = __fmul_rn(fbs, __fdiv_rn(__fsub_rn(v, mn), range));
+        return __float2uint_rz(fminf(fmaxf(f, 0.0f), fbs));
+    };
+    return spread3(cell(x)) | (spread3(cell(y)) << 1) | (spread3(cell(z)) << 2);
+}
+// First index in codes[0, u) whose code is >= code (u when none).
+__device__ __forceinline__ int64_t code_position(const uint64_t* __restrict__ codes, int64_t u, uint64_t code) {
+    int64_t lo = 0, hi = u;
+    while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (__ldg(codes + mid) < code) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
 // codeToPoint (reference src/MortonUtils.cu:21-29), with the FMA nvcc forms there.
 __device__ __forceinline__ float3 code_to_point(uint64_t code, float mn, float range, int code_bits) {
     const float fbs = (float)bitscale_of(code_bits);

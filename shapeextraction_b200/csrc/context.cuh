@@ -56,6 +56,8 @@ struct se_ctx {
     int32_t* idx_buf = nullptr;
     float* d2_buf = nullptr;
     float* q_buf = nullptr;
+    QueryOrder q_order{};       // order of foreign queries
+    int64_t q_order_cap = 0;
     DevState* h_st = nullptr;   // pinned mirror of the device state
 
     bool built = false;

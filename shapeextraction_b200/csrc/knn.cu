@@ -206,7 +206,10 @@ struct QArgs {
     float* out_d2;
     float* out_normals;
     const float* learned_r2;
-    const uint32_t* cell_lut;  // learned cell scan: code-range table (null: tree walk with the cap)
+    union {
+        const uint32_t* cell_lut;  // learned cell scan: code-range table (null: tree walk with the cap)
+        const uint64_t* order;     // foreign queries: their order (null: as given)
+    };
     float vx, vy, vz;
     float gap;
     int k;
@@ -215,7 +218,10 @@ struct QArgs {
     int learned_skip_seed;
     int device_count;  // 1: u = count = the build's unique-point count, read on the device (start 0)
     int step_limit;    // > 0: node visits per warp before the walk gives up (test hook)
-    int lut_shift;     // per-axis shift of the table's level (bits per axis - level)
+    union {
+        int lut_shift;    // per-axis shift of the table's level (bits per axis - level)
+        int order_shift;  // scale of the places in `order`
+    };
     int cell_pmax;     // cell scan: most points per warp before it falls back to the walk
     int cell_span;     // cell scan: most cells per axis covering one lane's ball (2..4)
     int warp_queries;  // queries per warp, 1..32
@@ -843,6 +849,7 @@ __device__ __forceinline__ void search(Nearest<K, EXACT>& nn, Query& q, WS& W, i
         int32_t f = 0, cnt = 0;
         uint32_t needm = FULL;
         const bool window = next < w1;
+        const bool own = window || w0 == w1;  // the lane's own [e0, e1) were offered so far, not the window
         if (window) {
             f = next;
             cnt = min(32, w1 - f);
@@ -888,7 +895,7 @@ __device__ __forceinline__ void search(Nearest<K, EXACT>& nn, Query& q, WS& W, i
                     continue;
                 }
                 f = __float_as_int(lo.w);
-                if (f >= w0 && f + __float_as_int(hi.w) <= w1) continue;  // all of it was in the window
+                if (f >= w0 && f + __float_as_int(hi.w) <= w1) continue;  // all of it was in the window (none: w1 = 0)
                 cnt = __float_as_int(hi.w);
                 if (cnt < 1 || cnt > kLeafMax || (uint32_t)f > (uint32_t)u - (uint32_t)cnt) {
                     if (lane == 0) set_err(&st->err, ERRBIT_BOUNDS);
@@ -902,7 +909,7 @@ __device__ __forceinline__ void search(Nearest<K, EXACT>& nn, Query& q, WS& W, i
         const float before = tau;
         uint32_t hits = 0;
         if (!done)
-            hits = scan_run(f, cnt, needm, window ? e0 : w0, window ? e1 : w1, q, tau, W, lane, pts);
+            hits = scan_run(f, cnt, needm, own ? e0 : w0, own ? e1 : w1, q, tau, W, lane, pts);
         take_hits<K, EXACT>(
             hits, done || (window && next >= w1),
             [&](int i, int32_t& idx) {
@@ -938,27 +945,24 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
     const int64_t qo = q0 + lane;
     const bool active = lane < a.warp_queries && qo < count;
     float qx, qy, qz;
-    int64_t center;  // tree index of the warp's first query (or its code position)
+    int64_t center;   // tree index of the warp's first query; foreign queries: the lane's place among the codes
+    int64_t row = qo;  // of the outputs
     if (EXT) {
-        const int64_t src = active ? qo : q0;
-        qx = __ldg(a.ext + 3 * src);
-        qy = __ldg(a.ext + 3 * src + 1);
-        qz = __ldg(a.ext + 3 * src + 2);
-        const float lx = __shfl_sync(FULL, qx, 0), ly = __shfl_sync(FULL, qy, 0), lz = __shfl_sync(FULL, qz, 0);
-        const float mn = st->min_coord, range = st->range;
-        const float fbs = (float)bitscale_of(a.code_bits);
-        auto q1 = [&](float v) {
-            float f = __fmul_rn(fbs, __fdiv_rn(__fsub_rn(v, mn), range));
-            f = fminf(fmaxf(f, 0.0f), fbs);
-            return __float2uint_rz(f);
-        };
-        const uint64_t code = spread3(q1(lx)) | (spread3(q1(ly)) << 1) | (spread3(q1(lz)) << 2);
-        int64_t lo = 0, hi = u;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (__ldg(codes + mid) < code) lo = mid + 1; else hi = mid;
+        row = active ? qo : q0;
+        uint64_t key = 0;
+        if (a.order) {
+            key = __ldg(a.order + row);
+            row = (int64_t)(key & ((1u << 30) - 1));
+            if (row >= count) {  // the sort failed
+                set_err(&st->err, ERRBIT_BOUNDS);
+                row = q0;
+            }
         }
-        center = lo - 16;
+        qx = __ldg(a.ext + 3 * row);
+        qy = __ldg(a.ext + 3 * row + 1);
+        qz = __ldg(a.ext + 3 * row + 2);
+        center = a.order ? min64(u, (int64_t)(key >> (kOrderShift + a.order_shift)))
+                         : code_position(codes, u, query_to_code(qx, qy, qz, st->min_coord, st->range, a.code_bits));
     } else {
         const float4 p = __ldg(pts + a.start + (active ? qo : q0));
         qx = p.x;
@@ -966,8 +970,16 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
         qz = p.z;
         center = a.start + q0;
     }
-    const int64_t w0 = max64(0, center - a.seed_halo);
-    const int64_t w1 = min64(u, center + (EXT ? 32 : a.warp_queries) + a.seed_halo);
+    // the seed window: the warp's. Sorted foreign queries can lie far apart, so
+    // there each lane only fills its list around its own place; unsorted ones
+    // come one to a warp, with a window around that.
+    const bool lone = EXT && a.order != nullptr;
+    int64_t w0 = 0, w1 = u;
+    if (!lone) {
+        const int64_t from = EXT ? __shfl_sync(FULL, center, 0) - 16 : center;
+        w0 = max64(0, from - a.seed_halo);
+        w1 = min64(u, from + (EXT ? 32 : a.warp_queries) + a.seed_halo);
+    }
 
     Nearest<K, EXACT> nn;
     Query q{qx, qy, qz, a.k, 0, 0};
@@ -983,7 +995,7 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
     for (int attempt = learned ? 0 : 1; attempt < 2; ++attempt) {
         const float cap = attempt == 0 ? cap0 : INFINITY;
         const bool seed = attempt == 1 || !a.learned_skip_seed;
-        const int64_t sw0 = seed ? w0 : 0, sw1 = seed ? w1 : 0;  // points offered by the seed
+        const int64_t sw0 = seed && !lone ? w0 : 0, sw1 = seed && !lone ? w1 : 0;  // points offered by the seed
         if (act) {
             nn.init();
             q.n = q.merged = 0;
@@ -999,7 +1011,7 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
         if (seed && act) {
             // Seed: K points of the Morton window around the lane's own
             // position fill its list; the search offers the rest of the window.
-            const int64_t at = EXT ? center + 16 : center + lane;
+            const int64_t at = EXT ? center : center + lane;
             e0 = (int32_t)max64(w0, min64(at - (K / 2 - 1), w1 - K));
             e1 = (int32_t)min64(w1, e0 + K);
 #pragma unroll
@@ -1080,13 +1092,13 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
         nbr[j] = key_idx(key[j]);
     }
     if (a.out_idx) {
-        int32_t* o = a.out_idx + qo * a.k;
+        int32_t* o = a.out_idx + row * a.k;
 #pragma unroll
         for (int j = 0; j < K; ++j)
             if (j < a.k) o[j] = nbr[j];
     }
     if (a.out_d2) {
-        float* o = a.out_d2 + qo * a.k;
+        float* o = a.out_d2 + row * a.k;
 #pragma unroll
         for (int j = 0; j < K; ++j)
             if (j < a.k) o[j] = lost ? __int_as_float(0x7fc00000) : key_d(key[j]);
@@ -1308,6 +1320,24 @@ cudaError_t enqueue_query_batch(const BatchCloud* clouds, int n_clouds, int64_t 
     return launch_batch<32, false>(clouds, n_clouds, n_items, counter, a, s, num_sms, bps, wpb);
 }
 
+int queries_per_warp(int64_t count, int num_sms, bool foreign) {
+    // Few queries: fewer per warp, down to one, until there are ten warps per
+    // SM. 32 queries of one warp mostly wait for one another (the union of
+    // their nodes, the longest of their lists), and a small call lasts as long
+    // as one warp: 2k points, k = 8, 74 us with 32 queries per warp and 39 us
+    // with one; 10k points, k = 16, 162 and 115 us (eight per warp). With 20
+    // warps per SM as the aim the wider spread costs more than it shortens
+    // (10k points 141 us, 40k points 230 against 197 us); from 48k points on
+    // every choice is 32.
+    // Foreign queries share less, and until they are two to a warp they need not
+    // be sorted: 60 warps per SM (10k queries in a 2M-point precision mix, k = 8
+    // and 32: 345 and 597 us at 10 per SM, 122 and 360 us at 60; 60k: 609 and
+    // 1072, 532 and 1115; at 120 k = 32 loses: 1314).
+    int per = 32;
+    while (per > 1 && (count + per - 1) / per < (int64_t)(foreign ? 60 : 10) * num_sms) per /= 2;
+    return per;
+}
+
 cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t s, int num_sms) {
     if (q.count <= 0) return cudaSuccess;
     if (q.k < 1 || q.k > 32) return cudaErrorInvalidValue;
@@ -1331,23 +1361,18 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     a.learned_skip_seed = q.learned_skip_seed;
     a.device_count = q.device_count;
     a.step_limit = q.step_limit;
-    a.cell_lut = q.learned_r2 ? q.cell_lut : nullptr;
-    a.lut_shift = q.lut_shift;
+    if (q.ext_queries) {
+        a.order = q.order;
+        a.order_shift = q.order_shift;
+    } else {
+        a.cell_lut = q.learned_r2 ? q.cell_lut : nullptr;
+        a.lut_shift = q.lut_shift;
+    }
     a.cell_pmax = q.cell_pmax;
     a.cell_span = q.cell_span < 2 ? 2 : (q.cell_span > 4 ? 4 : q.cell_span);
     if (a.seed_halo > kMaxHalo) a.seed_halo = kMaxHalo;
     if (a.seed_halo < 0) a.seed_halo = 0;
-    // Few queries: fewer per warp, down to one, until there are ten warps per
-    // SM. 32 queries of one warp mostly wait for one another (the union of
-    // their nodes, the longest of their lists), and a small call lasts as long
-    // as one warp: 2k points, k = 8, 74 us with 32 queries per warp and 39 us
-    // with one; 10k points, k = 16, 162 and 115 us (eight per warp). With 20
-    // warps per SM as the aim the wider spread costs more than it shortens
-    // (10k points 141 us, 40k points 230 against 197 us); from 48k points on
-    // every choice is 32.
-    a.warp_queries = 32;
-    while (a.warp_queries > 1 && (q.count + a.warp_queries - 1) / a.warp_queries < (int64_t)10 * num_sms)
-        a.warp_queries /= 2;
+    a.warp_queries = queries_per_warp(q.count, num_sms, q.ext_queries != nullptr);
     const bool ext = q.ext_queries != nullptr;
     const bool nrm = q.out_normals != nullptr && !ext;
     switch (q.k) {

@@ -189,12 +189,33 @@ cudaError_t enqueue_adam(float* params, const float* grads, float* m, float* v, 
 cudaError_t enqueue_sort_keys(uint64_t* keys, uint64_t* tmp, int64_t n, uint32_t* lookback, DevState* st,
                               cudaStream_t s, int num_sms);
 
+// Foreign queries in the order of their places among the tree's codes: keys
+// hold the place (30 bits, scaled to the top of them) from bit kOrderShift up
+// and the query's number in the low 30 bits, sorted by as many of the place's
+// leading bits as the number of queries calls for.
+constexpr int kOrderShift = 33;
+struct QueryOrder {
+    uint64_t* keys0;
+    uint64_t* keys1;
+    uint32_t* lookback;  // kSortBins words per 4096-key tile
+    DevState* st;
+};
+// *order receives the sorted keys (keys0 or keys1), *shift the scale of the
+// places, *launches the number of kernels launched.
+cudaError_t enqueue_query_order(const BuildBufs& b, const QueryOrder& o, const float* queries, int64_t n, int64_t u,
+                                int code_bits, const uint64_t** order, int* shift, cudaStream_t s, int num_sms,
+                                int* launches);
+// Queries per warp of a search of `count` queries.
+int queries_per_warp(int64_t count, int num_sms, bool foreign);
+
 struct QueryParams {
     int k;
     int64_t start;      // first query (self queries)
     int64_t count;      // number of queries
     int64_t u;          // tree points
     const float* ext_queries;  // AoS xyz external queries or nullptr (self queries)
+    const uint64_t* order = nullptr;  // external queries: their order (enqueue_query_order), or nullptr: as given
+    int order_shift = 0;
     int32_t* out_idx;   // count*k or nullptr
     float* out_d2;      // count*k or nullptr
     float* out_normals; // count*3 or nullptr

@@ -109,3 +109,27 @@ def test_few_queries_per_warp(native, oracle, n):
         p = c.points()
         assert np.array_equal(c.knn_self(16), oracle.knn_exact(p, p, 16)[0])
         assert np.array_equal(c.knn_self(16, 5, 301), oracle.knn_exact(p, p[5:306], 16)[0])
+
+
+@pytest.mark.parametrize("k", [1, 8, 16, 31])
+@pytest.mark.parametrize("shape", ["uniform", "far_pairs"])
+def test_foreign_queries_in_any_order(native, oracle, shape, k):
+    """Counts on both sides of the rule that sorts them; queries inside, on and
+    far outside the tree's cube, and repeated ones; host and device memory."""
+    import torch
+
+    rng = np.random.default_rng(17)
+    x, y, z = np.ascontiguousarray(SHAPES[shape](rng, 40_000).astype(np.float32).T)
+    with native.Context() as c:
+        c.build(x, y, z)
+        p = c.points()
+        for n in (1, 33, 3_000, 17_759, 17_761, 40_001):
+            q = rng.random((n, 3)).astype(np.float32)
+            q[::5] = p[rng.integers(0, len(p), len(q[::5]))]
+            q[::11] = q[0]
+            q[::13] *= 3.0
+            ei, ed = oracle.knn_exact(p, q, k)
+            idx, d2 = c.knn(q, k, with_d2=True)
+            assert np.array_equal(idx, ei) and np.array_equal(d2, ed), n
+            ti = c.knn(torch.from_numpy(q).cuda(), k)
+            assert np.array_equal(ti.cpu().numpy(), ei), n
