@@ -118,15 +118,59 @@ __device__ __forceinline__ void load_bbox(const DevState* st, float& mn, float& 
     range = __fsub_rn(mx, mn);  // float tree_range = max - min, src/RadixTree.cu:246
 }
 
+// Digit offsets, trivial-pass detection and ping-pong parity, by one block of
+// NT threads (kSortBins / NT adjacent digits each). With first < last only
+// passes [first, last) run, all of them; otherwise those of the first `passes`
+// whose digits are not all equal.
+template <int NT>
+__device__ __forceinline__ void sort_prep(int64_t n, int passes, DevState* st, int first, int last) {
+    constexpr int kPer = kSortBins / NT;
+    __shared__ uint32_t s_w[NT / 32 + 1];
+    __shared__ int s_triv[kSortPasses];
+    for (int p = 0; p < passes; ++p) {
+        uint32_t h[kPer], sum = 0, tot;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            h[i] = __ldcg(&st->hist[p][kPer * threadIdx.x + i]);
+            sum += h[i];
+        }
+        uint32_t ex = block_excl_scan<NT, uint32_t>(sum, s_w, &tot);
+        if (threadIdx.x == 0) s_triv[p] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            st->digit_off[p][kPer * threadIdx.x + i] = ex;
+            ex += h[i];
+            if ((int64_t)h[i] == n) s_triv[p] = 1;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        int act = 0;
+        for (int p = 0; p < kSortPasses; ++p) {
+            const bool run = first < last ? p >= first && p < last : p < passes && !s_triv[p];
+            st->pass_active[p] = run;
+            st->pass_parity[p] = act & 1;
+            act += run;
+        }
+        st->n_active = act;
+    }
+}
+__global__ void __launch_bounds__(kSortBins) k_sort_prep(int64_t n, DevState* st, int first = 0, int last = 0) {
+    sort_prep<kSortBins>(n, kSortPasses, st, first, last);
+}
+
 // ---------------------------------------------------------------------------
 // encode: replaces makeCodes (src/RadixTree.cu:21-39, 244-248); also builds
-// the digit histograms of the onesweep sort's passes in the same pass.
+// the digit histograms of the onesweep sort's passes in the same pass, and its
+// last block to finish prepares the passes.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_encode(const float* __restrict__ x, const float* __restrict__ y,
-                                                const float* __restrict__ z, int64_t n, int code_bits,
+                                                const float* __restrict__ z, int64_t n, int code_bits, int passes,
                                                 uint64_t* __restrict__ keys, DevState* st) {
-    __shared__ uint32_t s_h[kSortPasses][kSortBins];
-    for (int i = threadIdx.x; i < kSortPasses * kSortBins; i += blockDim.x) (&s_h[0][0])[i] = 0;
+    __shared__ uint32_t s_h[kCodePasses][kSortBins];
+    __shared__ bool s_last;
+    for (int i = threadIdx.x; i < passes * kSortBins; i += blockDim.x) (&s_h[0][0])[i] = 0;
     __syncthreads();
     float mn, range;
     load_bbox(st, mn, range);
@@ -140,41 +184,21 @@ __global__ void __launch_bounds__(256) k_encode(const float* __restrict__ x, con
         const uint64_t c = point_to_code(__ldcs(x + i), __ldcs(y + i), __ldcs(z + i), mn, range, code_bits);
         keys[i] = c;
 #pragma unroll
-        for (int p = 0; p < kSortPasses; ++p) atomicAdd(&s_h[p][(c >> (kSortBits * p)) & (kSortBins - 1)], 1u);
+        for (int p = 0; p < kCodePasses; ++p)
+            if (p < passes) atomicAdd(&s_h[p][(c >> (kSortBits * p)) & (kSortBins - 1)], 1u);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kSortPasses * kSortBins; i += blockDim.x) {
+    for (int i = threadIdx.x; i < passes * kSortBins; i += blockDim.x) {
         const uint32_t v = (&s_h[0][0])[i];
         if (v) atomicAdd(&(&st->hist[0][0])[i], v);
     }
-}
-
-// Digit offsets, trivial-pass detection and ping-pong parity, on one block.
-// With first < last only passes [first, last) run, all of them.
-__global__ void __launch_bounds__(kSortBins) k_sort_prep(int64_t n, DevState* st, int first = 0, int last = 0) {
-    __shared__ uint32_t s_w[kSortBins / 32 + 1];
-    __shared__ int s_triv[kSortPasses];
-    const int d = threadIdx.x;
-    for (int p = 0; p < kSortPasses; ++p) {
-        const uint32_t h = st->hist[p][d];
-        uint32_t tot;
-        const uint32_t ex = block_excl_scan<kSortBins, uint32_t>(h, s_w, &tot);
-        st->digit_off[p][d] = ex;
-        if (d == 0) s_triv[p] = 0;
-        __syncthreads();
-        if ((int64_t)h == n) s_triv[p] = 1;
-        __syncthreads();
-    }
-    if (d == 0) {
-        int act = 0;
-        for (int p = 0; p < kSortPasses; ++p) {
-            const bool run = first < last ? p >= first && p < last : !s_triv[p];
-            st->pass_active[p] = run;
-            st->pass_parity[p] = act & 1;
-            act += run;
-        }
-        st->n_active = act;
-    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&st->tile_counter[kSortPasses + 3], 1u) + 1 == gridDim.x;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    sort_prep<256>(n, passes, st, 0, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -422,6 +446,171 @@ __global__ void __launch_bounds__(kDedupThreads) k_dedup(const uint64_t* buf0, c
 }
 
 // ---------------------------------------------------------------------------
+// Front of the build for small clouds: bbox, encode, sort, dedup and decode (as
+// the kernels above) in one block, keys in shared memory. A small build is a
+// chain of launches whose kernels have little to do; this one replaces eleven
+// of them and three memsets (it clears the state and scratch itself). Up to 8192
+// points, what 1024 threads hold at 8 keys each: these stages took 126 us on
+// 2011 points and take 33 us (whole build 199 and 84 us); at 8192 points the
+// whole build takes 136 us, with the separate kernels 180 us.
+// IPT keys per thread; element order is warp by warp, so ranking by warps is
+// stable. Slots past n hold all ones and stay last.
+// ---------------------------------------------------------------------------
+constexpr int kFrontThreads = 1024;
+constexpr int kFrontWarps = kFrontThreads / 32;
+static_assert(kFrontMax == 8 * kFrontThreads, "8 keys per thread");
+
+template <int IPT>
+struct FrontSmem {
+    uint64_t keys[IPT * kFrontThreads];
+    uint32_t hist[kFrontWarps][kSortBins];
+    uint32_t start[kSortBins];
+    uint32_t scan_w[kFrontWarps + 1];
+    float lo[kFrontWarps], hi[kFrontWarps];
+    uint32_t diff_lo[kFrontWarps], diff_hi[kFrontWarps];
+    uint32_t cnt[kFrontWarps];
+    int bad;
+};
+
+template <int IPT>
+__global__ void __launch_bounds__(kFrontThreads) k_front(const float* __restrict__ x, const float* __restrict__ y,
+                                                         const float* __restrict__ z, int n, int code_bits,
+                                                         uint64_t* __restrict__ codes_out, float4* __restrict__ pts4,
+                                                         float* __restrict__ pts3, uint32_t* __restrict__ scratch,
+                                                         int scratch_words, DevState* st) {
+    constexpr unsigned kFull = 0xffffffffu;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    FrontSmem<IPT>& S = *reinterpret_cast<FrontSmem<IPT>*>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < scratch_words; i += kFrontThreads) scratch[i] = 0;
+    // the state up to the sort's histograms, which nothing reads here
+    for (int i = tid; i < (int)(offsetof(DevState, hist) / 4); i += kFrontThreads) reinterpret_cast<uint32_t*>(st)[i] = 0;
+    if (tid == 0) S.bad = 0;
+    const int base = warp * 32 * IPT + lane;
+    float px[IPT], py[IPT], pz[IPT];
+    float lo = FLT_MAX, hi = -FLT_MAX;
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+        const int e = base + 32 * i;
+        if (e < n) {
+            px[i] = x[e];
+            py[i] = y[e];
+            pz[i] = z[e];
+            lo = fminf(lo, fminf(px[i], fminf(py[i], pz[i])));
+            hi = fmaxf(hi, fmaxf(px[i], fmaxf(py[i], pz[i])));
+            bad |= !(isfinite(px[i]) && isfinite(py[i]) && isfinite(pz[i]));
+        }
+    }
+    lo = warp_min(lo);
+    hi = warp_max(hi);
+    if (lane == 0) {
+        S.lo[warp] = lo;
+        S.hi[warp] = hi;
+    }
+    __syncthreads();  // S.bad is clear, the state is clear
+    if (bad) S.bad = 1;
+    lo = warp_min(S.lo[lane]);
+    hi = warp_max(S.hi[lane]);
+    const float mn = lo, range = __fsub_rn(hi, lo);
+    uint64_t key[IPT];
+    uint64_t diff = 0;
+    const uint64_t key0 = point_to_code(x[0], y[0], z[0], mn, range, code_bits);
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+        key[i] = ~0ull;
+        if (base + 32 * i < n) {
+            key[i] = point_to_code(px[i], py[i], pz[i], mn, range, code_bits);
+            diff |= key[i] ^ key0;
+        }
+        S.keys[base + 32 * i] = key[i];
+    }
+    // digits in which no two keys differ need no pass
+    const uint32_t dl = __reduce_or_sync(kFull, (uint32_t)diff), dh = __reduce_or_sync(kFull, (uint32_t)(diff >> 32));
+    if (lane == 0) {
+        S.diff_lo[warp] = dl;
+        S.diff_hi[warp] = dh;
+    }
+    __syncthreads();
+    diff = ((uint64_t)__reduce_or_sync(kFull, S.diff_hi[lane]) << 32) | __reduce_or_sync(kFull, S.diff_lo[lane]);
+    for (int shift = 0; shift < code_bits; shift += kSortBits) {
+        if (!((diff >> shift) & (kSortBins - 1))) continue;
+        for (int i = tid; i < kFrontWarps * kSortBins; i += kFrontThreads) (&S.hist[0][0])[i] = 0;
+        __syncthreads();
+        uint32_t rank[IPT];
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            const uint32_t d = (uint32_t)(key[i] >> shift) & (kSortBins - 1);
+            uint32_t peers = kFull;
+#pragma unroll
+            for (int bb = 0; bb < kSortBits; ++bb) {
+                const uint32_t v = __ballot_sync(kFull, (d >> bb) & 1u);
+                peers &= ((d >> bb) & 1u) ? v : ~v;
+            }
+            const uint32_t b = S.hist[warp][d];
+            __syncwarp();
+            if (lane == 31 - __clz(peers)) S.hist[warp][d] = b + __popc(peers);
+            __syncwarp();
+            rank[i] = b + __popc(peers & lanemask_lt());
+        }
+        __syncthreads();
+        uint32_t cnt = 0;
+        if (tid < kSortBins)
+            for (int w = 0; w < kFrontWarps; ++w) {
+                const uint32_t c = S.hist[w][tid];
+                S.hist[w][tid] = cnt;
+                cnt += c;
+            }
+        uint32_t tot;
+        const uint32_t at = block_excl_scan<kFrontThreads, uint32_t>(cnt, S.scan_w, &tot);
+        if (tid < kSortBins) S.start[tid] = at;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) {
+            const uint32_t d = (uint32_t)(key[i] >> shift) & (kSortBins - 1);
+            S.keys[S.start[d] + S.hist[warp][d] + rank[i]] = key[i];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < IPT; ++i) key[i] = S.keys[base + 32 * i];
+        __syncthreads();
+    }
+    // dedup and decode
+    uint32_t m[IPT], wcnt = 0;
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+        const int e = base + 32 * i;
+        m[i] = __ballot_sync(kFull, e < n && (e == 0 || S.keys[e - 1] != key[i]));
+        wcnt += __popc(m[i]);
+    }
+    if (lane == 0) S.cnt[warp] = wcnt;
+    __syncthreads();
+    const uint32_t c = S.cnt[lane];
+    const uint32_t inc = warp_incl_scan(c);
+    uint32_t pos = __shfl_sync(kFull, inc - c, warp);
+    if (tid == 0) {
+        st->min_coord = mn;
+        st->max_coord = hi;
+        st->range = range;
+        if (S.bad) st->err = ERRBIT_NONFINITE;
+    }
+    if (tid == 31) st->u = inc;
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+        if ((m[i] >> lane) & 1u) {
+            const uint32_t o = pos + __popc(m[i] & lanemask_lt());
+            const float3 p = code_to_point(key[i], mn, range, code_bits);
+            codes_out[o] = key[i];
+            pts4[o] = make_float4(p.x, p.y, p.z, 0.0f);
+            pts3[3 * o + 0] = p.x;
+            pts3[3 * o + 1] = p.y;
+            pts3[3 * o + 2] = p.z;
+        }
+        pos += __popc(m[i]);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Karras radix tree: replaces constructTree (src/RadixTree.cu:99-194,
 // launched at :351-364). One thread per internal node, same search steps and
 // integer semantics as the reference, so topology is bit-exact. Node 0 is
@@ -491,6 +680,9 @@ __global__ void __launch_bounds__(256) k_karras(const uint64_t* __restrict__ cod
     const int64_t u = (int64_t)st->u;
     const int64_t N = u - 1;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    // entries of `parent` that no node claims are 0: those of the root, of the
+    // last leaf's number, and, with the compat root, of the full root's children
+    if (i == N) parent[i] = 0;
     if (i >= N) return;
     const KNode f = karras_node(codes, i, N, code_bits, false);
     // full root range
@@ -503,20 +695,22 @@ __global__ void __launch_bounds__(256) k_karras(const uint64_t* __restrict__ cod
     prefix_n[i] = (uint8_t)e.dnode;
     hll[i] = e.hl;
     hlr[i] = e.hr;
-    // The compat root's parent claims are written after this kernel (k_root_parent)
+    // The compat root's parent claims are written after this kernel (by k_leaves)
     // so that, in a tree the compat root breaks, they win deterministically.
-    if (i != 0 || !root_compat) {
-        if (!e.hl) parent[e.gamma] = (int32_t)i;
-        if (!e.hr) parent[e.gamma + 1] = (int32_t)i;
-    }
+    if (!f.hl) parent[f.gamma] = (int32_t)i;
+    if (!f.hr) parent[f.gamma + 1] = (int32_t)i;
+    if (i == 0) parent[0] = 0;
 }
 
-__global__ void k_root_parent(const int32_t* __restrict__ left_child, int32_t* __restrict__ parent,
-                              const uint8_t* __restrict__ hll, const uint8_t* __restrict__ hlr, DevState* st) {
-    const int64_t u = (int64_t)st->u;
+__device__ __forceinline__ void root_parent(const int32_t* __restrict__ left_child, int32_t* __restrict__ parent,
+                                            const uint8_t* __restrict__ hll, const uint8_t* __restrict__ hlr,
+                                            int64_t u, DevState* st) {
     if (u < 2) return;
     const int32_t g = left_child[0];
-    if (g < 0 || g + 1 >= u) { set_err(&st->err, ERRBIT_BOUNDS); return; }
+    if (g < 0 || g + 1 >= u) {
+        set_err(&st->err, ERRBIT_BOUNDS);
+        return;
+    }
     if (!hll[0]) parent[g] = 0;
     if (!hlr[0]) parent[g + 1] = 0;
 }
@@ -544,7 +738,11 @@ __global__ void k_root_parent(const int32_t* __restrict__ left_child, int32_t* _
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kLeafThreads) k_leaves(const uint64_t* __restrict__ codes, int M,
                                                          int32_t* __restrict__ leaf_start,
-                                                         uint32_t* __restrict__ lookback, DevState* st,
+                                                         uint32_t* __restrict__ lookback, int root_compat,
+                                                         const int32_t* __restrict__ left_child,
+                                                         int32_t* __restrict__ parent,
+                                                         const uint8_t* __restrict__ hll,
+                                                         const uint8_t* __restrict__ hlr, DevState* st,
                                                          int spin_limit) {
     constexpr int kHalo = kLeafMax, kSpan = kLeafTile + 2 * kHalo;
     constexpr int kCells = kLeafIpt * kLeafThreads / 32;  // 32-code steps of a tile
@@ -560,6 +758,7 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaves(const uint64_t* __restr
     __syncthreads();
     const uint32_t tile = s_tile;
     const int64_t t0 = (int64_t)tile * kLeafTile;
+    if (root_compat && tile == 0 && tid == 0) root_parent(left_child, parent, hll, hlr, u, st);
     if (t0 >= u) return;
     for (int j = tid; j < kSpan; j += kLeafThreads) {
         const int64_t i = t0 - kHalo + j;
@@ -727,13 +926,14 @@ __global__ void __launch_bounds__(128) k_boxes(const float4* __restrict__ pts, c
 // ---------------------------------------------------------------------------
 // Octree: replaces calcEdgeCounts + InclusiveSum (src/Octree.cu:38-50,
 // 215-247) with one counting + decoupled look-back scan kernel writing the
-// exclusive offsets and the node total.
+// exclusive offsets and the node total, and zeroing the nodes.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kScanThreads) k_oct_scan(const uint8_t* __restrict__ prefix_n,
                                                            const int32_t* __restrict__ parent,
                                                            int32_t* __restrict__ counts,
                                                            int32_t* __restrict__ offsets,
                                                            unsigned long long* __restrict__ lookback,
+                                                           OtNode* __restrict__ nodes, int64_t cap,
                                                            DevState* st, int spin_limit) {
     __shared__ long long s_w[kScanThreads / 32 + 1];
     __shared__ uint32_t s_tile;
@@ -803,20 +1003,12 @@ __global__ void __launch_bounds__(kScanThreads) k_oct_scan(const uint8_t* __rest
         if (j <= N) offsets[j] = (int32_t)run;
         run += c[i];
     }
-}
-
-// Zero the node array (src/Octree.cu:250-253). The root's corner and size are
-// written by k_oct_make's thread 0 (src/Octree.cu:257-261).
-__global__ void __launch_bounds__(256) k_oct_zero(OtNode* __restrict__ nodes, int64_t cap, DevState* st) {
-    const int64_t m = (int64_t)st->n_oct;
-    if (m > cap) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) set_err(&st->err, ERRBIT_OCT_CAPACITY);
-        return;
-    }
-    uint2* w = reinterpret_cast<uint2*>(nodes);  // 56 B = 7 x 8 B per node
-    const int64_t words = m * 7;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < words; i += stride) w[i] = make_uint2(0u, 0u);
+    // zero the tile's own nodes (src/Octree.cu:250-253); the root's corner and
+    // size are written by k_oct_make (src/Octree.cu:257-261)
+    const long long z0 = s_excl < 0 ? 0 : s_excl, z1 = s_excl + tot < cap ? s_excl + tot : (long long)cap;
+    if (tid == 0 && s_excl + tot > cap) set_err(&st->err, ERRBIT_OCT_CAPACITY);
+    uint2* words = reinterpret_cast<uint2*>(nodes);  // 56 B = 7 x 8 B per node
+    for (long long w = 7 * z0 + tid; w < 7 * z1; w += kScanThreads) words[w] = make_uint2(0u, 0u);
 }
 
 __device__ __forceinline__ int64_t oct_walk_up(int64_t r, const int32_t* __restrict__ counts,
@@ -833,17 +1025,10 @@ __device__ __forceinline__ int64_t oct_walk_up(int64_t r, const int32_t* __restr
 // makeNodes, src/Octree.cu:114-161: each radix node emits its chain of
 // counts[i] octree nodes (deepest first) and links the chain's top under the
 // bottom node of its nearest contributing ancestor.
-__global__ void __launch_bounds__(256) k_oct_make(OtNode* __restrict__ nodes, int64_t cap,
-                                                  const int32_t* __restrict__ offsets,
-                                                  const int32_t* __restrict__ counts,
-                                                  const uint64_t* __restrict__ codes,
-                                                  const uint8_t* __restrict__ prefix_n,
-                                                  const int32_t* __restrict__ parent, int code_bits, DevState* st) {
-    const int64_t m = (int64_t)st->n_oct;
-    if (m > cap || m < 1) return;
-    const int64_t N = (int64_t)st->u - 1;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= N) return;
+__device__ __forceinline__ void make_chain(int64_t i, int64_t m, int64_t N, OtNode* __restrict__ nodes,
+                                           const int32_t* __restrict__ offsets, const int32_t* __restrict__ counts,
+                                           const uint64_t* __restrict__ codes, const uint8_t* __restrict__ prefix_n,
+                                           const int32_t* __restrict__ parent, int code_bits, DevState* st) {
     const float mn = st->min_coord, range = st->range;
     const int CL = code_bits;
     const int root_level = st->root_level;
@@ -899,7 +1084,31 @@ __global__ void __launch_bounds__(256) k_oct_make(OtNode* __restrict__ nodes, in
 
 // linkLeafNodes, src/Octree.cu:65-112: each leaf child of a radix node goes
 // into the bottom octree node of the nearest contributing ancestor.
-__global__ void __launch_bounds__(256) k_oct_link(OtNode* __restrict__ nodes, int64_t cap,
+__device__ __forceinline__ void link_leaves(int64_t i, int64_t m, int64_t u, OtNode* __restrict__ nodes,
+                                            const int32_t* __restrict__ offsets, const int32_t* __restrict__ counts,
+                                            const uint64_t* __restrict__ codes, const uint8_t* __restrict__ hll,
+                                            const uint8_t* __restrict__ hlr, const uint8_t* __restrict__ prefix_n,
+                                            const int32_t* __restrict__ parent,
+                                            const int32_t* __restrict__ left_child, int code_bits, DevState* st) {
+    const bool sides[2] = {hll[i] != 0, hlr[i] != 0};
+    if (!sides[0] && !sides[1]) return;
+    const int lvl = prefix_n[i] / 3 + 1;
+    const int64_t rn = oct_walk_up(i, counts, parent, u - 1, st);
+    if (rn < 0) return;
+    const int64_t node = offsets[rn];
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        if (!sides[side]) continue;
+        const int64_t leaf = (int64_t)left_child[i] + side;
+        if (leaf < 0 || leaf >= u || node < 0 || node >= m) { set_err(&st->err, ERRBIT_BOUNDS); continue; }
+        const uint64_t pre = shr_clamp(codes[leaf], code_bits - 3 * lvl);
+        nodes[node].children[pre & 7] = (int32_t)leaf;
+        atomicOr(&nodes[node].child_leaf_mask, 1 << (pre & 7));
+    }
+}
+
+// Both for radix node i: they write different children and masks.
+__global__ void __launch_bounds__(256) k_oct_make(OtNode* __restrict__ nodes, int64_t cap,
                                                   const int32_t* __restrict__ offsets,
                                                   const int32_t* __restrict__ counts,
                                                   const uint64_t* __restrict__ codes,
@@ -914,21 +1123,8 @@ __global__ void __launch_bounds__(256) k_oct_link(OtNode* __restrict__ nodes, in
     const int64_t N = u - 1;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= N) return;
-    const bool sides[2] = {hll[i] != 0, hlr[i] != 0};
-    if (!sides[0] && !sides[1]) return;
-    const int lvl = prefix_n[i] / 3 + 1;
-    const int64_t rn = oct_walk_up(i, counts, parent, N, st);
-    if (rn < 0) return;
-    const int64_t node = offsets[rn];
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {
-        if (!sides[side]) continue;
-        const int64_t leaf = (int64_t)left_child[i] + side;
-        if (leaf < 0 || leaf >= u || node < 0 || node >= m) { set_err(&st->err, ERRBIT_BOUNDS); continue; }
-        const uint64_t pre = shr_clamp(codes[leaf], code_bits - 3 * lvl);
-        nodes[node].children[pre & 7] = (int32_t)leaf;
-        atomicOr(&nodes[node].child_leaf_mask, 1 << (pre & 7));
-    }
+    if (m >= 1) make_chain(i, m, N, nodes, offsets, counts, codes, prefix_n, parent, code_bits, st);
+    link_leaves(i, m, u, nodes, offsets, counts, codes, hll, hlr, prefix_n, parent, left_child, code_bits, st);
 }
 
 // Digit histograms of given keys (the histogram half of k_encode), for
@@ -1038,31 +1234,54 @@ cudaError_t enqueue_query_order(const BuildBufs& b, const QueryOrder& o, const f
                                                                b.st, o.st);
     k_sort_prep<<<1, kSortBins, 0, s>>>(n, o.st, first, kSortPasses - 1);
     const int64_t tiles = (n + kSortTile - 1) / kSortTile;
-    for (int pass = first; pass < kSortPasses - 1; ++pass) {
-        cudaMemsetAsync(o.lookback, 0, sizeof(uint32_t) * kSortBins * tiles, s);
-        k_onesweep<<<(unsigned)tiles, kSortThreads, sizeof(SortSmem), s>>>(o.keys0, o.keys1, n, pass, o.lookback, o.st,
-                                                                            kSpinLimit, 0);
-    }
+    cudaMemsetAsync(o.lookback, 0, sizeof(uint32_t) * kSortBins * tiles * passes, s);
+    for (int pass = first; pass < kSortPasses - 1; ++pass)
+        k_onesweep<<<(unsigned)tiles, kSortThreads, sizeof(SortSmem), s>>>(
+            o.keys0, o.keys1, n, pass, o.lookback + kSortBins * tiles * (pass - first), o.st, kSpinLimit, 0);
     *order = passes & 1 ? o.keys1 : o.keys0;
     *launches += 2 + passes;
     return cudaGetLastError();
 }
 
-cudaError_t enqueue_octree(const BuildBufs& b, const BuildParams& p, cudaStream_t s, int num_sms, int* launches) {
+template <int IPT>
+static cudaError_t launch_front_n(const BuildBufs& b, int64_t n, int code_bits, const ScratchLayout& scratch,
+                                  cudaStream_t s) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_front<IPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FrontSmem<IPT>));
+    if (e != cudaSuccess) return e;
+    k_front<IPT><<<1, kFrontThreads, sizeof(FrontSmem<IPT>), s>>>(b.x, b.y, b.z, (int)n, code_bits, b.codes, b.pts4,
+                                                                  b.pts3, b.scratch, (int)scratch.sort, b.st);
+    return cudaGetLastError();
+}
+static cudaError_t launch_front(const BuildBufs& b, int64_t n, int code_bits, const ScratchLayout& scratch,
+                                cudaStream_t s) {
+    if (n <= kFrontThreads) return launch_front_n<1>(b, n, code_bits, scratch, s);
+    if (n <= 2 * kFrontThreads) return launch_front_n<2>(b, n, code_bits, scratch, s);
+    if (n <= 4 * kFrontThreads) return launch_front_n<4>(b, n, code_bits, scratch, s);
+    return launch_front_n<8>(b, n, code_bits, scratch, s);
+}
+
+// With `again` the scan's scratch is cleared first (a build starts with it clear).
+static cudaError_t launch_octree(const BuildBufs& b, const BuildParams& p, cudaStream_t s, bool again, int* launches) {
     const int64_t n = p.n;
     const int64_t scan_tiles = (n + kScanTile - 1) / kScanTile;
-    cudaMemsetAsync(b.lookback64, 0, sizeof(unsigned long long) * scan_tiles, s);
-    cudaMemsetAsync(&b.st->tile_counter[kSortPasses + 1], 0, sizeof(uint32_t), s);
-    k_oct_scan<<<(unsigned)scan_tiles, kScanThreads, 0, s>>>(b.prefix_n, b.parent, b.oct_counts, b.oct_offsets,
-                                                             b.lookback64, b.st, p.spin_limit);
-    k_oct_zero<<<grid_for(b.oct_cap * 7, 256, num_sms * 8), 256, 0, s>>>((OtNode*)b.oct_nodes, b.oct_cap, b.st);
-    k_oct_make<<<grid_for(n, 256, 0), 256, 0, s>>>((OtNode*)b.oct_nodes, b.oct_cap, b.oct_offsets, b.oct_counts,
-                                                   b.codes, b.prefix_n, b.parent, p.code_bits, b.st);
-    k_oct_link<<<grid_for(n, 256, 0), 256, 0, s>>>((OtNode*)b.oct_nodes, b.oct_cap, b.oct_offsets, b.oct_counts,
-                                                   b.codes, b.has_leaf_left, b.has_leaf_right, b.prefix_n, b.parent,
-                                                   b.left_child, p.code_bits, b.st);
-    if (launches) *launches += 4;
+    unsigned long long* lookback = reinterpret_cast<unsigned long long*>(b.scratch + ScratchLayout(n).oct);
+    if (again) {
+        cudaMemsetAsync(lookback, 0, sizeof(unsigned long long) * scan_tiles, s);
+        cudaMemsetAsync(&b.st->tile_counter[kSortPasses + 1], 0, sizeof(uint32_t), s);
+    }
+    OtNode* nodes = static_cast<OtNode*>(b.oct_nodes);
+    k_oct_scan<<<(unsigned)scan_tiles, kScanThreads, 0, s>>>(b.prefix_n, b.parent, b.oct_counts, b.oct_offsets, lookback,
+                                                             nodes, b.oct_cap, b.st, p.spin_limit);
+    k_oct_make<<<grid_for(n, 256, 0), 256, 0, s>>>(nodes, b.oct_cap, b.oct_offsets, b.oct_counts, b.codes,
+                                                   b.has_leaf_left, b.has_leaf_right, b.prefix_n, b.parent, b.left_child,
+                                                   p.code_bits, b.st);
+    if (launches) *launches += 2;
     return cudaGetLastError();
+}
+
+cudaError_t enqueue_octree(const BuildBufs& b, const BuildParams& p, cudaStream_t s, int* launches) {
+    return launch_octree(b, p, s, true, launches);
 }
 
 cudaError_t enqueue_build(const BuildBufs& b, const BuildParams& p, cudaStream_t s, int num_sms, cudaEvent_t* ev,
@@ -1083,58 +1302,68 @@ cudaError_t enqueue_build(const BuildBufs& b, const BuildParams& p, cudaStream_t
         if (e != cudaSuccess) return e;
     }
     const int64_t n = p.n;
+    const int passes = sort_passes(p.code_bits);
+    const ScratchLayout scratch(n);
+    bool front = false;
     mark(0);
-    cudaMemsetAsync(b.st, 0, sizeof(DevState), s);
     if (n <= 0) {
+        cudaMemsetAsync(b.st, 0, sizeof(DevState), s);
         for (int i = 1; i < kBuildEvents; ++i) mark(i);
         if (launches) *launches = 0;
         return cudaGetLastError();
     }
-    k_bbox<<<grid_for((n + 3) / 4, 256, num_sms * 4), 256, 0, s>>>(b.x, b.y, b.z, n, b.st);
-    mark(1);
-    k_encode<<<grid_for(n, 256, num_sms * 4), 256, 0, s>>>(b.x, b.y, b.z, n, p.code_bits, b.keys0, b.st);
-    k_sort_prep<<<1, kSortBins, 0, s>>>(n, b.st);
-    mark(2);
-    nl += 3;
-    const int64_t sort_tiles = (n + kSortTile - 1) / kSortTile;
-    for (int pass = 0; pass < kSortPasses; ++pass) {
-        cudaMemsetAsync(b.lookback, 0, sizeof(uint32_t) * kSortBins * sort_tiles, s);
-        k_onesweep<<<(unsigned)sort_tiles, kSortThreads, sizeof(SortSmem), s>>>(b.keys0, b.keys1, n, pass,
-                                                                                 b.lookback, b.st, p.spin_limit,
-                                                                                 p.stall_first_tile);
+    if (n <= kFrontMax && !p.stall_first_tile) {
+        // one block from coordinates to unique decoded points; it also clears
+        // the state and the scratch of what follows
+        const cudaError_t e = launch_front(b, n, p.code_bits, scratch, s);
+        if (e != cudaSuccess) {
+            nvtxRangePop();
+            return e;
+        }
+        ++nl;
+        // the stages in one: stage 0 takes their time (an event between two
+        // kernels costs 2.7 us, as much as a small kernel)
+        if (ev) cudaEventRecord(ev[1], s);
+        front = true;
+    } else {
+        cudaMemsetAsync(b.st, 0, sizeof(DevState), s);
+        cudaMemsetAsync(b.scratch, 0, sizeof(uint32_t) * scratch.words(passes), s);
+        k_bbox<<<grid_for((n + 3) / 4, 256, num_sms * 4), 256, 0, s>>>(b.x, b.y, b.z, n, b.st);
+        mark(1);
+        k_encode<<<grid_for(n, 256, num_sms * 4), 256, 0, s>>>(b.x, b.y, b.z, n, p.code_bits, passes, b.keys0, b.st);
+        mark(2);
+        nl += 2;
+        const int64_t sort_tiles = (n + kSortTile - 1) / kSortTile;
+        for (int pass = 0; pass < passes; ++pass) {
+            k_onesweep<<<(unsigned)sort_tiles, kSortThreads, sizeof(SortSmem), s>>>(
+                b.keys0, b.keys1, n, pass, b.scratch + scratch.sort + pass * scratch.sort_pass, b.st, p.spin_limit,
+                p.stall_first_tile);
+            ++nl;
+        }
+        mark(3);
+        const int64_t dd_tiles = (n + kDedupTile - 1) / kDedupTile;
+        k_dedup<<<(unsigned)dd_tiles, kDedupThreads, 0, s>>>(b.keys0, b.keys1, n, p.code_bits, b.codes, b.pts4, b.pts3,
+                                                             b.scratch + scratch.dedup, b.st, p.spin_limit);
         ++nl;
     }
-    mark(3);
-    const int64_t dd_tiles = (n + kDedupTile - 1) / kDedupTile;
-    cudaMemsetAsync(b.lookback, 0, sizeof(uint32_t) * dd_tiles, s);
-    k_dedup<<<(unsigned)dd_tiles, kDedupThreads, 0, s>>>(b.keys0, b.keys1, n, p.code_bits, b.codes, b.pts4, b.pts3,
-                                                         b.lookback, b.st, p.spin_limit);
-    ++nl;
-    mark(4);
+    if (!front) mark(4);
     if (p.build_radix) {
-        cudaMemsetAsync(b.parent, 0, sizeof(int32_t) * n, s);
-        cudaMemsetAsync(b.sparent, 0xff, sizeof(int32_t) * n, s);
-        cudaMemsetAsync(b.leaf_parent, 0xff, sizeof(int32_t) * n, s);
         k_karras<<<grid_for(n, 256, 0), 256, 0, s>>>(b.codes, p.code_bits, p.root_compat, b.left_child, b.parent,
                                                      b.prefix_n, b.has_leaf_left, b.has_leaf_right, b.sparent,
                                                      b.leaf_parent, b.range_end, b.st);
         ++nl;
-        if (p.root_compat) {
-            k_root_parent<<<1, 1, 0, s>>>(b.left_child, b.parent, b.has_leaf_left, b.has_leaf_right, b.st);
-            ++nl;
-        }
     }
     mark(5);
     const int64_t leaf_tiles = (n + kLeafTile - 1) / kLeafTile;
-    cudaMemsetAsync(b.lookback, 0, sizeof(uint32_t) * leaf_tiles, s);
-    cudaMemsetAsync(b.arrivals, 0, sizeof(uint32_t) * arrival_words(n), s);
-    k_leaves<<<(unsigned)leaf_tiles, kLeafThreads, 0, s>>>(b.codes, p.bucket < kLeafMax ? p.bucket : kLeafMax,
-                                                           b.leaf_start, b.lookback, b.st, p.spin_limit);
-    k_boxes<<<grid_for(n, 32 * 128, num_sms * 8), 128, 0, s>>>(b.pts4, b.leaf_start, b.arrivals, b.snodes, b.st);
+    k_leaves<<<(unsigned)leaf_tiles, kLeafThreads, 0, s>>>(
+        b.codes, p.bucket < kLeafMax ? p.bucket : kLeafMax, b.leaf_start, b.scratch + scratch.leaves,
+        p.build_radix && p.root_compat, b.left_child, b.parent, b.has_leaf_left, b.has_leaf_right, b.st, p.spin_limit);
+    k_boxes<<<grid_for(n, 32 * 128, num_sms * 8), 128, 0, s>>>(b.pts4, b.leaf_start, b.scratch + scratch.arrivals,
+                                                               b.snodes, b.st);
     nl += 2;
     mark(6);
     if (p.build_octree) {
-        cudaError_t e = enqueue_octree(b, p, s, num_sms, &nl);
+        cudaError_t e = launch_octree(b, p, s, false, &nl);
         if (e != cudaSuccess) {
             nvtxRangePop();  // the octree stage's range
             return e;

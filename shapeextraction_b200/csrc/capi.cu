@@ -65,9 +65,9 @@ namespace {
 
 void free_build(se_ctx* c) {
     BuildBufs& b = c->b;
-    void* ptrs[] = {b.keys0,     b.keys1,     b.lookback,    b.lookback64, b.codes,     b.pts4,
+    void* ptrs[] = {b.keys0,     b.keys1,     b.scratch,     b.codes,      b.pts4,
                     b.pts3,      b.left_child, b.parent,     b.prefix_n,   b.has_leaf_left, b.has_leaf_right,
-                    b.sparent,   b.leaf_parent, b.range_end, b.leaf_start, b.arrivals,  b.snodes,
+                    b.sparent,   b.leaf_parent, b.range_end, b.leaf_start, b.snodes,
                     b.oct_counts, b.oct_offsets, c->in_xyz};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -90,12 +90,9 @@ int ensure_build_capacity(se_ctx* c, int64_t n) {
     }
     const int64_t cap = n < 1024 ? 1024 : n;
     BuildBufs& b = c->b;
-    const int64_t sort_tiles = (cap + kSortTile - 1) / kSortTile;
-    const int64_t scan_tiles = (cap + kScanTile - 1) / kScanTile;
     SE_CUDA(c, regrow(b.keys0, cap), "alloc keys");
     SE_CUDA(c, regrow(b.keys1, cap), "alloc keys");
-    SE_CUDA(c, regrow(b.lookback, sort_tiles * kSortBins + 64), "alloc lookback");
-    SE_CUDA(c, regrow(b.lookback64, scan_tiles + 64), "alloc lookback");
+    SE_CUDA(c, regrow(b.scratch, ScratchLayout(cap).words(kCodePasses)), "alloc scratch");
     SE_CUDA(c, regrow(b.codes, cap), "alloc codes");
     SE_CUDA(c, regrow(b.pts4, cap), "alloc points");
     SE_CUDA(c, regrow(b.pts3, 3 * cap), "alloc points");
@@ -108,7 +105,6 @@ int ensure_build_capacity(se_ctx* c, int64_t n) {
     SE_CUDA(c, regrow(b.leaf_parent, cap), "alloc search");
     SE_CUDA(c, regrow(b.range_end, cap), "alloc search");
     SE_CUDA(c, regrow(b.leaf_start, cap), "alloc search");
-    SE_CUDA(c, regrow(b.arrivals, arrival_words(cap)), "alloc search");
     SE_CUDA(c, regrow(b.snodes, hierarchy_nodes(cap)), "alloc search");
     SE_CUDA(c, regrow(b.oct_counts, cap), "alloc octree");
     SE_CUDA(c, regrow(b.oct_offsets, cap + 1), "alloc octree");
@@ -131,7 +127,7 @@ int ensure_oct_capacity(se_ctx* c, int64_t m) {
 
 
 int read_state(se_ctx* c) {
-    SE_CUDA(c, cudaMemcpyAsync(c->h_st, c->b.st, sizeof(DevState), cudaMemcpyDeviceToHost, c->stream), "read state");
+    SE_CUDA(c, cudaMemcpyAsync(c->h_st, c->b.st, kHostStateBytes, cudaMemcpyDeviceToHost, c->stream), "read state");
     SE_CUDA(c, cudaStreamSynchronize(c->stream), "synchronize");
     return SE_OK;
 }
@@ -229,7 +225,7 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
         if (!o.st) SE_CUDA(c, cudaMalloc(&o.st, sizeof(DevState)), "alloc query order");
         SE_CUDA(c, regrow(o.keys0, count), "alloc query order");
         SE_CUDA(c, regrow(o.keys1, count), "alloc query order");
-        SE_CUDA(c, regrow(o.lookback, (count + kSortTile - 1) / kSortTile * kSortBins), "alloc query order");
+        SE_CUDA(c, regrow(o.lookback, 3 * ((count + kSortTile - 1) / kSortTile) * kSortBins), "alloc query order");
         c->q_order_cap = count;
     }
     // Pinned host outputs are written by the kernel itself (mapped host
@@ -273,8 +269,7 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
         }
     }
     // clear the error word and counters of the previous call
-    SE_CUDA(c, cudaMemsetAsync(&c->b.st->err, 0, sizeof(uint32_t), c->stream), "reset");
-    SE_CUDA(c, cudaMemsetAsync(c->b.st->counters, 0, sizeof(DevState) - offsetof(DevState, counters), c->stream), "reset");
+    SE_CUDA(c, cudaMemsetAsync(c->b.st, 0, kQueryStateBytes, c->stream), "reset");
     c->have_query_times = false;
     SE_CUDA(c, cudaEventRecord(c->query_ev[0], c->stream), "event");
     if (use_learned)
@@ -302,19 +297,15 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
     }
     c->query_launches = (use_learned ? 2 : 1) + (lut_launched ? 1 : 0) + order_launches;
     c->have_query_times = true;
-    SE_CUDA(c, cudaMemcpyAsync(&c->h_st->err, &c->b.st->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream),
-            "read state");
-    c->h_st->pad0 = 0;
+    SE_CUDA(c, cudaMemcpyAsync(c->h_st, c->b.st, kQueryStateBytes, cudaMemcpyDeviceToHost, c->stream), "read state");
+    c->h_st->n_active = 0;
     if (sorted)  // the error word of the queries' sort
-        SE_CUDA(c, cudaMemcpyAsync(&c->h_st->pad0, &c->q_order.st->err, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+        SE_CUDA(c, cudaMemcpyAsync(&c->h_st->n_active, &c->q_order.st->err, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                    c->stream),
                 "read state");
-    SE_CUDA(c, cudaMemcpyAsync(c->h_st->counters, c->b.st->counters, sizeof(c->b.st->counters),
-                               cudaMemcpyDeviceToHost, c->stream),
-            "read state");
     SE_CUDA(c, cudaStreamSynchronize(c->stream), "synchronize");
     for (int i = 0; i < kQueryCounters; ++i) c->last_counters[i] = (int64_t)c->h_st->counters[i];
-    return check_err_bits(c, c->h_st->err | c->h_st->pad0);
+    return check_err_bits(c, c->h_st->err | (uint32_t)c->h_st->n_active);
 }
 
 }  // namespace
@@ -437,8 +428,7 @@ int se_destroy(se_ctx* c) {
     if (c->lut_buf) cudaFree(c->lut_buf);
     for (BatchLane& l : c->lanes) {
         if (l.stream) cudaStreamSynchronize(l.stream);
-        void* ptrs[] = {l.b.keys0, l.b.keys1,      l.b.lookback, l.b.codes,
-                        l.b.pts3,  l.b.leaf_start, l.b.arrivals, l.b.st};
+        void* ptrs[] = {l.b.keys0, l.b.keys1, l.b.scratch, l.b.codes, l.b.pts3, l.b.leaf_start, l.b.st};
         for (void* p : ptrs)
             if (p) cudaFree(p);
         if (l.done) cudaEventDestroy(l.done);
@@ -509,13 +499,14 @@ int se_build(se_ctx* c, const float* x, const float* y, const float* z, int64_t 
     SE_CUDA(c, enqueue_build(b, p, c->stream, c->num_sms, c->build_ev, &c->build_launches), "launch build");
     if (int rc = read_state(c)) return rc;
     c->have_build_times = true;
+    c->build_front = n > 0 && n <= kFrontMax && !p.stall_first_tile;
     // any other failure first: the octree count of a failed build means nothing
     if (int rc = check_err_bits(c, c->h_st->err & ~(uint32_t)ERRBIT_OCT_CAPACITY)) return rc;
     if (c->h_st->err & ERRBIT_OCT_CAPACITY) {
         const int64_t m = (int64_t)c->h_st->n_oct;
         if (int rc = ensure_oct_capacity(c, m)) return rc;
         SE_CUDA(c, cudaMemsetAsync(&b.st->err, 0, sizeof(uint32_t), c->stream), "reset");
-        SE_CUDA(c, enqueue_octree(b, p, c->stream, c->num_sms, &c->build_launches), "launch octree");
+        SE_CUDA(c, enqueue_octree(b, p, c->stream, &c->build_launches), "launch octree");
         if (int rc = read_state(c)) return rc;
         c->have_build_times = false;
     }
@@ -642,8 +633,12 @@ int se_get_profile(se_ctx* c, se_profile* prof) {
     std::memset(prof, 0, sizeof(*prof));
     if (int rc = prologue(c)) return rc;
     if (c->have_build_times) {
-        for (int i = 1; i < kBuildEvents; ++i)
-            SE_CUDA(c, cudaEventElapsedTime(&prof->build_ms[i - 1], c->build_ev[i - 1], c->build_ev[i]), "event time");
+        int last = 0;  // the event before event i
+        for (int i = 1; i < kBuildEvents; ++i) {
+            if (c->build_front && i >= 2 && i <= 4) continue;
+            SE_CUDA(c, cudaEventElapsedTime(&prof->build_ms[i - 1], c->build_ev[last], c->build_ev[i]), "event time");
+            last = i;
+        }
         SE_CUDA(c, cudaEventElapsedTime(&prof->build_ms[7], c->build_ev[0], c->build_ev[kBuildEvents - 1]),
                 "event time");
     }

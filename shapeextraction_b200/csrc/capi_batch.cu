@@ -33,14 +33,12 @@ int lane_capacity(se_ctx* c, BatchLane& l, int64_t n) {
     ++c->batch_epoch;
     BuildBufs& b = l.b;
     const int64_t cap = n < 1024 ? 1024 : n;
-    const int64_t sort_tiles = (cap + kSortTile - 1) / kSortTile;
     SE_CUDA(c, regrow(b.keys0, cap), "alloc lane");
     SE_CUDA(c, regrow(b.keys1, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.lookback, sort_tiles * kSortBins + 64), "alloc lane");
+    SE_CUDA(c, regrow(b.scratch, ScratchLayout(cap).words(kCodePasses)), "alloc lane");
     SE_CUDA(c, regrow(b.codes, cap), "alloc lane");
     SE_CUDA(c, regrow(b.pts3, 3 * cap), "alloc lane");
     SE_CUDA(c, regrow(b.leaf_start, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.arrivals, arrival_words(cap)), "alloc lane");
     b.cap = cap;
     l.cap = cap;
     return SE_OK;

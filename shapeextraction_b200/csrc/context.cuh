@@ -116,6 +116,7 @@ struct se_ctx {
     cudaEvent_t build_ev[kBuildEvents] = {};
     cudaEvent_t query_ev[2] = {};
     bool have_build_times = false, have_query_times = false;
+    bool build_front = false;  // the last build's stages 0 to 3 were one kernel
     int build_launches = 0, query_launches = 0;
 };
 

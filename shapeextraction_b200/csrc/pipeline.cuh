@@ -1,6 +1,7 @@
 // Internal interface between the C ABI layer (capi.cu) and the kernels.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -38,28 +39,52 @@ enum { CNT_FP64 = 0, CNT_NODES, CNT_BUCKETS, CNT_CANDIDATES, CNT_MERGE, CNT_INSE
 
 // Small device-resident state of one build (zeroed at the start of each build).
 struct DevState {
+    // what a query clears and the host reads after it
     uint32_t err;
-    uint32_t min_ord;  // ordered-uint encodings (f2ord) of the bbox min / max
-    uint32_t max_ord;
-    uint32_t pad0;
+    uint32_t work;  // next work item of a persistent search launch
+    unsigned long long counters[kQueryCounters];  // in the order of se_stats
+    // what the host reads after a build
+    unsigned long long u;      // unique codes
+    unsigned long long n_oct;  // octree nodes
     float min_coord, max_coord, range;
-    int32_t n_active;                       // non-trivial sort passes
-    int32_t pass_active[kSortPasses];
-    int32_t pass_parity[kSortPasses];
-    uint32_t tile_counter[16];              // dynamic tile ids: sort passes, dedup, octree scan
-    uint32_t hist[kSortPasses][kSortBins];       // per-digit histograms of the codes
-    uint32_t digit_off[kSortPasses][kSortBins];  // exclusive digit offsets
-    unsigned long long u;                   // unique codes
-    unsigned long long n_oct;               // octree nodes
     int32_t root_level;
     // search hierarchy: level l holds level_count[l] nodes from level_off[l] on;
     // the top level is the first of at most kFan nodes
     int32_t top_level;
     uint32_t level_off[kMaxLevels];
     uint32_t level_count[kMaxLevels];
-    // query counters, in the order of se_stats
-    unsigned long long counters[kQueryCounters];
-    uint32_t work;  // next work item of a persistent search launch
+    // build scratch
+    uint32_t min_ord;  // ordered-uint encodings (f2ord) of the bbox min / max
+    uint32_t max_ord;
+    int32_t n_active;                       // non-trivial sort passes
+    int32_t pass_active[kSortPasses];
+    int32_t pass_parity[kSortPasses];
+    uint32_t tile_counter[16];              // dynamic tile ids: sort passes, dedup, octree scan, leaves; encode's blocks
+    uint32_t hist[kSortPasses][kSortBins];       // per-digit histograms of the codes
+    uint32_t digit_off[kSortPasses][kSortBins];  // exclusive digit offsets
+};
+constexpr size_t kQueryStateBytes = offsetof(DevState, u);          // err, work, counters
+constexpr size_t kHostStateBytes = offsetof(DevState, level_off);   // what the host reads
+
+// Codes of at most 63 bits take this many digit passes.
+constexpr int sort_passes(int code_bits) { return (code_bits + kSortBits - 1) / kSortBits; }
+constexpr int kCodePasses = sort_passes(63);
+
+// Scratch of one build that must start at zero, in 32-bit words: the octree
+// scan's look-back (64-bit), the hierarchy's arrival counters, the look-backs
+// of the leaf scan and of dedup, and last those of the sort passes.
+struct ScratchLayout {
+    int64_t oct, arrivals, leaves, dedup, sort, sort_pass;
+    explicit ScratchLayout(int64_t n) {
+        const int64_t tiles = (n + kSortTile - 1) / kSortTile;
+        oct = 0;
+        arrivals = 2 * ((n + kScanTile - 1) / kScanTile);
+        leaves = arrivals + n / 512 + 16;  // one counter per hierarchy node of level 2 and up
+        dedup = leaves + (n + kLeafTile - 1) / kLeafTile;
+        sort = dedup + (n + kDedupTile - 1) / kDedupTile;
+        sort_pass = kSortBins * tiles;
+    }
+    int64_t words(int passes) const { return sort + passes * sort_pass; }
 };
 
 // Byte layout of OT::OTNode (reference src/Octree.hpp:19-36), 56 bytes.
@@ -89,9 +114,6 @@ __host__ __device__ constexpr int64_t hierarchy_nodes(int64_t n) {
     }
     return total;
 }
-// Words of the arrival counters that its build needs (one per node of level 2 and up).
-__host__ __device__ constexpr int64_t arrival_words(int64_t n) { return n / 512 + 16; }
-
 struct BuildBufs {
     int64_t cap;  // capacity in points
     const float* x;
@@ -99,8 +121,7 @@ struct BuildBufs {
     const float* z;
     uint64_t* keys0;
     uint64_t* keys1;
-    uint32_t* lookback;  // sort/dedup look-back words
-    unsigned long long* lookback64;  // octree-scan look-back words
+    uint32_t* scratch;   // ScratchLayout(cap).words(kCodePasses)
     uint64_t* codes;     // unique sorted codes
     float4* pts4;        // decoded points, padded for 16-byte loads
     float* pts3;         // decoded points, AoS xyz
@@ -116,7 +137,6 @@ struct BuildBufs {
     int32_t* range_end;
     // search hierarchy
     int32_t* leaf_start;  // first point of each leaf
-    uint32_t* arrivals;   // arrival counters of the hierarchy build
     SNode* snodes;        // hierarchy_nodes(cap) entries
     // octree
     int32_t* oct_counts;
@@ -140,14 +160,16 @@ struct BuildParams {
 // Stage events of one build: [0] start, then after bbox, encode, sort, dedup,
 // radix tree, search boxes, octree.
 constexpr int kBuildEvents = 8;
+constexpr int kFrontMax = 8192;
 
 // Enqueue the whole build on `s`. Reads x/y/z from bufs; results stay on the
 // device. `ev` (kBuildEvents events, may be null) are recorded between stages;
-// *launches receives the number of kernels launched.
+// *launches receives the number of kernels launched. Of a cloud of at most
+// kFrontMax points events 2 to 4 are not recorded: one kernel does stages 0 to 3.
 cudaError_t enqueue_build(const BuildBufs& b, const BuildParams& p, cudaStream_t s, int num_sms, cudaEvent_t* ev,
                           int* launches);
 // Enqueue only the octree stage (used to redo it after a capacity regrow).
-cudaError_t enqueue_octree(const BuildBufs& b, const BuildParams& p, cudaStream_t s, int num_sms, int* launches);
+cudaError_t enqueue_octree(const BuildBufs& b, const BuildParams& p, cudaStream_t s, int* launches);
 
 // ---- learned search-radius proposal (mlp.cu) --------------------------------
 constexpr int kMlpF = 32;  // features per point
