@@ -26,6 +26,19 @@
 // [slot][thread] arrays, so the threads of a warp touch 32 distinct banks
 // whatever slots they address. Queries are the tree's Morton-ordered points
 // (or caller queries), so neighbouring threads walk similar paths.
+//
+// Bound by divergence and the latency of dependent node loads: every thread's
+// heaps take their own paths, and walks differ in length (488 pops on average,
+// 1305 for the longest of 32, on a 200k-point scene). So threads are persistent
+// and take a new query as soon as theirs ends (waiting until 4, 8 or 16 of a
+// warp have ended, to write results together: 19.7, 20.7, 22.3 ms against 18.9);
+// each step a thread pops if it has dealt with its node, and inserts one thing,
+// its next point that the results take or its next child node, through one copy
+// of the code; an item on its way through a heap is carried in registers and
+// written once; one loop climbs minimum and maximum levels alike. 200k points,
+// k = 16: 53.2 ms with one query per thread in lockstep over the eight child
+// numbers, 31.7 ms with the carried items and each thread's own next child,
+// 18.9 ms now; warp instructions 12.3 G -> 8.9 G -> 6.4 G.
 
 #include <cstdint>
 
@@ -36,7 +49,7 @@ namespace shapex {
 
 namespace {
 
-constexpr int kCompatThreads = 128;
+constexpr int kCompatThreads = 64;
 constexpr int kSearchSlots = 32;  // SEARCH_Q_SIZE, src/Octree.hpp:17
 
 // Bounded min-max heap over one thread's column of [slot][thread] arrays.
@@ -48,13 +61,10 @@ struct ColumnHeap {
     int cap;
 
     __device__ __forceinline__ float P(int i) const { return pri[i * kCompatThreads]; }
-    __device__ __forceinline__ void swp(int a, int b) {
-        const float pa = pri[a * kCompatThreads];
-        const int32_t ia = item[a * kCompatThreads];
-        pri[a * kCompatThreads] = pri[b * kCompatThreads];
-        item[a * kCompatThreads] = item[b * kCompatThreads];
-        pri[b * kCompatThreads] = pa;
-        item[b * kCompatThreads] = ia;
+    __device__ __forceinline__ int32_t I(int i) const { return item[i * kCompatThreads]; }
+    __device__ __forceinline__ void put(int i, float p, int32_t it) {
+        pri[i * kCompatThreads] = p;
+        item[i * kCompatThreads] = it;
     }
     static __device__ __forceinline__ int par(int i) { return (i - 1) / 2; }
     static __device__ __forceinline__ int lc(int i) { return 2 * i + 1; }
@@ -62,57 +72,15 @@ struct ColumnHeap {
     static __device__ __forceinline__ bool min_level(int i) { return ((31 - __clz(i + 1)) & 1) == 0; }
 
     __device__ __forceinline__ int largest() const {
-        if (size >= 2) {
-            if (size == 2) return 1;
-            return P(1) > P(2) ? 1 : 2;
-        }
-        return 0;
-    }
-    __device__ void up_min(int i) {
-        while (i >= 3) {
-            const int g = par(par(i));
-            if (P(i) < P(g)) {
-                swp(i, g);
-                i = g;
-            } else {
-                break;
-            }
-        }
-    }
-    __device__ void up_max(int i) {
-        while (i >= 3) {
-            const int g = par(par(i));
-            if (P(i) > P(g)) {
-                swp(i, g);
-                i = g;
-            } else {
-                break;
-            }
-        }
-    }
-    __device__ void bubble_up(int i) {
-        if (min_level(i)) {
-            if (i > 0 && P(i) > P(par(i))) {
-                swp(i, par(i));
-                up_max(par(i));
-            } else {
-                up_min(i);
-            }
-        } else {
-            if (i > 0 && P(i) < P(par(i))) {
-                swp(i, par(i));
-                up_min(par(i));
-            } else {
-                up_max(i);
-            }
-        }
+        if (size >= 3) return P(1) > P(2) ? 1 : 2;
+        return size - 1;  // 1 of two, 0 of one
     }
     // smallest (MIN) or largest (!MIN) of i's children and grandchildren,
     // first in the order lc, rc, lc(lc), rc(lc), lc(rc), rc(rc) on ties
     template <bool MIN>
-    __device__ __forceinline__ int pick(int i) const {
+    __device__ __forceinline__ int pick(int i, float& pm) const {
         int m = lc(i);
-        float pm = P(m);
+        pm = P(m);
         const int desc[5] = {rc(i), lc(lc(i)), rc(lc(i)), lc(rc(i)), rc(rc(i))};
 #pragma unroll
         for (int d = 0; d < 5; ++d) {
@@ -126,53 +94,64 @@ struct ColumnHeap {
         }
         return m;
     }
+    // Place item (w, it) at slot i or below it (percolate of src/dequeue.hpp),
+    // i on a minimum level (MIN) or a maximum level (!MIN).
     template <bool MIN>
-    __device__ void down(int i) {
+    __device__ __forceinline__ void down(int i, float w, int32_t it) {
         while (lc(i) < size) {
-            const int m = pick<MIN>(i);
-            if (m > rc(i)) {  // a grandchild
-                if (MIN ? P(m) < P(i) : P(m) > P(i)) {
-                    swp(i, m);
-                    if (MIN ? P(m) > P(par(m)) : P(m) < P(par(m))) swp(par(m), m);
-                    i = m;
-                } else {
-                    break;
-                }
-            } else {  // a child
-                if (MIN ? P(m) < P(i) : P(m) > P(i)) swp(i, m);
-                break;
+            float pm;
+            const int m = pick<MIN>(i, pm);
+            if (!(MIN ? pm < w : pm > w)) break;
+            put(i, pm, I(m));
+            const bool grandchild = m > rc(i);
+            i = m;
+            if (!grandchild) break;
+            const int q = par(m);
+            const float pp = P(q);
+            if (MIN ? w > pp : w < pp) {  // the carried item stays at the parent, the parent's goes on
+                const int32_t pit = I(q);
+                put(q, w, it);
+                w = pp;
+                it = pit;
             }
         }
-    }
-    __device__ __forceinline__ void percolate(int i) {
-        if (min_level(i)) down<true>(i);
-        else down<false>(i);
+        put(i, w, it);
     }
     __device__ __forceinline__ void remove_min(float& p, int32_t& it) {
         p = P(0);
-        it = item[0];
+        it = I(0);
         --size;
-        pri[0] = P(size);
-        item[0] = item[size * kCompatThreads];
-        percolate(0);
+        down<true>(0, P(size), I(size));
     }
-    __device__ __forceinline__ void remove_max() {
-        const int l = largest();
-        --size;
-        pri[l * kCompatThreads] = P(size);
-        item[l * kCompatThreads] = item[size * kCompatThreads];
-        percolate(l);
-    }
+    // Insert; the caller has checked that a full heap's largest is not below w.
     __device__ __forceinline__ void insert(int32_t it, float w) {
-        if (size == cap) {
-            if (P(largest()) >= w) remove_max();
-            else return;
+        if (size == cap) {  // drop the largest
+            const int l = largest();
+            --size;
+            if (l > 0) down<false>(l, P(size), I(size));
         }
-        ++size;
-        pri[(size - 1) * kCompatThreads] = w;
-        item[(size - 1) * kCompatThreads] = it;
-        bubble_up(size - 1);
+        int i = size++;
+        bool lvl = min_level(i);
+        if (i > 0) {
+            const int q = par(i);
+            const float pq = P(q);
+            if (lvl ? w > pq : w < pq) {
+                put(i, pq, I(q));
+                i = q;
+                lvl = !lvl;
+            }
+        }
+        while (i >= 3) {
+            const int g = par(par(i));
+            const float pg = P(g);
+            if (!(lvl ? w < pg : w > pg)) break;
+            put(i, pg, I(g));
+            i = g;
+        }
+        put(i, w, it);
     }
+    // Whether insert() would keep an item of priority w (src/dequeue.hpp:60-67).
+    __device__ __forceinline__ bool takes(float w) const { return size < cap || P(largest()) >= w; }
 };
 
 // nodeBoxDistance, src/Octree.cu:326-352
@@ -206,74 +185,13 @@ struct CompatArgs {
     float vx, vy, vz;
 };
 
-template <bool EXT, bool NORMALS>
-__global__ void __launch_bounds__(kCompatThreads)
-    k_knn_compat(const OtNode* __restrict__ nodes, const float4* __restrict__ pts, CompatArgs a, DevState* st) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int tid = threadIdx.x;
-    float* s_pri = reinterpret_cast<float*>(smem_raw);
-    int32_t* s_item = reinterpret_cast<int32_t*>(s_pri + kSearchSlots * kCompatThreads);
-    float* r_pri = reinterpret_cast<float*>(s_item + kSearchSlots * kCompatThreads);
-    int32_t* r_item = reinterpret_cast<int32_t*>(r_pri + a.k * kCompatThreads);
-    const int64_t qi = (int64_t)blockIdx.x * kCompatThreads + tid;
-    if (qi >= a.count) return;
-    float qx, qy, qz;
-    if (EXT) {
-        qx = a.ext[3 * qi];
-        qy = a.ext[3 * qi + 1];
-        qz = a.ext[3 * qi + 2];
-    } else {
-        const float4 q = pts[a.start + qi];
-        qx = q.x;
-        qy = q.y;
-        qz = q.z;
-    }
-    ColumnHeap sq{s_pri + tid, s_item + tid, 0, kSearchSlots};
-    ColumnHeap rq{r_pri + tid, r_item + tid, 0, a.k};
-    uint32_t err = 0;
-    sq.insert(0, 0.0f);
-    // every node enters the heap at most once (children of a popped node), so
-    // a walk of more than m pops means a malformed octree
-    int64_t pops = 0;
-    while (sq.size > 0) {
-        float pr;
-        int32_t ni;
-        sq.remove_min(pr, ni);
-        if (++pops > a.m) {
-            err |= ERRBIT_SEARCH_LIMIT;
-            break;
-        }
-        const OtNode& nd = nodes[ni];
-        const int leaf_mask = nd.child_leaf_mask, node_mask = nd.child_node_mask;
-        if (leaf_mask) {
-#pragma unroll 1
-            for (int c = 0; c < 8; ++c) {
-                if (leaf_mask & (1 << c)) {
-                    const int32_t li = nd.children[c];
-                    if (li < 0 || li >= a.u) {
-                        err |= ERRBIT_BOUNDS;
-                        continue;
-                    }
-                    rq.insert(li, ref_distance2(qx, qy, qz, __ldg(pts + li)));
-                }
-            }
-        }
-#pragma unroll 1
-        for (int c = 0; c < 8; ++c) {
-            if (node_mask & (1 << c)) {
-                const int32_t ci = nd.children[c];
-                if (ci < 0 || ci >= a.m) {
-                    err |= ERRBIT_BOUNDS;
-                    continue;
-                }
-                sq.insert(ci, face_distance(qx, qy, qz, nodes[ci]));
-            }
-        }
-    }
-    // results in remove-min order, written back into the (empty) node heap's
-    // column so that the covariance reads them in that order
-    int32_t* order = s_item + tid;
-    float* order_d2 = s_pri + tid;
+// One thread's finished query: its results in remove-min order and, with
+// NORMALS, its normal. The order goes into the (empty) node heap's column so
+// that the covariance reads the neighbours in it.
+template <bool NORMALS>
+__device__ __forceinline__ void write_results(ColumnHeap& rq, int32_t* order, float* order_d2, float qx, float qy,
+                                              float qz, int64_t qi, const float4* __restrict__ pts,
+                                              const CompatArgs& a) {
     int32_t first = -1;
     float first_d2 = __int_as_float(0x7f800000);
     for (int c = 0; c < a.k; ++c) {
@@ -344,15 +262,134 @@ __global__ void __launch_bounds__(kCompatThreads)
             out[2] = nz;
         }
     }
+}
+
+template <bool EXT, bool NORMALS>
+__global__ void __launch_bounds__(kCompatThreads)
+    k_knn_compat(const OtNode* __restrict__ nodes, const float4* __restrict__ pts, CompatArgs a, DevState* st) {
+    constexpr unsigned kFull = 0xffffffffu;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int tid = threadIdx.x, lane = tid & 31;
+    float* s_pri = reinterpret_cast<float*>(smem_raw) + tid;
+    int32_t* s_item = reinterpret_cast<int32_t*>(s_pri + kSearchSlots * kCompatThreads);
+    float* r_pri = reinterpret_cast<float*>(s_item + kSearchSlots * kCompatThreads);
+    int32_t* r_item = reinterpret_cast<int32_t*>(r_pri + a.k * kCompatThreads);
+    ColumnHeap sq{s_pri, s_item, 0, kSearchSlots};
+    ColumnHeap rq{r_pri, r_item, 0, a.k};
+    uint32_t err = 0;
+    float qx = 0.0f, qy = 0.0f, qz = 0.0f;
+    uint32_t qi = 0;
+    bool live = false;       // the thread has a query
+    bool more = true;        // the counter still had queries (the same for the whole warp)
+    // the popped node's points and child nodes not dealt with yet
+    uint32_t leaf_mask = 0, node_mask = 0;
+    const int32_t* child = nullptr;
+    // every node enters the heap at most once (children of a popped node), so
+    // a walk of more than m pops means a malformed octree
+    int32_t pops = 0;
+    for (;;) {
+        // A thread whose walk has ended writes its results and takes a new query.
+        const bool ended = live && sq.size == 0 && !(leaf_mask | node_mask);
+        const uint32_t idle = __ballot_sync(kFull, ended || !live);
+        if (idle == kFull || (more && idle)) {
+            if (ended) {
+                write_results<NORMALS>(rq, s_item, s_pri, qx, qy, qz, qi, pts, a);
+                live = false;
+            }
+            __syncwarp();
+            if (!more) break;
+            const uint32_t want = __ballot_sync(kFull, !live);
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&st->work, (uint32_t)__popc(want));
+            base = __shfl_sync(kFull, base, 0);
+            more = (int64_t)base + __popc(want) < a.count;
+            qi = live ? qi : base + __popc(want & lanemask_lt());
+            if (!live && qi < a.count) {
+                if (EXT) {
+                    qx = a.ext[3 * (int64_t)qi];
+                    qy = a.ext[3 * (int64_t)qi + 1];
+                    qz = a.ext[3 * (int64_t)qi + 2];
+                } else {
+                    const float4 q = pts[a.start + qi];
+                    qx = q.x;
+                    qy = q.y;
+                    qz = q.z;
+                }
+                live = true;
+                rq.size = 0;
+                pops = 0;
+                sq.size = 1;
+                sq.put(0, 0.0f, 0);  // the root
+            }
+            __syncwarp();
+        }
+        // threads that have dealt with their node pop the next
+        if (!(leaf_mask | node_mask) && sq.size > 0) {
+            float pr;
+            int32_t ni;
+            sq.remove_min(pr, ni);
+            child = nodes[ni].children;
+            node_mask = (uint32_t)nodes[ni].child_node_mask & 0xffu;
+            leaf_mask = (uint32_t)nodes[ni].child_leaf_mask & 0xffu;
+            if (++pops > a.m) {
+                err |= ERRBIT_SEARCH_LIMIT;
+                sq.size = 0;
+                leaf_mask = node_mask = 0;
+            }
+        }
+        __syncwarp();
+        // one insertion per thread: its next point that the results take, or
+        // else its next child node (the two heaps are independent)
+        bool take = false, leaf = false;
+        int32_t it = 0;
+        float w = 0.0f;
+        while (leaf_mask && !take) {
+            const int c = __ffs(leaf_mask) - 1;
+            leaf_mask &= leaf_mask - 1;
+            it = child[c];
+            if (it < 0 || it >= a.u) {
+                err |= ERRBIT_BOUNDS;
+                continue;
+            }
+            w = ref_distance2(qx, qy, qz, __ldg(pts + it));
+            take = leaf = rq.takes(w);
+        }
+        __syncwarp();
+        if (!take && node_mask) {
+            const int c = __ffs(node_mask) - 1;
+            node_mask &= node_mask - 1;
+            it = child[c];
+            if (it < 0 || it >= a.m) {
+                err |= ERRBIT_BOUNDS;
+            } else {
+                w = face_distance(qx, qy, qz, nodes[it]);
+                take = sq.takes(w);
+            }
+        }
+        __syncwarp();
+        if (take) {
+            ColumnHeap h{leaf ? r_pri : s_pri, leaf ? r_item : s_item, leaf ? rq.size : sq.size,
+                         leaf ? a.k : kSearchSlots};
+            h.insert(it, w);
+            if (leaf) rq.size = h.size;
+            else sq.size = h.size;
+        }
+        __syncwarp();
+    }
     if (err) atomicOr(&st->err, err);
 }
 
 template <bool EXT, bool NORMALS>
-cudaError_t launch_compat(const BuildBufs& b, const CompatArgs& a, cudaStream_t s) {
+cudaError_t launch_compat(const BuildBufs& b, const CompatArgs& a, cudaStream_t s, int num_sms) {
     const int smem = (kSearchSlots + a.k) * kCompatThreads * 8;
     cudaError_t e = cudaFuncSetAttribute(k_knn_compat<EXT, NORMALS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const unsigned blocks = (unsigned)((a.count + kCompatThreads - 1) / kCompatThreads);
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_knn_compat<EXT, NORMALS>, kCompatThreads, smem);
+    if (e != cudaSuccess) return e;
+    const int64_t want = (a.count + kCompatThreads - 1) / kCompatThreads;
+    const int64_t resident = (int64_t)(per_sm > 0 ? per_sm : 1) * num_sms;
+    const unsigned blocks = (unsigned)(want < resident ? want : resident);
     k_knn_compat<EXT, NORMALS><<<blocks, kCompatThreads, smem, s>>>(static_cast<const OtNode*>(b.oct_nodes), b.pts4,
                                                                     a, b.st);
     return cudaGetLastError();
@@ -360,7 +397,7 @@ cudaError_t launch_compat(const BuildBufs& b, const CompatArgs& a, cudaStream_t 
 
 }  // namespace
 
-cudaError_t enqueue_query_compat(const BuildBufs& b, const QueryParams& q, cudaStream_t s) {
+cudaError_t enqueue_query_compat(const BuildBufs& b, const QueryParams& q, cudaStream_t s, int num_sms) {
     if (q.count <= 0) return cudaSuccess;
     if (q.k < 1 || q.k > 32 || q.n_octree < 1 || !b.oct_nodes) return cudaErrorInvalidValue;
     CompatArgs a;
@@ -376,9 +413,9 @@ cudaError_t enqueue_query_compat(const BuildBufs& b, const QueryParams& q, cudaS
     a.vx = q.vx;
     a.vy = q.vy;
     a.vz = q.vz;
-    if (a.ext) return launch_compat<true, false>(b, a, s);
-    if (a.out_normals) return launch_compat<false, true>(b, a, s);
-    return launch_compat<false, false>(b, a, s);
+    if (a.ext) return launch_compat<true, false>(b, a, s, num_sms);
+    if (a.out_normals) return launch_compat<false, true>(b, a, s, num_sms);
+    return launch_compat<false, false>(b, a, s, num_sms);
 }
 
 }  // namespace shapex

@@ -1341,7 +1341,7 @@ int queries_per_warp(int64_t count, int num_sms, bool foreign) {
 cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t s, int num_sms) {
     if (q.count <= 0) return cudaSuccess;
     if (q.k < 1 || q.k > 32) return cudaErrorInvalidValue;
-    if (q.compat) return enqueue_query_compat(b, q, s);
+    if (q.compat) return enqueue_query_compat(b, q, s, num_sms);
     QArgs a;
     a.k = q.k;
     a.start = q.start;

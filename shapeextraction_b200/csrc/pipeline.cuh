@@ -297,6 +297,6 @@ cudaError_t enqueue_query_batch(const BatchCloud* clouds, int n_clouds, int64_t 
                                 const QueryParams& q, cudaStream_t s, int num_sms);
 // Reference-compatible search over the OTNode array (enqueue_query forwards
 // to it when q.compat is set).
-cudaError_t enqueue_query_compat(const BuildBufs& b, const QueryParams& q, cudaStream_t s);
+cudaError_t enqueue_query_compat(const BuildBufs& b, const QueryParams& q, cudaStream_t s, int num_sms);
 
 }  // namespace shapex

@@ -133,3 +133,19 @@ def test_foreign_queries_in_any_order(native, oracle, shape, k):
             assert np.array_equal(idx, ei) and np.array_equal(d2, ed), n
             ti = c.knn(torch.from_numpy(q).cuda(), k)
             assert np.array_equal(ti.cpu().numpy(), ei), n
+
+
+@pytest.mark.parametrize("k", [1, 2, 16, 32])
+def test_compat_search_at_thread_counts(native, oracle, k):
+    """The reference's search on counts around a warp and a block, and on more
+    queries than there are threads at once (threads take several)."""
+    rng = np.random.default_rng(23)
+    x, y, z = rng.random((3, 90_000)).astype(np.float32)
+    with native.Context(search_compat=True) as c:
+        c.build(x, y, z)
+        p, nodes = c.points(), c.octree()
+        for start, n in ((0, 1), (7, 31), (100, 33), (0, 64), (5, 65), (3, 1_000)):
+            assert np.array_equal(c.knn_self(k, start, n), oracle.knn_compat(nodes, p, p[start:start + n], k))
+        idx = c.knn_self(k)
+        s = slice(0, len(p), 37)
+        assert np.array_equal(idx[s], oracle.knn_compat(nodes, p, p[s], k))
