@@ -102,10 +102,10 @@ typedef struct se_options {
     /* se_normals_batch scheduling (0: the default of each); se_tune_batch
      * measures and sets them, with leaf_bucket and seed_halo. */
     int32_t batch_lanes;           /* streams the clouds' builds are spread over (1..16;
-                                      default 8) */
+                                      default 16) */
     int32_t batch_lane_min_points; /* clouds of at least this many points are queried on
                                       their stream right after their build, the others in
-                                      the shared persistent launches (default 65536) */
+                                      the shared persistent launches (default 262144) */
     int32_t batch_blocks_per_sm;   /* resident blocks per SM of the persistent launches
                                       (default: as many as fit) */
     int32_t batch_warps_per_block; /* warps per block of the persistent launches: 2 or 4
