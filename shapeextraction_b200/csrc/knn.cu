@@ -308,9 +308,10 @@ __device__ __forceinline__ void prune(Query& q, float tau, int room, WS& W, int 
 // Append every lane's hits among a run of points (bit i of `hits`: point
 // `first` + i, at(i) its coordinates) to its candidates, making room on the
 // way; a hit that a bound tightened meanwhile excludes is passed over. With
-// `settle` all candidates are merged in any case.
+// `settle` all candidates are merged in any case. A prune leaves at most `room`
+// candidates.
 template <int K, bool EXACT, class WS, class At>
-__device__ __forceinline__ void take_hits(uint32_t hits, bool settle, At at, Nearest<K, EXACT>& nn, Query& q, float& tau,
+__device__ __forceinline__ void take_hits(uint32_t hits, bool settle, int room, At at, Nearest<K, EXACT>& nn, Query& q, float& tau,
                                           float cap, WS& W, int lane, Counters& ct) {
     constexpr int kBuf = KnnCfg<K>::buf;
     for (;;) {
@@ -320,7 +321,7 @@ __device__ __forceinline__ void take_hits(uint32_t hits, bool settle, At at, Nea
         if (settle || __any_sync(FULL, q.n + mine > kBuf)) {
             settle = false;
             merge_fresh(nn, q, W, lane, ct);
-            prune(q, nn.tau, kBuf - 8, W, lane, ct);
+            prune(q, nn.tau, room, W, lane, ct);
             if (tau >= 0.0f) tau = fminf(nn.tau, cap);
             rounds = min(rounds, (int)__reduce_min_sync(FULL, (unsigned)(kBuf - q.n)));
         }
@@ -627,7 +628,7 @@ __device__ __forceinline__ bool cell_scan(Nearest<K, EXACT>& nn, Query& q, WS& W
             if (dist2(qx, qy, qz, p.x, p.y, p.z) <= b2) hits |= 1u << t;
         }
         take_hits<K, EXACT>(
-            hits, !merged,
+            hits, !merged, KnnCfg<K>::buf - 8,
             [&](int i, int32_t& idx) {
                 const float4 p = W.pts[i];
                 idx = __float_as_int(p.w);
@@ -911,7 +912,7 @@ __device__ __forceinline__ void search(Nearest<K, EXACT>& nn, Query& q, WS& W, i
         if (!done)
             hits = scan_run(f, cnt, needm, own ? e0 : w0, own ? e1 : w1, q, tau, W, lane, pts);
         take_hits<K, EXACT>(
-            hits, done || (window && next >= w1),
+            hits, done || (window && next >= w1), done ? K : KnnCfg<K>::buf - 8,
             [&](int i, int32_t& idx) {
                 const float* c = reinterpret_cast<const float*>(W.pts);
                 const int o = 4 * (i >> 1) + (i & 1);
@@ -1032,11 +1033,13 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
                 for (int t = 0; t < K; ++t) ct.cand -= nn.d[t] > cap && nn.d[t] < INFINITY;
             }
         }
-        if (!scanned)
+        if (!CELLS || !scanned)
             search<K, EXACT>(nn, q, W, lane, ct, pts, snodes, a, st, act, cap, (int32_t)u, (int32_t)sw0, (int32_t)sw1, e0,
                              e1, steps);
-        else
+        else {
             merge_fresh(nn, q, W, lane, ct);
+            prune(q, nn.tau, K, W, lane, ct);
+        }
         if (attempt == 0) {
             // a lane the cell scan could not serve (its cap is +inf or not a
             // number) was offered nothing: search it again as a miss
@@ -1047,7 +1050,6 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
             if (!__any_sync(FULL, act)) break;
         }
     }
-    if (__any_sync(FULL, q.n > K)) prune(q, nn.tau, K, W, lane, ct);
     {
         const unsigned cand = __reduce_add_sync(FULL, (unsigned)ct.cand);
         const unsigned ins = __reduce_add_sync(FULL, (unsigned)ct.ins);
