@@ -421,8 +421,7 @@ int se_destroy(se_ctx* c) {
     void* obufs[] = {c->q_order.keys0, c->q_order.keys1, c->q_order.lookback, c->q_order.st};
     for (void* p : obufs)
         if (p) cudaFree(p);
-    float* mlp_bufs[] = {c->mlp, c->mlp_m, c->mlp_v, c->mlp_g, c->mlp_loss, c->r2_buf, c->xs_buf,
-                         c->mw.yhat, c->mw.h1, c->mw.h2, c->mw.dy, c->mw.dh1, c->mw.dh2};
+    float* mlp_bufs[] = {c->mlp, c->mlp_m, c->mlp_v, c->mlp_g, c->mlp_loss, c->r2_buf, c->xs_buf, c->losses_buf};
     for (float* p : mlp_bufs)
         if (p) cudaFree(p);
     if (c->lut_buf) cudaFree(c->lut_buf);

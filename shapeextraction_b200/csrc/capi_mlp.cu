@@ -31,18 +31,6 @@ int mlp_alloc(se_ctx* c) {
     return SE_OK;
 }
 
-int mlp_work(se_ctx* c, int64_t n) {
-    if (n <= c->mw_cap) return SE_OK;
-    SE_CUDA(c, regrow(c->mw.yhat, n), "alloc mlp work");
-    SE_CUDA(c, regrow(c->mw.h1, n * kMlpH), "alloc mlp work");
-    SE_CUDA(c, regrow(c->mw.h2, n * kMlpH), "alloc mlp work");
-    SE_CUDA(c, regrow(c->mw.dy, n), "alloc mlp work");
-    SE_CUDA(c, regrow(c->mw.dh1, n * kMlpH), "alloc mlp work");
-    SE_CUDA(c, regrow(c->mw.dh2, n * kMlpH), "alloc mlp work");
-    c->mw_cap = n;
-    return SE_OK;
-}
-
 // Device pointer for n floats given by the caller: host data goes through the
 // context's staging buffer at float offset `off` (the buffer holds `total`).
 int stage_in(se_ctx* c, const float* src, int64_t n, int mem, int64_t off, int64_t total, const float** out) {
@@ -206,11 +194,13 @@ int se_mlp_grad(se_ctx* c, const float* features, const float* targets, int64_t 
     if (int rc = check_mem(c, mem)) return rc;
     if (!c->mlp_ready) return fail(c, SE_ERR_NOT_BUILT, "model not initialised");
     if (n < 1 || !features || !targets) return fail(c, SE_ERR_INVALID_ARG, "bad arguments");
-    if (int rc = mlp_work(c, n)) return rc;
     const float *X, *Y;
     if (int rc = stage_in(c, features, n * kMlpF, mem, 0, n * kMlpF + n, &X)) return rc;
     if (int rc = stage_in(c, targets, n, mem, n * kMlpF, n * kMlpF + n, &Y)) return rc;
-    SE_CUDA(c, enqueue_mlp_grad(c->mlp, X, Y, n, c->mlp_tau, c->mw, c->mlp_g, c->mlp_loss, c->stream), "launch grad");
+    SE_CUDA(c, cudaMemsetAsync(c->mlp_g, 0, sizeof(float) * kMlpParams, c->stream), "clear gradients");
+    SE_CUDA(c, cudaMemsetAsync(c->mlp_loss, 0, sizeof(float), c->stream), "clear loss");
+    SE_CUDA(c, enqueue_mlp_grad(c->mlp, X, Y, n, c->mlp_tau, c->mlp_g, c->mlp_loss, c->stream, c->num_sms),
+            "launch grad");
     const cudaMemcpyKind k = mem == SE_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
     if (grads) SE_CUDA(c, cudaMemcpyAsync(grads, c->mlp_g, sizeof(float) * kMlpParams, k, c->stream), "copy grads");
     if (loss) SE_CUDA(c, cudaMemcpyAsync(loss, c->mlp_loss, sizeof(float), k, c->stream), "copy loss");
@@ -227,29 +217,27 @@ int se_mlp_train(se_ctx* c, const float* features, const float* targets, int64_t
     if (n < 1 || steps < 0 || batch < 1 || !features || !targets || !(lr > 0.0f))
         return fail(c, SE_ERR_INVALID_ARG, "bad arguments");
     if (batch > n) batch = (int)n;
-    if (int rc = mlp_work(c, batch)) return rc;
     const float *X, *Y;
     if (int rc = stage_in(c, features, n * kMlpF, mem, 0, n * kMlpF + n, &X)) return rc;
     if (int rc = stage_in(c, targets, n, mem, n * kMlpF, n * kMlpF + n, &Y)) return rc;
-    float* dloss = nullptr;
-    if (losses) {
-        SE_CUDA(c, regrow(dloss, steps > 0 ? steps : 1), "alloc losses");
+    if (losses && c->losses_cap < steps) {
+        SE_CUDA(c, regrow(c->losses_buf, steps), "alloc losses");
+        c->losses_cap = steps;
     }
+    float* dloss = losses ? c->losses_buf : nullptr;
+    if (dloss && steps > 0) SE_CUDA(c, cudaMemsetAsync(dloss, 0, sizeof(float) * steps, c->stream), "clear losses");
+    SE_CUDA(c, cudaMemsetAsync(c->mlp_g, 0, sizeof(float) * kMlpParams, c->stream), "clear gradients");
     int64_t row = 0;
     for (int it = 0; it < steps; ++it) {
         if (row + batch > n) row = 0;
-        SE_CUDA(c, enqueue_mlp_grad(c->mlp, X + row * kMlpF, Y + row, batch, c->mlp_tau, c->mw, c->mlp_g,
-                                    dloss ? dloss + it : c->mlp_loss, c->stream),
+        SE_CUDA(c, enqueue_mlp_grad(c->mlp, X + row * kMlpF, Y + row, batch, c->mlp_tau, c->mlp_g,
+                                    dloss ? dloss + it : c->mlp_loss, c->stream, c->num_sms),
                 "launch grad");
         SE_CUDA(c, enqueue_adam(c->mlp, c->mlp_g, c->mlp_m, c->mlp_v, lr, ++c->mlp_step, c->stream), "launch adam");
         row += batch;
     }
-    if (dloss) {
-        cudaError_t e = cudaMemcpyAsync(losses, dloss, sizeof(float) * steps, cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        cudaFree(dloss);
-        if (e != cudaSuccess) return cuda_fail(c, e, "copy losses");
-    }
+    if (dloss && steps > 0)
+        SE_CUDA(c, cudaMemcpyAsync(losses, dloss, sizeof(float) * steps, cudaMemcpyDeviceToHost, c->stream), "copy losses");
     SE_CUDA(c, cudaStreamSynchronize(c->stream), "synchronize");
     return SE_OK;
 }

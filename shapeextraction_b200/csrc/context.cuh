@@ -75,8 +75,8 @@ struct se_ctx {
     float mlp_margin = 0.0f;
     float mlp_tau = 0.0f;  // training loss: 0 squared error, else the pinball loss of this quantile
     bool mlp_ready = false;
-    MlpWork mw{};
-    int64_t mw_cap = 0;
+    float* losses_buf = nullptr;  // losses of a training call's steps
+    int64_t losses_cap = 0;
     float* r2_buf = nullptr;
     int64_t r2_cap = 0;
     // code-range table of the current build for the learned cell scan

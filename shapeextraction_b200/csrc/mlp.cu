@@ -137,11 +137,13 @@ __global__ void __launch_bounds__(128) k_mlp_forward(const float* __restrict__ p
 }
 
 // Adam (Kingma & Ba, 2015) on the FP32 master parameters.
-__global__ void k_adam(float* __restrict__ params, const float* __restrict__ grads, float* __restrict__ m,
+// Clears the gradients it has used for the next step to add to.
+__global__ void k_adam(float* __restrict__ params, float* __restrict__ grads, float* __restrict__ m,
                        float* __restrict__ v, int np, float lr, float b1, float b2, float eps, float c1, float c2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
     const float g = grads[i];
+    grads[i] = 0.0f;
     const float mi = b1 * m[i] + (1.0f - b1) * g;
     const float vi = b2 * v[i] + (1.0f - b2) * g * g;
     m[i] = mi;
@@ -301,31 +303,34 @@ __global__ void __launch_bounds__(128) k_predict_radius(const float* __restrict_
 // ---------------------------------------------------------------------------
 // Training step on the tensor cores: forward, backward and weight gradients of
 // the loss (mean squared error, or with tau > 0 the pinball loss of quantile
-// tau) for one batch in one kernel. A warp takes 32 rows at
-// a time: both hidden layers, dh1 = (h1 > 0) * (dh2 W2^T) and the weight
-// gradients dW1 = X^T dh1 and dW2 = h1^T dh2 (K = the 32 rows) are
-// mma.sync.m16n8k16 products over BF16 tiles in shared memory (row-major tiles
-// for the layers, transposed ones for the gradients) with FP32 accumulation;
-// dh1 and dh2 enter the weight gradients rounded to BF16, the bias gradients
-// unrounded. Each warp's gradient tiles are added to the FP32 gradient
-// vector with reductions; the bias, w3 and loss terms are reduced across the
-// warp first.
+// tau) for one batch in one kernel. A block takes 64 rows at a time, 16 per
+// warp: both hidden layers and dh1 = (h1 > 0) * (dh2 W2^T) are mma.sync.m16n8k16
+// products of the warp's rows; the weight gradients dW1 = X^T dh1 and
+// dW2 = h1^T dh2 (K = the block's 64 rows) are split over the warps by output
+// tile, so that each element leaves the block once, accumulated over all its
+// rows, in one reduction. BF16 tiles in shared memory (row-major for the layers,
+// transposed for the gradients), FP32 accumulation; dh1 and dh2 enter the
+// weight gradients rounded to BF16, the bias gradients unrounded.
+//
+// A step is short and latency-bound: an 8192-row batch is 128 blocks. With 32
+// rows per warp and every warp adding its own gradient tiles to global memory
+// (64 blocks, twice the reductions) the kernel took 29.4 us, now 14.4 us; a step
+// with Adam, which clears the gradients for the next, 33.7 us and 16.4 us.
 // ---------------------------------------------------------------------------
+constexpr int kTrainRows = 64;  // rows of a block at a time
 struct MlpTrainSmem {
-    __nv_bfloat16 w1t[kMlpH][kMlpF + 8];  // forward layer 1: [out][in]
-    __nv_bfloat16 w2t[kMlpH][kMlpH + 8];  // forward layer 2: [out][in]
-    __nv_bfloat16 w2n[kMlpH][kMlpH + 8];  // backward: W2 as stored, [in][out]
+    __nv_bfloat16 w1t[kMlpH][kMlpF + 8];        // forward layer 1: [out][in]
+    __nv_bfloat16 w2t[kMlpH][kMlpH + 8];        // forward layer 2: [out][in]
+    __nv_bfloat16 w2n[kMlpH][kMlpH + 8];        // backward: W2 as stored, [in][out]
+    __nv_bfloat16 x[kTrainRows][kMlpF + 8];     // [row][feature]
+    __nv_bfloat16 xt[kMlpF][kTrainRows + 8];    // [feature][row]
+    __nv_bfloat16 h1[kTrainRows][kMlpH + 8];    // [row][unit]
+    __nv_bfloat16 h1t[kMlpH][kTrainRows + 8];   // [unit][row]
+    __nv_bfloat16 d2[kTrainRows][kMlpH + 8];    // dh2 [row][unit]
+    __nv_bfloat16 d2t[kMlpH][kTrainRows + 8];
+    __nv_bfloat16 d1t[kMlpH][kTrainRows + 8];   // dh1 [unit][row]
     float b1[kMlpH], b2[kMlpH], w3[kMlpH];
-    struct Warp {
-        __nv_bfloat16 x[32][kMlpF + 8];   // [row][feature]
-        __nv_bfloat16 xt[kMlpF][32 + 8];  // [feature][row]
-        __nv_bfloat16 h1[32][kMlpH + 8];  // [row][unit]
-        __nv_bfloat16 h1t[kMlpH][32 + 8]; // [unit][row]
-        __nv_bfloat16 d2[32][kMlpH + 8];  // dh2 [row][unit]
-        __nv_bfloat16 d2t[kMlpH][32 + 8];
-        __nv_bfloat16 d1t[kMlpH][32 + 8]; // dh1 [unit][row]
-        float sums[3][kMlpH];             // this warp's b1, b2 and w3 gradient sums
-    } w[4];
+    float sums[4][3][kMlpH];                    // each warp's b1, b2 and w3 gradient sums
 };
 
 // Sum v over the 8 row groups of the lanes (lanes with the same t), and add
@@ -344,20 +349,45 @@ __device__ __forceinline__ void add_columns(float (&v)[16], float* __restrict__ 
     }
 }
 
-// grads[base + row * kMlpH + col] += acc (the 32 x 64 product of mma_layer),
-// rows offset by row0.
-__device__ __forceinline__ void add_tile(float* __restrict__ grads, int base, int row0, const float (&acc)[2][8][4],
-                                         int lane) {
+// acc += a[row0 .. row0 + 16) * b[col0 .. col0 + 8 NB)^T over K, both stored
+// K-contiguous.
+template <int K, int NB, int LDA, int LDB>
+__device__ __forceinline__ void mma_tile(const __nv_bfloat16 (*a)[LDA], int row0, const __nv_bfloat16 (*b)[LDB], int col0,
+                                         int lane, float (&acc)[NB][4]) {
     const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int mb = 0; mb < 2; ++mb)
+    for (int kb = 0; kb < K / 16; ++kb) {
+        const int k0 = kb * 16 + 2 * t;
+        const uint32_t fa[4] = {ld_b32(&a[row0 + g][k0]), ld_b32(&a[row0 + g + 8][k0]), ld_b32(&a[row0 + g][k0 + 8]),
+                                ld_b32(&a[row0 + g + 8][k0 + 8])};
 #pragma unroll
-        for (int nb = 0; nb < 8; ++nb)
+        for (int nb = 0; nb < NB; ++nb) {
+            const int n0 = col0 + nb * 8 + g;
+            const uint32_t fb[2] = {ld_b32(&b[n0][k0]), ld_b32(&b[n0][k0 + 8])};
+            mma_bf16_16816(acc[nb], fa, fb);
+        }
+    }
+}
+
+template <int NB>
+__device__ __forceinline__ void clear(float (&acc)[NB][4]) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int row = row0 + mb * 16 + g + 8 * (e >> 1), col = nb * 8 + 2 * t + (e & 1);
-                atomicAdd(grads + base + row * kMlpH + col, acc[mb][nb][e]);
-            }
+    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[nb][e] = 0.0f;
+}
+
+// dst[row][col] += acc, the 16 x 8 NB tile at (row0, col0) of a kMlpH-wide
+// matrix, two columns per reduction.
+template <int NB>
+__device__ __forceinline__ void add_tile(float* __restrict__ dst, int row0, int col0, const float (&acc)[NB][4], int lane) {
+    const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            atomicAdd(reinterpret_cast<float2*>(dst + (row0 + g + 8 * h) * kMlpH + col0 + nb * 8 + 2 * t),
+                      make_float2(acc[nb][2 * h], acc[nb][2 * h + 1]));
 }
 
 __global__ void __launch_bounds__(128, 1) k_mlp_train_tc(const float* __restrict__ params,
@@ -366,149 +396,157 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train_tc(const float* __restrict
                                                          float* __restrict__ loss) {
     extern __shared__ __align__(16) unsigned char mlp_smem[];
     MlpTrainSmem& S = *reinterpret_cast<MlpTrainSmem*>(mlp_smem);
-    for (int i = threadIdx.x; i < kMlpF * kMlpH; i += blockDim.x) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    // rows of X go through registers as they come (8 threads per row, 16 rows a
+    // step); rows past n are zero
+    auto load_rows = [&](int64_t q0, float4 (&v)[4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int64_t r = q0 + 16 * i + (tid >> 3);
+            const float* p = X + r * kMlpF + 4 * (tid & 7);
+            v[i] = r < n ? make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3))
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    int64_t q0 = (int64_t)blockIdx.x * kTrainRows;
+    float4 xv[4];
+    load_rows(q0, xv);
+#pragma unroll 4
+    for (int i = tid; i < kMlpF * kMlpH; i += 128) {
         const int in = i / kMlpH, out = i % kMlpH;
         S.w1t[out][in] = __float2bfloat16_rn(params[MlpLayout::W1 + i]);
     }
-    for (int i = threadIdx.x; i < kMlpH * kMlpH; i += blockDim.x) {
+#pragma unroll 8
+    for (int i = tid; i < kMlpH * kMlpH; i += 128) {
         const int in = i / kMlpH, out = i % kMlpH;
         const __nv_bfloat16 v = __float2bfloat16_rn(params[MlpLayout::W2 + i]);
         S.w2t[out][in] = v;
         S.w2n[in][out] = v;
     }
-    for (int i = threadIdx.x; i < kMlpH; i += blockDim.x) {
+    for (int i = tid; i < kMlpH; i += 128) {
         S.b1[i] = params[MlpLayout::B1 + i];
         S.b2[i] = params[MlpLayout::B2 + i];
         S.w3[i] = bf16r(params[MlpLayout::W3 + i]);
     }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    MlpTrainSmem::Warp& T = S.w[warp];
+    for (int i = tid; i < 4 * 3 * kMlpH; i += 128) (&S.sums[0][0][0])[i] = 0.0f;
     const float b3 = params[MlpLayout::B3];
     const float inv_n = 1.0f / (float)n;
-    for (int i = lane; i < 3 * kMlpH; i += 32) (&T.sums[0][0])[i] = 0.0f;
-    __syncwarp();
+    const int r0 = 16 * warp;  // the warp's rows, and its rows of dW2
+    float gw1[4][4], gw2[8][4];
+    clear(gw1);
+    clear(gw2);
     float db3 = 0.0f, lsum = 0.0f;
-    for (int64_t chunk = blockIdx.x;; chunk += gridDim.x) {
-        const int64_t q0 = (chunk * 4 + warp) * 32;
-        if (q0 >= n) break;
-        {
-            const int64_t r = q0 + lane;
-            const bool valid = r < n;
-#pragma unroll 8
-            for (int j = 0; j < kMlpF; ++j) {
-                const __nv_bfloat16 b = __float2bfloat16_rn(valid ? __ldg(X + r * kMlpF + j) : 0.0f);
-                T.x[lane][j] = b;
-                T.xt[j][lane] = b;
+    for (; q0 < n; q0 += (int64_t)gridDim.x * kTrainRows) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = 16 * i + (tid >> 3), f = 4 * (tid & 7);
+            const float v[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const __nv_bfloat16 b = __float2bfloat16_rn(v[j]);
+                S.x[r][f + j] = b;
+                S.xt[f + j][r] = b;
             }
         }
-        __syncwarp();
-        float acc[2][8][4];
-        mma_layer<kMlpF>(T.x, S.w1t, lane, acc);
+        __syncthreads();
+        load_rows(q0 + (int64_t)gridDim.x * kTrainRows, xv);  // the next chunk's
+        float acc[8][4];
+        clear(acc);
+        mma_tile<kMlpF>(S.x, r0, S.w1t, 0, lane, acc);
 #pragma unroll
-        for (int mb = 0; mb < 2; ++mb)
+        for (int nb = 0; nb < 8; ++nb)
 #pragma unroll
-            for (int nb = 0; nb < 8; ++nb)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int row = mb * 16 + g + 8 * (e >> 1), col = nb * 8 + 2 * t + (e & 1);
-                    const __nv_bfloat16 h = __float2bfloat16_rn(fmaxf(acc[mb][nb][e] + S.b1[col], 0.0f));
-                    T.h1[row][col] = h;
-                    T.h1t[col][row] = h;
-                }
-        __syncwarp();
-        mma_layer<kMlpH>(T.h1, S.w2t, lane, acc);
-        float y[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll
-        for (int mb = 0; mb < 2; ++mb)
-#pragma unroll
-            for (int nb = 0; nb < 8; ++nb)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int col = nb * 8 + 2 * t + (e & 1);
-                    const float h2 = bf16r(fmaxf(acc[mb][nb][e] + S.b2[col], 0.0f));
-                    acc[mb][nb][e] = h2;
-                    y[mb][e >> 1] = fmaf(h2, S.w3[col], y[mb][e >> 1]);
-                }
-        float dy[2][2];
-#pragma unroll
-        for (int mb = 0; mb < 2; ++mb)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float v = y[mb][h];
-                v += __shfl_xor_sync(FULL, v, 1);
-                v += __shfl_xor_sync(FULL, v, 2);
-                const int64_t o = q0 + mb * 16 + g + 8 * h;
-                const float err = o < n ? v + b3 - __ldg(Y + o) : 0.0f;
-                float l;
-                if (tau > 0.0f) {  // pinball loss at quantile tau: tau (y - yhat)+ + (1 - tau) (yhat - y)+
-                    dy[mb][h] = (err > 0.0f ? 1.0f - tau : (err < 0.0f ? -tau : 0.0f)) * inv_n;
-                    l = (err > 0.0f ? (1.0f - tau) * err : -tau * err) * inv_n;
-                } else {  // mean squared error
-                    dy[mb][h] = 2.0f * err * inv_n;
-                    l = err * err * inv_n;
-                }
-                if (t == 0) {
-                    lsum += l;
-                    db3 += dy[mb][h];
-                }
+            for (int e = 0; e < 4; ++e) {
+                const int row = r0 + g + 8 * (e >> 1), col = nb * 8 + 2 * t + (e & 1);
+                const __nv_bfloat16 h = __float2bfloat16_rn(fmaxf(acc[nb][e] + S.b1[col], 0.0f));
+                S.h1[row][col] = h;
+                S.h1t[col][row] = h;
             }
+        __syncwarp();
+        clear(acc);
+        mma_tile<kMlpH>(S.h1, r0, S.w2t, 0, lane, acc);
+        float y[2] = {0.f, 0.f};
+#pragma unroll
+        for (int nb = 0; nb < 8; ++nb)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int col = nb * 8 + 2 * t + (e & 1);
+                const float h2 = bf16r(fmaxf(acc[nb][e] + S.b2[col], 0.0f));
+                acc[nb][e] = h2;
+                y[e >> 1] = fmaf(h2, S.w3[col], y[e >> 1]);
+            }
+        float dy[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float v = y[h];
+            v += __shfl_xor_sync(FULL, v, 1);
+            v += __shfl_xor_sync(FULL, v, 2);
+            const int64_t o = q0 + r0 + g + 8 * h;
+            const float err = o < n ? v + b3 - __ldg(Y + o) : 0.0f;
+            float l;
+            if (tau > 0.0f) {  // pinball loss at quantile tau: tau (y - yhat)+ + (1 - tau) (yhat - y)+
+                dy[h] = (err > 0.0f ? 1.0f - tau : (err < 0.0f ? -tau : 0.0f)) * inv_n;
+                l = (err > 0.0f ? (1.0f - tau) * err : -tau * err) * inv_n;
+            } else {  // mean squared error
+                dy[h] = 2.0f * err * inv_n;
+                l = err * err * inv_n;
+            }
+            if (t == 0) {
+                lsum += l;
+                db3 += dy[h];
+            }
+        }
         // dh2 = (h2 > 0) * dy * w3; w3 and b2 gradients (per lane: columns nb * 8 + 2t + b)
         float db2[16], dw3[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) db2[i] = dw3[i] = 0.0f;
 #pragma unroll
-        for (int mb = 0; mb < 2; ++mb)
+        for (int nb = 0; nb < 8; ++nb)
 #pragma unroll
-            for (int nb = 0; nb < 8; ++nb)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int row = mb * 16 + g + 8 * (e >> 1), col = nb * 8 + 2 * t + (e & 1);
-                    const float h2 = acc[mb][nb][e], d = dy[mb][e >> 1];
-                    const float d2 = h2 > 0.0f ? d * S.w3[col] : 0.0f;
-                    db2[nb * 2 + (e & 1)] += d2;
-                    dw3[nb * 2 + (e & 1)] = fmaf(d, h2, dw3[nb * 2 + (e & 1)]);
-                    const __nv_bfloat16 b = __float2bfloat16_rn(d2);
-                    T.d2[row][col] = b;
-                    T.d2t[col][row] = b;
-                }
-        add_columns(db2, T.sums[1], lane);
-        add_columns(dw3, T.sums[2], lane);
+            for (int e = 0; e < 4; ++e) {
+                const int row = r0 + g + 8 * (e >> 1), col = nb * 8 + 2 * t + (e & 1);
+                const float h2 = acc[nb][e], d = dy[e >> 1];
+                const float d2 = h2 > 0.0f ? d * S.w3[col] : 0.0f;
+                db2[nb * 2 + (e & 1)] += d2;
+                dw3[nb * 2 + (e & 1)] = fmaf(d, h2, dw3[nb * 2 + (e & 1)]);
+                const __nv_bfloat16 b = __float2bfloat16_rn(d2);
+                S.d2[row][col] = b;
+                S.d2t[col][row] = b;
+            }
+        add_columns(db2, S.sums[warp][1], lane);
+        add_columns(dw3, S.sums[warp][2], lane);
         __syncwarp();
         // dh1 = (h1 > 0) * (dh2 W2^T)
-        mma_layer<kMlpH>(T.d2, S.w2n, lane, acc);
+        clear(acc);
+        mma_tile<kMlpH>(S.d2, r0, S.w2n, 0, lane, acc);
         float db1[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) db1[i] = 0.0f;
 #pragma unroll
-        for (int mb = 0; mb < 2; ++mb)
+        for (int nb = 0; nb < 8; ++nb)
 #pragma unroll
-            for (int nb = 0; nb < 8; ++nb)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int row = mb * 16 + g + 8 * (e >> 1), col = nb * 8 + 2 * t + (e & 1);
-                    const float d1 = __bfloat162float(T.h1[row][col]) > 0.0f ? acc[mb][nb][e] : 0.0f;
-                    db1[nb * 2 + (e & 1)] += d1;
-                    T.d1t[col][row] = __float2bfloat16_rn(d1);
-                }
-        add_columns(db1, T.sums[0], lane);
-        __syncwarp();
-        // weight gradients of these 32 rows
-        mma_layer<32>(T.xt, T.d1t, lane, acc);
-        add_tile(grads, MlpLayout::W1, 0, acc, lane);
-        mma_layer<32>(T.h1t, T.d2t, lane, acc);
-        add_tile(grads, MlpLayout::W2, 0, acc, lane);
-        mma_layer<32>(T.h1t + 32, T.d2t, lane, acc);
-        add_tile(grads, MlpLayout::W2, 32, acc, lane);
-        __syncwarp();  // this warp's tiles are rewritten by its next chunk
+            for (int e = 0; e < 4; ++e) {
+                const int row = r0 + g + 8 * (e >> 1), col = nb * 8 + 2 * t + (e & 1);
+                const float d1 = __bfloat162float(S.h1[row][col]) > 0.0f ? acc[nb][e] : 0.0f;
+                db1[nb * 2 + (e & 1)] += d1;
+                S.d1t[col][row] = __float2bfloat16_rn(d1);
+            }
+        add_columns(db1, S.sums[warp][0], lane);
+        __syncthreads();
+        // weight gradients of the block's rows: 16 rows of dW2 per warp, and a
+        // quarter of dW1
+        mma_tile<kTrainRows>(S.h1t, r0, S.d2t, 0, lane, gw2);
+        mma_tile<kTrainRows>(S.xt, 16 * (warp & 1), S.d1t, 32 * (warp >> 1), lane, gw1);
+        __syncthreads();  // the tiles are rewritten by the next chunk
     }
-    // this warp's column sums: one reduction per column
-    __syncwarp();
-    for (int i = lane; i < kMlpH; i += 32) {
-        atomicAdd(grads + MlpLayout::B1 + i, T.sums[0][i]);
-        atomicAdd(grads + MlpLayout::B2 + i, T.sums[1][i]);
-        atomicAdd(grads + MlpLayout::W3 + i, T.sums[2][i]);
+    add_tile(grads + MlpLayout::W2, r0, 0, gw2, lane);
+    add_tile(grads + MlpLayout::W1, 16 * (warp & 1), 32 * (warp >> 1), gw1, lane);
+    __syncthreads();
+    for (int i = tid; i < 3 * kMlpH; i += 128) {
+        const int which = i / kMlpH, c = i % kMlpH;
+        const int at = which == 0 ? MlpLayout::B1 : (which == 1 ? MlpLayout::B2 : MlpLayout::W3);
+        atomicAdd(grads + at + c, S.sums[0][which][c] + S.sums[1][which][c] + S.sums[2][which][c] + S.sums[3][which][c]);
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -557,25 +595,19 @@ cudaError_t enqueue_mlp_forward(const float* params, const float* X, int64_t n, 
     return cudaGetLastError();
 }
 
-cudaError_t enqueue_mlp_grad(const float* params, const float* X, const float* y, int64_t n, float tau,
-                             MlpWork& /*w*/, float* grads, float* loss, cudaStream_t s) {
-    cudaMemsetAsync(grads, 0, sizeof(float) * kMlpParams, s);
-    cudaMemsetAsync(loss, 0, sizeof(float), s);
+cudaError_t enqueue_mlp_grad(const float* params, const float* X, const float* y, int64_t n, float tau, float* grads,
+                             float* loss, cudaStream_t s, int num_sms) {
     if (n <= 0) return cudaGetLastError();
     constexpr int smem = (int)sizeof(MlpTrainSmem);
     cudaError_t e = cudaFuncSetAttribute(k_mlp_train_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    const int64_t want = (n + 127) / 128;  // 4 warps x 32 rows per block and pass
-    const unsigned blocks = (unsigned)(want < sms ? want : (sms > 0 ? sms : 1));
+    const int64_t want = (n + kTrainRows - 1) / kTrainRows;
+    const unsigned blocks = (unsigned)(want < 2 * num_sms ? want : 2 * num_sms);
     k_mlp_train_tc<<<blocks, 128, smem, s>>>(params, X, y, n, tau, grads, loss);
     return cudaGetLastError();
 }
 
-cudaError_t enqueue_adam(float* params, const float* grads, float* m, float* v, float lr, int step, cudaStream_t s) {
+cudaError_t enqueue_adam(float* params, float* grads, float* m, float* v, float lr, int step, cudaStream_t s) {
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
     k_adam<<<blocks_for(kMlpParams, 256), 256, 0, s>>>(params, grads, m, v, kMlpParams, lr, b1, b2, 1e-8f, c1, c2);

@@ -186,25 +186,17 @@ struct MlpLayout {
 };
 constexpr int kMlpParams = MlpLayout::N;
 
-// Training work arrays for n samples.
-struct MlpWork {
-    float* yhat;  // n
-    float* h1;    // n x kMlpH
-    float* h2;    // n x kMlpH
-    float* dy;    // n
-    float* dh1;   // n x kMlpH
-    float* dh2;   // n x kMlpH
-};
-
 cudaError_t enqueue_features(const BuildBufs& b, int64_t u, int code_bits, int64_t start, int64_t count, float* out,
                              cudaStream_t s);
 cudaError_t enqueue_predict_radius(const BuildBufs& b, const float* params, float margin, int64_t u, int code_bits,
                                    int64_t start, int64_t count, float* r2_out, float* yhat_out, cudaStream_t s);
 cudaError_t enqueue_mlp_forward(const float* params, const float* X, int64_t n, float* yhat, float* h1, float* h2,
                                 cudaStream_t s);
-cudaError_t enqueue_mlp_grad(const float* params, const float* X, const float* y, int64_t n, float tau, MlpWork& w,
-                             float* grads, float* loss, cudaStream_t s);
-cudaError_t enqueue_adam(float* params, const float* grads, float* m, float* v, float lr, int step, cudaStream_t s);
+// Adds the gradient of a batch to grads and its loss to *loss (both start at zero).
+cudaError_t enqueue_mlp_grad(const float* params, const float* X, const float* y, int64_t n, float tau, float* grads,
+                             float* loss, cudaStream_t s, int num_sms);
+// One Adam step; leaves grads at zero.
+cudaError_t enqueue_adam(float* params, float* grads, float* m, float* v, float lr, int step, cudaStream_t s);
 
 // Sort n 64-bit keys in place in `keys` (ascending) with the onesweep passes;
 // `tmp` (n keys), `lookback` (kSortBins words per 4096-key tile) and `st` are scratch.
