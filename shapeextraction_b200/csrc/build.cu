@@ -726,10 +726,13 @@ __device__ __forceinline__ void root_parent(const int32_t* __restrict__ left_chi
 // prefix that codes i - 1 and i share. So with w(a) = the common prefix of
 // codes a and a + M, point i starts a leaf when the largest w(a) over a in
 // [i - M, i - 1] is at least the common prefix of codes i - 1 and i: a sliding
-// maximum in shared memory (doubling windows), one ballot per 32 codes, and a
-// decoupled look-back over the tiles' leaf counts. With k_boxes it takes
-// 0.294 ms on 13M codes (20M precision mix), where merging the boxes of a
-// binary tree bottom-up took 0.530 ms; it reads no radix tree, so batched
+// maximum, one ballot per 32 codes, and a decoupled look-back over the tiles'
+// leaf counts. For M = 32 the maximum takes shuffles alone; smaller M (a small
+// leaf_bucket) takes doubling windows in shared memory. On 13M codes (20M
+// precision mix) this and k_boxes take 0.220 ms (0.288 ms with the shared-memory
+// windows and 1024-code tiles; 4096-code tiles 0.200 ms, but 2 us more on a 2k
+// cloud), where merging the boxes of a binary tree bottom-up took 0.530 ms; it
+// reads no radix tree, so batched
 // builds make none. M is at most 32, one point per lane of the scan: of the
 // layouts simulated on 400k-point clouds (fixed runs of 16, 32 and 64 points,
 // runs cut at the best prefix, subtrees of at most 32 and 96) subtrees of at
@@ -746,7 +749,8 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaves(const uint64_t* __restr
                                                          int spin_limit) {
     constexpr int kHalo = kLeafMax, kSpan = kLeafTile + 2 * kHalo;
     constexpr int kCells = kLeafIpt * kLeafThreads / 32;  // 32-code steps of a tile
-    static_assert(kCells == 32, "one warp scans the steps' counts");
+    constexpr int kPerLane = kCells / 32;  // counts of steps per lane of the scanning warp
+    static_assert(kCells % 32 == 0, "one warp scans the steps' counts");
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ uint64_t s_code[kSpan];   // codes [t0 - kHalo, t0 + kLeafTile + kHalo)
     __shared__ int8_t s_w[2][kSpan];     // window maxima of w, ping-pong
@@ -760,38 +764,80 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaves(const uint64_t* __restr
     const int64_t t0 = (int64_t)tile * kLeafTile;
     if (root_compat && tile == 0 && tid == 0) root_parent(left_child, parent, hll, hlr, u, st);
     if (t0 >= u) return;
-    for (int j = tid; j < kSpan; j += kLeafThreads) {
-        const int64_t i = t0 - kHalo + j;
-        s_code[j] = i >= 0 && i < u ? codes[i] : 0ull;
-    }
-    __syncthreads();
-    for (int j = tid; j < kSpan; j += kLeafThreads) {
-        const int64_t a = t0 - kHalo + j;
-        s_w[0][j] = a >= 0 && j + M < kSpan && a + M < u ? (int8_t)__clzll((long long)(s_code[j] ^ s_code[j + M])) : -1;
-    }
-    __syncthreads();
-    int p = 1, cur = 0;  // s_w[cur][j] = the largest w over [j, j + p)
-    for (; 2 * p <= M; p *= 2, cur ^= 1) {
-        for (int j = tid; j < kSpan; j += kLeafThreads)
-            s_w[cur ^ 1][j] = j + p < kSpan ? max(s_w[cur][j], s_w[cur][j + p]) : s_w[cur][j];
-        __syncthreads();
-    }
+    // warp by warp, 32 codes a step: step r of the warp starts at this code
+    const int64_t at = t0 + (int64_t)warp * 32 * kLeafIpt;
     uint32_t flags[kLeafIpt];
+    if (M == kHalo) {
+        // w of a step's codes needs the next step's code on the same lane only,
+        // and the window [i - 32, i - 1] is the end of the step before and the
+        // start of this one: a suffix and a prefix maximum by shuffles
+        uint64_t c = at + lane >= 32 && at + lane - 32 < u ? codes[at + lane - 32] : 0ull;
+        uint64_t next = at + lane < u ? codes[at + lane] : 0ull;
+        int before = -1;     // the suffix maximum of the step before
+        uint64_t last = 0;   // its last code
 #pragma unroll
-    for (int r = 0; r < kLeafIpt; ++r) {
-        const int e = r * kLeafThreads + tid, j = kHalo + e;
-        const int64_t i = t0 + e;
-        bool f = i < u;
-        if (f && i > 0) {
-            const int d = __clzll((long long)(s_code[j - 1] ^ s_code[j]));
-            f = max(s_w[cur][j - M], s_w[cur][j - p]) >= d;
+        for (int r = -1; r < kLeafIpt; ++r) {
+            const int64_t i = at + 32 * r + lane;
+            int w = i >= 0 && i + 32 < u ? __clzll((long long)(c ^ next)) : -1;
+            int pre = __shfl_up_sync(kFull, w, 1);
+            if (lane == 0) pre = -1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(kFull, pre, o);
+                pre = lane >= o ? max(pre, v) : pre;
+                const int x = __shfl_down_sync(kFull, w, o);
+                w = lane + o < 32 ? max(w, x) : w;
+            }
+            uint64_t prev = __shfl_up_sync(kFull, c, 1);
+            if (lane == 0) prev = last;
+            last = __shfl_sync(kFull, c, 31);
+            if (r >= 0) {
+                const int d = __clzll((long long)(prev ^ c));
+                const bool f = i < u && (i == 0 || max(before, pre) >= d);
+                flags[r] = __ballot_sync(kFull, f);
+                if (lane == 0) s_cnt[warp * kLeafIpt + r] = __popc(flags[r]);
+            }
+            before = w;
+            c = next;
+            const int64_t n2 = i + 64;
+            next = r + 1 < kLeafIpt && n2 < u ? codes[n2] : 0ull;
         }
-        flags[r] = __ballot_sync(kFull, f);
-        if (lane == 0) s_cnt[r * (kLeafThreads / 32) + warp] = __popc(flags[r]);
+    } else {
+        for (int j = tid; j < kSpan; j += kLeafThreads) {
+            const int64_t i = t0 - kHalo + j;
+            s_code[j] = i >= 0 && i < u ? codes[i] : 0ull;
+        }
+        __syncthreads();
+        for (int j = tid; j < kSpan; j += kLeafThreads) {
+            const int64_t a = t0 - kHalo + j;
+            s_w[0][j] =
+                a >= 0 && j + M < kSpan && a + M < u ? (int8_t)__clzll((long long)(s_code[j] ^ s_code[j + M])) : -1;
+        }
+        __syncthreads();
+        int p = 1, cur = 0;  // s_w[cur][j] = the largest w over [j, j + p)
+        for (; 2 * p <= M; p *= 2, cur ^= 1) {
+            for (int j = tid; j < kSpan; j += kLeafThreads)
+                s_w[cur ^ 1][j] = j + p < kSpan ? max(s_w[cur][j], s_w[cur][j + p]) : s_w[cur][j];
+            __syncthreads();
+        }
+#pragma unroll
+        for (int r = 0; r < kLeafIpt; ++r) {
+            const int64_t i = at + 32 * r + lane;
+            const int j = kHalo + (int)(i - t0);
+            bool f = i < u;
+            if (f && i > 0) {
+                const int d = __clzll((long long)(s_code[j - 1] ^ s_code[j]));
+                f = max(s_w[cur][j - M], s_w[cur][j - p]) >= d;
+            }
+            flags[r] = __ballot_sync(kFull, f);
+            if (lane == 0) s_cnt[warp * kLeafIpt + r] = __popc(flags[r]);
+        }
     }
     __syncthreads();
     if (warp == 0) {
-        const uint32_t c = s_cnt[lane];
+        uint32_t c = 0;
+#pragma unroll
+        for (int e = 0; e < kPerLane; ++e) c += s_cnt[kPerLane * lane + e];
         const uint32_t inc = warp_incl_scan(c);
         const uint32_t tot = __shfl_sync(kFull, inc, 31);
         // look-back, 32 predecessors per step (as k_dedup)
@@ -821,7 +867,13 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaves(const uint64_t* __restr
             }
             if (lane == 0) st_relaxed(lookback + tile, LB_PRE | (excl + tot));
         }
-        s_cnt[lane] = excl + inc - c;
+        uint32_t first = excl + inc - c;
+#pragma unroll
+        for (int e = 0; e < kPerLane; ++e) {
+            const uint32_t mine = s_cnt[kPerLane * lane + e];
+            s_cnt[kPerLane * lane + e] = first;
+            first += mine;
+        }
         if (lane == 0 && t0 + kLeafTile >= u) {
             uint32_t n = excl + tot, off = 0;
             int l = 0;
@@ -839,8 +891,8 @@ __global__ void __launch_bounds__(kLeafThreads) k_leaves(const uint64_t* __restr
 #pragma unroll
     for (int r = 0; r < kLeafIpt; ++r) {
         if (!((flags[r] >> lane) & 1u)) continue;
-        const uint32_t pos = s_cnt[r * (kLeafThreads / 32) + warp] + __popc(flags[r] & lanemask_lt());
-        const int64_t i = t0 + r * kLeafThreads + tid;
+        const uint32_t pos = s_cnt[warp * kLeafIpt + r] + __popc(flags[r] & lanemask_lt());
+        const int64_t i = at + 32 * r + lane;
         if ((int64_t)pos < u) leaf_start[pos] = (int32_t)i;
         else set_err(&st->err, ERRBIT_BOUNDS);
     }

@@ -24,7 +24,7 @@ constexpr int kScanThreads = 256;
 constexpr int kScanIpt = 16;
 constexpr int kScanTile = kScanThreads * kScanIpt;
 constexpr int kLeafThreads = 256;
-constexpr int kLeafIpt = 4;
+constexpr int kLeafIpt = 8;
 constexpr int kLeafTile = kLeafThreads * kLeafIpt;
 // Search hierarchy: leaves of at most kLeafMax points, kFan nodes under each
 // inner node, at most kMaxLevels levels (32^6 leaves).
