@@ -1456,7 +1456,10 @@ cudaError_t enqueue_build(const BuildBufs& b, const BuildParams& p, cudaStream_t
     k_leaves<<<(unsigned)leaf_tiles, kLeafThreads, 0, s>>>(
         b.codes, p.bucket < kLeafMax ? p.bucket : kLeafMax, b.leaf_start, b.scratch + scratch.leaves,
         p.build_radix && p.root_compat, b.left_child, b.parent, b.has_leaf_left, b.has_leaf_right, b.st, p.spin_limit);
-    k_boxes<<<grid_for(n, 32 * 128, num_sms * 8), 128, 0, s>>>(b.pts4, b.leaf_start, b.scratch + scratch.arrivals,
+    // 32 leaves per warp, about 20 points each: a grid for four warps per 1024
+    // points (per 4096 the warps took several groups in turn: 100k points 32 us for
+    // leaves and boxes, now 26; 2M 62 and 50 us)
+    k_boxes<<<grid_for(n, 1024, num_sms * 8), 128, 0, s>>>(b.pts4, b.leaf_start, b.scratch + scratch.arrivals,
                                                                b.snodes, b.st);
     nl += 2;
     mark(6);
