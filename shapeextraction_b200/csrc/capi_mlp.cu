@@ -220,10 +220,7 @@ int se_mlp_train(se_ctx* c, const float* features, const float* targets, int64_t
     const float *X, *Y;
     if (int rc = stage_in(c, features, n * kMlpF, mem, 0, n * kMlpF + n, &X)) return rc;
     if (int rc = stage_in(c, targets, n, mem, n * kMlpF, n * kMlpF + n, &Y)) return rc;
-    if (losses && c->losses_cap < steps) {
-        SE_CUDA(c, regrow(c->losses_buf, steps), "alloc losses");
-        c->losses_cap = steps;
-    }
+    if (losses) SE_CUDA(c, grow(c->losses_cap, steps, Buf{c->losses_buf, steps}), "alloc losses");
     float* dloss = losses ? c->losses_buf : nullptr;
     if (dloss && steps > 0) SE_CUDA(c, cudaMemsetAsync(dloss, 0, sizeof(float) * steps, c->stream), "clear losses");
     SE_CUDA(c, cudaMemsetAsync(c->mlp_g, 0, sizeof(float) * kMlpParams, c->stream), "clear gradients");

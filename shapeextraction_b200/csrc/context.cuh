@@ -150,5 +150,27 @@ cudaError_t regrow(T*& p, int64_t count) {
     return cudaMalloc((void**)&p, sizeof(T) * (size_t)count);
 }
 
+// A grow-only buffer and the elements it should hold.
+template <typename T>
+struct Buf {
+    T*& p;
+    int64_t count;
+};
+template <typename T>
+Buf(T*&, int64_t) -> Buf<T>;
+
+// Buffers of one capacity, regrown together once `need` exceeds it. While any
+// of them may be missing the capacity is 0: after a failed allocation it would
+// otherwise still vouch for a buffer that has been freed.
+template <typename... T>
+cudaError_t grow(int64_t& cap, int64_t need, Buf<T>... bufs) {
+    if (need <= cap) return cudaSuccess;
+    cap = 0;
+    cudaError_t e = cudaSuccess;
+    ((e = e == cudaSuccess ? regrow(bufs.p, bufs.count) : e), ...);
+    if (e == cudaSuccess) cap = need;
+    return e;
+}
+
 }  // namespace capi
 }  // namespace shapex

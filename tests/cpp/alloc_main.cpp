@@ -1,0 +1,200 @@
+// Allocation failures inside the C ABI, on the CPU. The host code of the entry
+// points (capi.cu, capi_mlp.cu, capi_batch.cu: no kernels) is linked against
+// stand-ins for the CUDA runtime (alloc_runtime.cpp) and the kernel launchers
+// (below). Device memory is host memory, every launcher checks that each buffer it is handed is
+// alive and large enough and fills its outputs, and the runtime fails one
+// allocation of a call on request.
+//
+// A scenario is a small, a middle and a large call on one context. For every
+// allocation of the large call after the small one: that allocation fails, the
+// call says so, and the three calls then work.
+#include <cstdio>
+#include <functional>
+#include <string>
+#include <vector>
+
+#include "alloc_runtime.hpp"
+#include "pipeline.cuh"
+#include "shapex.h"
+
+using namespace shapex;
+using fake::complain;
+using fake::live;
+
+// ---- the kernel launchers ----------------------------------------------------
+namespace shapex {
+static void fill(float* p, int64_t n) {
+    for (int64_t i = 0; i < n; ++i) p[i] = 7.0f;
+}
+cudaError_t enqueue_build(const BuildBufs& b, const BuildParams& p, cudaStream_t, int, cudaEvent_t*, int* launches) {
+    const int64_t n = p.n;
+    if (launches) *launches = 1;
+    if (!live(b.st, sizeof(DevState), "build: st")) return cudaErrorInvalidValue;
+    *b.st = DevState{};
+    if (n == 0) return cudaSuccess;
+    bool ok = live(b.x, 4 * n, "build: x") && live(b.y, 4 * n, "build: y") && live(b.z, 4 * n, "build: z") &&
+              live(b.keys0, 8 * n, "build: keys0") && live(b.keys1, 8 * n, "build: keys1") &&
+              live(b.scratch, 4 * ScratchLayout(n).words(kCodePasses), "build: scratch") &&
+              live(b.codes, 8 * n, "build: codes") && live(b.pts4, 16 * n, "build: pts4") &&
+              live(b.pts3, 12 * n, "build: pts3") && live(b.leaf_start, 4 * n, "build: leaf_start") &&
+              live(b.snodes, sizeof(SNode) * hierarchy_nodes(n), "build: snodes");
+    if (ok && p.build_radix)
+        ok = live(b.left_child, 4 * n, "build: left_child") && live(b.parent, 4 * n, "build: parent") &&
+             live(b.prefix_n, n, "build: prefix_n") && live(b.has_leaf_left, n, "build: has_leaf_left") &&
+             live(b.has_leaf_right, n, "build: has_leaf_right") && live(b.sparent, 4 * n, "build: sparent") &&
+             live(b.leaf_parent, 4 * n, "build: leaf_parent") && live(b.range_end, 4 * n, "build: range_end");
+    if (ok && p.build_octree)
+        ok = live(b.oct_counts, 4 * n, "build: oct_counts") && live(b.oct_offsets, 4 * n + 4, "build: oct_offsets") &&
+             live(b.oct_nodes, sizeof(OtNode) * b.oct_cap, "build: oct_nodes");
+    if (!ok) return cudaErrorInvalidValue;
+    b.st->u = (unsigned long long)n;
+    b.st->n_oct = 1;
+    return cudaSuccess;
+}
+cudaError_t enqueue_octree(const BuildBufs&, const BuildParams&, cudaStream_t, int*) { return cudaSuccess; }
+int queries_per_warp(int64_t count, int, bool) { return count > 100 ? 32 : 1; }
+cudaError_t enqueue_query_order(const BuildBufs&, const QueryOrder& o, const float* q, int64_t n, int64_t, int,
+                                const uint64_t** order, int* shift, cudaStream_t, int, int* launches) {
+    const int64_t tiles = (n + kSortTile - 1) / kSortTile;
+    if (!(live(q, 12 * n, "order: queries") && live(o.keys0, 8 * n, "order: keys0") &&
+          live(o.keys1, 8 * n, "order: keys1") && live(o.lookback, 3 * 4 * tiles * kSortBins, "order: lookback") &&
+          live(o.st, sizeof(DevState), "order: st")))
+        return cudaErrorInvalidValue;
+    *order = o.keys0;
+    *shift = 0;
+    ++*launches;
+    return cudaSuccess;
+}
+cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t, int) {
+    bool ok = live(b.st, sizeof(DevState), "query: st") && live(b.pts4, 16 * q.u, "query: pts4") &&
+              live(b.snodes, sizeof(SNode), "query: snodes");
+    if (q.ext_queries) ok = live(q.ext_queries, 12 * q.count, "query: queries") && ok;
+    if (q.order) ok = live(q.order, 8 * q.count, "query: order") && ok;
+    if (q.learned_r2) ok = live(q.learned_r2, 4 * q.count, "query: learned_r2") && ok;
+    if (q.cell_lut) ok = live(q.cell_lut, 4, "query: cell_lut") && ok;
+    if (q.out_idx) ok = live(q.out_idx, 4 * q.k * q.count, "query: out_idx") && ok;
+    if (q.out_d2) ok = live(q.out_d2, 4 * q.k * q.count, "query: out_d2") && ok;
+    if (q.out_normals) ok = live(q.out_normals, 12 * q.count, "query: out_normals") && ok;
+    if (!ok) return cudaErrorInvalidValue;
+    for (int64_t i = 0; q.out_idx && i < q.k * q.count; ++i) q.out_idx[i] = 7;
+    if (q.out_d2) fill(q.out_d2, q.k * q.count);
+    if (q.out_normals) fill(q.out_normals, 3 * q.count);
+    return cudaSuccess;
+}
+cudaError_t enqueue_query_batch(const BatchCloud* clouds, int n_clouds, int64_t, unsigned long long* counter,
+                                const QueryParams&, cudaStream_t, int) {
+    if (!(live(clouds, sizeof(BatchCloud) * n_clouds, "batch: descriptors") && live(counter, 8, "batch: counter")))
+        return cudaErrorInvalidValue;
+    for (int i = 0; i < n_clouds; ++i) {
+        const BatchCloud& d = clouds[i];
+        if (!(live(d.st, sizeof(DevState), "batch: st") && live(d.pts, 16 * d.st->u, "batch: pts") &&
+              live(d.snodes, sizeof(SNode), "batch: snodes") && live(d.out_normals, 12 * d.st->u, "batch: out")))
+            return cudaErrorInvalidValue;
+        fill(d.out_normals, 3 * (int64_t)d.st->u);
+    }
+    return cudaSuccess;
+}
+cudaError_t enqueue_batch_collect(const DevState* st, int n, unsigned long long* u, uint32_t* err, cudaStream_t) {
+    for (int i = 0; i < n; ++i) {
+        u[i] = st[i].u;
+        err[i] = st[i].err;
+    }
+    return cudaSuccess;
+}
+cudaError_t enqueue_cell_lut(const BuildBufs&, int, int level, uint32_t* lut, cudaStream_t, int) {
+    return live(lut, 4 * (((int64_t)1 << (3 * level)) + 1), "cell table") ? cudaSuccess : cudaErrorInvalidValue;
+}
+cudaError_t enqueue_features(const BuildBufs&, int64_t, int, int64_t, int64_t count, float* out, cudaStream_t) {
+    if (!live(out, 4 * kMlpF * count, "features")) return cudaErrorInvalidValue;
+    fill(out, kMlpF * count);
+    return cudaSuccess;
+}
+cudaError_t enqueue_predict_radius(const BuildBufs&, const float* params, float, int64_t, int, int64_t, int64_t count,
+                                   float* r2, float* yhat, cudaStream_t) {
+    if (!live(params, 4 * kMlpParams, "predict: params")) return cudaErrorInvalidValue;
+    if (r2 && !live(r2, 4 * count, "predict: r2")) return cudaErrorInvalidValue;
+    if (yhat && !live(yhat, 4 * count, "predict: yhat")) return cudaErrorInvalidValue;
+    if (r2) fill(r2, count);
+    if (yhat) fill(yhat, count);
+    return cudaSuccess;
+}
+cudaError_t enqueue_mlp_forward(const float* params, const float* X, int64_t n, float* yhat, float*, float*,
+                                cudaStream_t) {
+    if (!(live(params, 4 * kMlpParams, "forward: params") && live(X, 4 * kMlpF * n, "forward: X") &&
+          live(yhat, 4 * n, "forward: yhat")))
+        return cudaErrorInvalidValue;
+    fill(yhat, n);
+    return cudaSuccess;
+}
+cudaError_t enqueue_mlp_grad(const float* params, const float* X, const float* y, int64_t n, float, float* grads,
+                             float* loss, cudaStream_t, int) {
+    if (!(live(params, 4 * kMlpParams, "grad: params") && live(X, 4 * kMlpF * n, "grad: X") && live(y, 4 * n, "grad: y") &&
+          live(grads, 4 * kMlpParams, "grad: grads") && live(loss, 4, "grad: loss")))
+        return cudaErrorInvalidValue;
+    *loss += 7.0f;
+    return cudaSuccess;
+}
+cudaError_t enqueue_adam(float* params, float* grads, float* m, float* v, float, int, cudaStream_t) {
+    const bool ok = live(params, 4 * kMlpParams, "adam: params") && live(grads, 4 * kMlpParams, "adam: grads") &&
+                    live(m, 4 * kMlpParams, "adam: m") && live(v, 4 * kMlpParams, "adam: v");
+    return ok ? cudaSuccess : cudaErrorInvalidValue;
+}
+}  // namespace shapex
+
+// ---- scenarios ---------------------------------------------------------------
+// A call of size s (0 small, 1 middle, 2 large) on the context: its status, or
+// -1 when it succeeded with outputs missing.
+using Call = std::function<int(se_ctx*, int)>;
+
+template <typename T>
+static int written(int status, const std::vector<T>& out) {
+    if (status != SE_OK) return status;
+    for (const T& v : out)
+        if (v != T(7)) return -1;
+    return SE_OK;
+}
+
+static int train(se_ctx* c, int s) {
+    const int steps = s == 0 ? 3 : (s == 1 ? 5 : 9);
+    std::vector<float> X(kMlpF * 64), y(64), losses(steps);
+    if (int rc = se_mlp_init(c, 1)) return rc;
+    return written(se_mlp_train(c, X.data(), y.data(), 64, steps, 16, 1e-3f, losses.data(), SE_MEM_HOST), losses);
+}
+
+static int check(const char* name, const se_options& opt, const Call& call) {
+    fake::where = name;
+    se_ctx* c = nullptr;
+    se_create(&c, &opt);
+    if (call(c, 0) != SE_OK) complain("the small call failed");
+    const int before = fake::allocs;
+    if (call(c, 2) != SE_OK) complain("the large call failed");
+    const int allocs = fake::allocs - before;
+    se_destroy(c);
+    for (int i = 1; i <= allocs; ++i) {
+        fake::where = std::string(name) + ", allocation " + std::to_string(i) + " of " + std::to_string(allocs);
+        se_create(&c, &opt);
+        call(c, 0);
+        fake::fail_at = fake::allocs + i;
+        const int rc = call(c, 2);
+        fake::fail_at = 0;
+        if (rc != SE_ERR_OOM) complain("its failure is not reported");
+        if (call(c, 0) != SE_OK) complain("the small call after it failed or left outputs out");
+        if (call(c, 1) != SE_OK) complain("the middle call after it failed or left outputs out");
+        if (call(c, 2) != SE_OK) complain("the large call after it failed or left outputs out");
+        se_destroy(c);
+    }
+    if (fake::blocks() > 0) complain("memory left after se_destroy");
+    std::printf("%s: %d allocations\n", name, allocs);
+    return allocs;
+}
+
+int main(int argc, char** argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    se_options opt;
+    se_options_init(&opt);
+    opt.batch_graph = 0;
+    int allocs = 0;
+    if (what == "train") allocs = check("train", opt, train);
+    if (allocs == 0) complain("no such scenario, or nothing allocated in it");
+    return fake::bad ? 1 : 0;
+}
