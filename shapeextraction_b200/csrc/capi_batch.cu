@@ -78,10 +78,10 @@ bool device_reachable(const void* p) {
 }
 
 extern "C++" {
-template <typename T>
-int grow_batch(se_ctx* c, T*& p, int64_t count, const char* what) {
-    ++c->batch_epoch;
-    SE_CUDA(c, regrow(p, count), what);
+template <typename... T>
+int grow_batch(se_ctx* c, int64_t& cap, int64_t need, const char* what, Buf<T>... bufs) {
+    if (need > cap) ++c->batch_epoch;
+    SE_CUDA(c, grow(cap, need, bufs...), what);
     return SE_OK;
 }
 }
@@ -244,19 +244,14 @@ int se_normals_batch(se_ctx* c, const float* x, const float* y, const float* z, 
     plan.node_off.assign(n_clouds + 1, 0);
     for (int i = 0; i < n_clouds; ++i)
         plan.node_off[i + 1] = plan.node_off[i] + hierarchy_nodes(offsets[i + 1] - offsets[i]);
-    if (c->batch_pts_cap < total) {
-        if (int rc = grow_batch(c, c->batch_pts4, total, "alloc batch points")) return rc;
-        c->batch_pts_cap = total;
-    }
-    if (c->batch_nodes_cap < plan.node_off[n_clouds]) {
-        if (int rc = grow_batch(c, c->batch_snodes, plan.node_off[n_clouds], "alloc batch hierarchy")) return rc;
-        c->batch_nodes_cap = plan.node_off[n_clouds];
-    }
-    if (host && total > 0 && c->batch_cap < total) {
-        if (int rc = grow_batch(c, c->batch_in, 3 * total, "alloc batch staging")) return rc;
-        if (int rc = grow_batch(c, c->batch_out, 3 * total, "alloc batch staging")) return rc;
-        c->batch_cap = total;
-    }
+    if (int rc = grow_batch(c, c->batch_pts_cap, total, "alloc batch points", Buf{c->batch_pts4, total})) return rc;
+    const int64_t nodes = plan.node_off[n_clouds];
+    if (int rc = grow_batch(c, c->batch_nodes_cap, nodes, "alloc batch hierarchy", Buf{c->batch_snodes, nodes}))
+        return rc;
+    if (host)
+        if (int rc = grow_batch(c, c->batch_cap, total, "alloc batch staging", Buf{c->batch_in, 3 * total},
+                                Buf{c->batch_out, 3 * total}))
+            return rc;
 
     // ---- plan ----
     // Clouds of at least kLaneQueryMin points are queried on their lane right

@@ -161,6 +161,22 @@ static int train(se_ctx* c, int s) {
     return written(se_mlp_train(c, X.data(), y.data(), 64, steps, 16, 1e-3f, losses.data(), SE_MEM_HOST), losses);
 }
 
+// Host arrays; `points` scales the clouds, the larger calls have more of them.
+static int batch(se_ctx* c, int s, int points) {
+    std::vector<int64_t> off{0}, u;
+    std::vector<int32_t> ks;
+    for (int i = 0; i < 2 + s; ++i) {
+        off.push_back(off.back() + points * (2 * s + 1) - 7 * i);
+        ks.push_back(i % 2 ? 8 : 16);
+    }
+    u.resize(ks.size());
+    const int64_t n = off.back();
+    std::vector<float> x(n), out(3 * n);
+    return written(se_normals_batch(c, x.data(), x.data(), x.data(), off.data(), (int)ks.size(), ks.data(), out.data(),
+                                    u.data(), SE_MEM_HOST),
+                   out);
+}
+
 static int check(const char* name, const se_options& opt, const Call& call) {
     fake::where = name;
     se_ctx* c = nullptr;
@@ -195,6 +211,10 @@ int main(int argc, char** argv) {
     opt.batch_graph = 0;
     int allocs = 0;
     if (what == "train") allocs = check("train", opt, train);
+    if (what == "batch slices") {
+        opt.batch_lanes = 1;  // one lane, never regrown: it holds 1024 points at least
+        allocs = check("batch slices", opt, [](se_ctx* c, int s) { return batch(c, s, 50); });
+    }
     if (allocs == 0) complain("no such scenario, or nothing allocated in it");
     return fake::bad ? 1 : 0;
 }
