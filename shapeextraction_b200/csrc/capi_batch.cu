@@ -36,18 +36,15 @@ int lane_capacity(se_ctx* c, BatchLane& l, int64_t n) {
         SE_CUDA(c, cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming), "lane event");
         SE_CUDA(c, cudaMalloc(&l.b.st, sizeof(DevState)), "lane state");
     }
-    if (n <= l.cap && l.b.keys0) return SE_OK;
+    const int64_t cap = n < 1024 ? 1024 : n;
+    if (cap <= l.cap) return SE_OK;
     ++c->batch_epoch;
     BuildBufs& b = l.b;
-    const int64_t cap = n < 1024 ? 1024 : n;
-    SE_CUDA(c, regrow(b.keys0, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.keys1, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.scratch, ScratchLayout(cap).words(kCodePasses)), "alloc lane");
-    SE_CUDA(c, regrow(b.codes, cap), "alloc lane");
-    SE_CUDA(c, regrow(b.pts3, 3 * cap), "alloc lane");
-    SE_CUDA(c, regrow(b.leaf_start, cap), "alloc lane");
+    SE_CUDA(c,
+            grow(l.cap, cap, Buf{b.keys0, cap}, Buf{b.keys1, cap}, Buf{b.scratch, ScratchLayout(cap).words(kCodePasses)},
+                 Buf{b.codes, cap}, Buf{b.pts3, 3 * cap}, Buf{b.leaf_start, cap}),
+            "alloc lane");
     b.cap = cap;
-    l.cap = cap;
     return SE_OK;
 }
 

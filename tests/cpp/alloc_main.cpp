@@ -215,6 +215,7 @@ int main(int argc, char** argv) {
         opt.batch_lanes = 1;  // one lane, never regrown: it holds 1024 points at least
         allocs = check("batch slices", opt, [](se_ctx* c, int s) { return batch(c, s, 50); });
     }
+    if (what == "batch lanes") allocs = check("batch lanes", opt, [](se_ctx* c, int s) { return batch(c, s, 2000); });
     if (allocs == 0) complain("no such scenario, or nothing allocated in it");
     return fake::bad ? 1 : 0;
 }
