@@ -18,7 +18,7 @@ extern "C" {
 namespace {
 
 int mlp_alloc(se_ctx* c) {
-    if (c->mlp) return SE_OK;
+    if (c->mlp_loss) return SE_OK;  // the last: all of them are there
     SE_CUDA(c, regrow(c->mlp, kMlpParams), "alloc mlp");
     SE_CUDA(c, regrow(c->mlp_m, kMlpParams), "alloc mlp");
     SE_CUDA(c, regrow(c->mlp_v, kMlpParams), "alloc mlp");

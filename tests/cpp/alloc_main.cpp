@@ -6,8 +6,9 @@
 // allocation of a call on request.
 //
 // A scenario is a small, a middle and a large call on one context. For every
-// allocation of the large call after the small one: that allocation fails, the
-// call says so, and the three calls then work.
+// allocation of the small call on a new context, and of the large call after
+// the small one: that allocation fails, the call says so, and the three calls
+// then work.
 #include <cstdio>
 #include <functional>
 #include <string>
@@ -177,27 +178,63 @@ static int batch(se_ctx* c, int s, int points) {
                    out);
 }
 
+static int build(se_ctx* c, int n) {
+    std::vector<float> x(n);
+    return se_build(c, x.data(), x.data(), x.data(), n, SE_MEM_HOST);
+}
+
+// Host arrays: foreign queries, lists, normals (with a learned radius when the
+// context has one).
+static int queries(se_ctx* c, int s) {
+    const int n = 700 * (s + 1), k = 5;
+    if (int rc = se_mlp_init(c, 1)) return rc;
+    if (int rc = build(c, n)) return rc;
+    std::vector<float> q(3 * n), d2(k * n), normals(3 * n);
+    std::vector<int32_t> idx(k * n), mine(k * n);
+    if (int rc = written(se_knn(c, k, q.data(), n, idx.data(), nullptr, SE_MEM_HOST), idx)) return rc;
+    if (int rc = written(se_knn_self(c, k, 0, n, mine.data(), d2.data(), SE_MEM_HOST), mine)) return rc;
+    if (int rc = written(SE_OK, d2)) return rc;
+    return written(se_normals(c, k, 0, n, normals.data(), SE_MEM_HOST), normals);
+}
+
+// The radius model's entry points on host arrays.
+static int model(se_ctx* c, int s) {
+    const int n = 40 * (s + 1);
+    if (int rc = se_mlp_init(c, 1)) return rc;
+    if (int rc = build(c, n)) return rc;
+    std::vector<float> X(kMlpF * n), y(n), r2(n), out(n), grads(kMlpParams);
+    float loss = 0.0f;
+    if (int rc = written(se_mlp_predict(c, 0, n, y.data(), r2.data(), SE_MEM_HOST), y)) return rc;
+    if (int rc = written(SE_OK, r2)) return rc;
+    if (int rc = written(se_mlp_forward(c, X.data(), n, out.data(), SE_MEM_HOST), out)) return rc;
+    if (int rc = se_mlp_grad(c, X.data(), y.data(), n, grads.data(), &loss, SE_MEM_HOST)) return rc;
+    if (loss != 7.0f) return -1;
+    return written(se_features(c, 0, n, X.data(), SE_MEM_HOST), X);
+}
+
 static int check(const char* name, const se_options& opt, const Call& call) {
-    fake::where = name;
-    se_ctx* c = nullptr;
-    se_create(&c, &opt);
-    if (call(c, 0) != SE_OK) complain("the small call failed");
-    const int before = fake::allocs;
-    if (call(c, 2) != SE_OK) complain("the large call failed");
-    const int allocs = fake::allocs - before;
-    se_destroy(c);
-    for (int i = 1; i <= allocs; ++i) {
-        fake::where = std::string(name) + ", allocation " + std::to_string(i) + " of " + std::to_string(allocs);
-        se_create(&c, &opt);
-        call(c, 0);
-        fake::fail_at = fake::allocs + i;
-        const int rc = call(c, 2);
-        fake::fail_at = 0;
-        if (rc != SE_ERR_OOM) complain("its failure is not reported");
-        if (call(c, 0) != SE_OK) complain("the small call after it failed or left outputs out");
-        if (call(c, 1) != SE_OK) complain("the middle call after it failed or left outputs out");
-        if (call(c, 2) != SE_OK) complain("the large call after it failed or left outputs out");
-        se_destroy(c);
+    int allocs = 0;
+    for (const bool fresh : {true, false}) {  // the first call's allocations, those of a larger call
+        const std::string title = std::string(name) + (fresh ? ", first call" : ", larger call");
+        const int size = fresh ? 0 : 2;
+        int n = 1;
+        for (int i = 0; i <= n; ++i) {  // i = 0: none fails, which counts them
+            fake::where = title + ", allocation " + std::to_string(i) + " of " + std::to_string(n);
+            se_ctx* c = nullptr;
+            se_create(&c, &opt);
+            if (!fresh && call(c, 0) != SE_OK) complain("the small call failed");
+            const int before = fake::allocs;
+            if (i > 0) fake::fail_at = before + i;
+            const int rc = call(c, size);
+            fake::fail_at = 0;
+            if (i == 0) n = fake::allocs - before;
+            if (rc != (i == 0 ? SE_OK : SE_ERR_OOM)) complain("its failure is not reported");
+            if (call(c, 0) != SE_OK) complain("the small call after it failed or left outputs out");
+            if (call(c, 1) != SE_OK) complain("the middle call after it failed or left outputs out");
+            if (call(c, 2) != SE_OK) complain("the large call after it failed or left outputs out");
+            se_destroy(c);
+        }
+        allocs += n;
     }
     if (fake::blocks() > 0) complain("memory left after se_destroy");
     std::printf("%s: %d allocations\n", name, allocs);
@@ -215,6 +252,12 @@ int main(int argc, char** argv) {
         opt.batch_lanes = 1;  // one lane, never regrown: it holds 1024 points at least
         allocs = check("batch slices", opt, [](se_ctx* c, int s) { return batch(c, s, 50); });
     }
+    if (what == "queries") allocs = check("queries", opt, queries);
+    if (what == "learned") {
+        opt.learned = opt.learned_skip_seed = opt.learned_cell_scan = 1;
+        allocs = check("learned", opt, queries);
+    }
+    if (what == "model") allocs = check("model", opt, model);
     if (what == "batch lanes") allocs = check("batch lanes", opt, [](se_ctx* c, int s) { return batch(c, s, 2000); });
     if (allocs == 0) complain("no such scenario, or nothing allocated in it");
     return fake::bad ? 1 : 0;
