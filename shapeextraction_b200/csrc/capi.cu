@@ -168,10 +168,7 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
     if (q.compat && q.n_octree < 1)
         return fail(c, SE_ERR_UNSUPPORTED, "the reference-compatible search needs the octree (build_octree = 1, u >= 2)");
     const bool use_learned = c->opt.learned && !ext && c->mlp_ready && !q.compat;
-    if (use_learned && c->r2_cap < count) {
-        SE_CUDA(c, regrow(c->r2_buf, count), "alloc learned bounds");
-        c->r2_cap = count;
-    }
+    if (use_learned) SE_CUDA(c, grow(c->r2_cap, count, Buf{c->r2_buf, count}), "alloc learned bounds");
     q.learned_r2 = use_learned ? c->r2_buf : nullptr;
     q.learned_skip_seed = c->opt.learned_skip_seed;
     // with learned_cell_scan the learned attempt scans Morton cells directly
@@ -184,10 +181,7 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
         int level = 1;
         while (level < bpa && level < 7 && ((int64_t)8 << (3 * level)) * 2 <= u) ++level;
         const int64_t n_ent = ((int64_t)1 << (3 * level)) + 1;
-        if (c->lut_cap < n_ent) {
-            SE_CUDA(c, regrow(c->lut_buf, n_ent), "alloc cell table");
-            c->lut_cap = n_ent;
-        }
+        SE_CUDA(c, grow(c->lut_cap, n_ent, Buf{c->lut_buf, n_ent}), "alloc cell table");
         SE_CUDA(c, enqueue_cell_lut(c->b, c->opt.code_bits, level, c->lut_buf, c->stream, c->num_sms),
                 "launch cell table");
         c->lut_level = level;
@@ -202,10 +196,7 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
     const bool host = mem == SE_MEM_HOST;
     if (ext) {
         if (host) {
-            if (c->q_cap < 3 * count) {
-                SE_CUDA(c, regrow(c->q_buf, 3 * count), "alloc queries");
-                c->q_cap = 3 * count;
-            }
+            SE_CUDA(c, grow(c->q_cap, 3 * count, Buf{c->q_buf, 3 * count}), "alloc queries");
             SE_CUDA(c, cudaMemcpyAsync(c->q_buf, ext, sizeof(float) * 3 * count, cudaMemcpyHostToDevice, c->stream),
                     "copy queries");
             q.ext_queries = c->q_buf;
@@ -219,14 +210,13 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
     // near a 2M-point scene, k = 8, in random order: 21.0 ms as given, 0.93 ms
     // with the sort, which takes about 70 us of it.)
     const bool sorted = ext && !q.compat && queries_per_warp(count, c->num_sms, true) > 1;
-    if (sorted && c->q_order_cap < count) {
+    if (sorted) {
         QueryOrder& o = c->q_order;
-        c->q_order_cap = 0;
-        if (!o.st) SE_CUDA(c, cudaMalloc(&o.st, sizeof(DevState)), "alloc query order");
-        SE_CUDA(c, regrow(o.keys0, count), "alloc query order");
-        SE_CUDA(c, regrow(o.keys1, count), "alloc query order");
-        SE_CUDA(c, regrow(o.lookback, 3 * ((count + kSortTile - 1) / kSortTile) * kSortBins), "alloc query order");
-        c->q_order_cap = count;
+        const int64_t lookback = 3 * ((count + kSortTile - 1) / kSortTile) * kSortBins;
+        SE_CUDA(c,
+                grow(c->q_order_cap, count, Buf{o.st, 1}, Buf{o.keys0, count}, Buf{o.keys1, count},
+                     Buf{o.lookback, lookback}),
+                "alloc query order");
     }
     // Pinned host outputs are written by the kernel itself (mapped host
     // memory), so the results cross PCIe while the kernel runs instead of in
@@ -245,11 +235,8 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
     void* m_nrm = mapped(out_normals);
     if (out_idx) {
         if (host) {
-            if (c->idx_cap < (int64_t)k * count) {
-                SE_CUDA(c, regrow(c->idx_buf, (int64_t)k * count), "alloc knn staging");
-                SE_CUDA(c, regrow(c->d2_buf, (int64_t)k * count), "alloc knn staging");
-                c->idx_cap = (int64_t)k * count;
-            }
+            SE_CUDA(c, grow(c->idx_cap, k * count, Buf{c->idx_buf, k * count}, Buf{c->d2_buf, k * count}),
+                    "alloc knn staging");
             q.out_idx = m_idx ? static_cast<int32_t*>(m_idx) : c->idx_buf;
             q.out_d2 = out_d2 ? (m_d2 ? static_cast<float*>(m_d2) : c->d2_buf) : nullptr;
         } else {
@@ -259,10 +246,7 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
     }
     if (out_normals) {
         if (host) {
-            if (c->out_cap < 3 * count) {
-                SE_CUDA(c, regrow(c->out_buf, 3 * count), "alloc normals staging");
-                c->out_cap = 3 * count;
-            }
+            SE_CUDA(c, grow(c->out_cap, 3 * count, Buf{c->out_buf, 3 * count}), "alloc normals staging");
             q.out_normals = m_nrm ? static_cast<float*>(m_nrm) : c->out_buf;
         } else {
             q.out_normals = out_normals;

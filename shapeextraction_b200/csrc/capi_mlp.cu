@@ -38,10 +38,7 @@ int stage_in(se_ctx* c, const float* src, int64_t n, int mem, int64_t off, int64
         *out = src;
         return SE_OK;
     }
-    if (c->xs_cap < total) {
-        SE_CUDA(c, regrow(c->xs_buf, total), "alloc staging");
-        c->xs_cap = total;
-    }
+    SE_CUDA(c, grow(c->xs_cap, total, Buf{c->xs_buf, total}), "alloc staging");
     SE_CUDA(c, cudaMemcpyAsync(c->xs_buf + off, src, sizeof(float) * n, cudaMemcpyHostToDevice, c->stream), "copy in");
     *out = c->xs_buf + off;
     return SE_OK;
@@ -66,10 +63,7 @@ int se_features(se_ctx* c, int64_t start, int64_t count, float* out, int mem) {
     if (!out) return fail(c, SE_ERR_INVALID_ARG, "null output");
     float* dst = out;
     if (mem == SE_MEM_HOST) {
-        if (c->xs_cap < count * kMlpF) {
-            SE_CUDA(c, regrow(c->xs_buf, count * kMlpF), "alloc staging");
-            c->xs_cap = count * kMlpF;
-        }
+        SE_CUDA(c, grow(c->xs_cap, count * kMlpF, Buf{c->xs_buf, count * kMlpF}), "alloc staging");
         dst = c->xs_buf;
     }
     SE_CUDA(c, enqueue_features(c->b, u, c->opt.code_bits, start, count, dst, c->stream), "launch features");
@@ -170,10 +164,7 @@ int se_mlp_predict(se_ctx* c, int64_t start, int64_t count, float* yhat, float* 
     if (count == 0) return SE_OK;
     float *dy = yhat, *dr = r2;
     if (mem == SE_MEM_HOST) {
-        if (c->xs_cap < 2 * count) {
-            SE_CUDA(c, regrow(c->xs_buf, 2 * count), "alloc staging");
-            c->xs_cap = 2 * count;
-        }
+        SE_CUDA(c, grow(c->xs_cap, 2 * count, Buf{c->xs_buf, 2 * count}), "alloc staging");
         dy = yhat ? c->xs_buf : nullptr;
         dr = r2 ? c->xs_buf + count : nullptr;
     }
