@@ -208,15 +208,20 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
     // lie close together, so they are taken in the order of their places in the
     // tree. With one query per warp there is nothing to share. (250k queries
     // near a 2M-point scene, k = 8, in random order: 21.0 ms as given, 0.93 ms
-    // with the sort, which takes about 70 us of it.)
-    const bool sorted = ext && !q.compat && queries_per_warp(count, c->num_sms, true) > 1;
+    // with the sort, which takes about 70 us of it.) Where the sort's 24 bytes
+    // per query cannot be had they are taken as given, one to a warp.
+    bool sorted = ext && !q.compat && queries_per_warp(count, c->num_sms, true) > 1;
     if (sorted) {
         QueryOrder& o = c->q_order;
         const int64_t lookback = 3 * ((count + kSortTile - 1) / kSortTile) * kSortBins;
-        SE_CUDA(c,
-                grow(c->q_order_cap, count, Buf{o.st, 1}, Buf{o.keys0, count}, Buf{o.keys1, count},
-                     Buf{o.lookback, lookback}),
-                "alloc query order");
+        const cudaError_t e = grow(c->q_order_cap, count, Buf{o.st, 1}, Buf{o.keys0, count}, Buf{o.keys1, count},
+                                   Buf{o.lookback, lookback});
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            sorted = false;
+        } else {
+            SE_CUDA(c, e, "alloc query order");
+        }
     }
     // Pinned host outputs are written by the kernel itself (mapped host
     // memory), so the results cross PCIe while the kernel runs instead of in

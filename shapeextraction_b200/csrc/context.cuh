@@ -160,8 +160,8 @@ template <typename T>
 Buf(T*&, int64_t) -> Buf<T>;
 
 // Buffers of one capacity, regrown together once `need` exceeds it. While any
-// of them may be missing the capacity is 0: after a failed allocation it would
-// otherwise still vouch for a buffer that has been freed.
+// of them may be missing the capacity is 0: after a failed allocation, which
+// frees them all, it would otherwise still vouch for a buffer that is gone.
 template <typename... T>
 cudaError_t grow(int64_t& cap, int64_t need, Buf<T>... bufs) {
     if (need <= cap) return cudaSuccess;
@@ -169,6 +169,7 @@ cudaError_t grow(int64_t& cap, int64_t need, Buf<T>... bufs) {
     cudaError_t e = cudaSuccess;
     ((e = e == cudaSuccess ? regrow(bufs.p, bufs.count) : e), ...);
     if (e == cudaSuccess) cap = need;
+    else (regrow(bufs.p, 0), ...);
     return e;
 }
 

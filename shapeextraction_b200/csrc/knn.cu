@@ -1374,7 +1374,7 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     a.cell_span = q.cell_span < 2 ? 2 : (q.cell_span > 4 ? 4 : q.cell_span);
     if (a.seed_halo > kMaxHalo) a.seed_halo = kMaxHalo;
     if (a.seed_halo < 0) a.seed_halo = 0;
-    a.warp_queries = queries_per_warp(q.count, num_sms, q.ext_queries != nullptr);
+    a.warp_queries = q.ext_queries && !q.order ? 1 : queries_per_warp(q.count, num_sms, q.ext_queries != nullptr);
     const bool ext = q.ext_queries != nullptr;
     const bool nrm = q.out_normals != nullptr && !ext;
     switch (q.k) {

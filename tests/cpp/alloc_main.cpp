@@ -7,8 +7,8 @@
 //
 // A scenario is a small, a middle and a large call on one context. For every
 // allocation of the small call on a new context, and of the large call after
-// the small one: that allocation fails, the call says so, and the three calls
-// then work.
+// the small one: that allocation fails, the call says so (or, where it copes,
+// works all the same), and the three calls then work.
 #include <cstdio>
 #include <functional>
 #include <string>
@@ -53,7 +53,7 @@ cudaError_t enqueue_build(const BuildBufs& b, const BuildParams& p, cudaStream_t
     return cudaSuccess;
 }
 cudaError_t enqueue_octree(const BuildBufs&, const BuildParams&, cudaStream_t, int*) { return cudaSuccess; }
-int queries_per_warp(int64_t count, int, bool) { return count > 100 ? 32 : 1; }
+int queries_per_warp(int64_t count, int, bool) { return count > 5000 ? 32 : 1; }
 cudaError_t enqueue_query_order(const BuildBufs&, const QueryOrder& o, const float* q, int64_t n, int64_t, int,
                                 const uint64_t** order, int* shift, cudaStream_t, int, int* launches) {
     const int64_t tiles = (n + kSortTile - 1) / kSortTile;
@@ -197,6 +197,16 @@ static int queries(se_ctx* c, int s) {
     return written(se_normals(c, k, 0, n, normals.data(), SE_MEM_HOST), normals);
 }
 
+// Foreign queries on device arrays, enough of them to be ordered: the order's
+// buffers are all that the call allocates.
+static int foreign(se_ctx* c, int s) {
+    const int n = 6000 * (s + 1), k = 5;
+    std::vector<float> q(3 * n);
+    std::vector<int32_t> idx(k * n);
+    fake::Device dq(q.data(), 4 * q.size()), di(idx.data(), 4 * idx.size());
+    return written(se_knn(c, k, (float*)q.data(), n, idx.data(), nullptr, SE_MEM_DEVICE), idx);
+}
+
 // The radius model's entry points on host arrays.
 static int model(se_ctx* c, int s) {
     const int n = 40 * (s + 1);
@@ -212,7 +222,8 @@ static int model(se_ctx* c, int s) {
     return written(se_features(c, 0, n, X.data(), SE_MEM_HOST), X);
 }
 
-static int check(const char* name, const se_options& opt, const Call& call) {
+static int check(const char* name, const se_options& opt, const Call& call, bool copes = false,
+                 int (*prepare)(se_ctx*) = nullptr) {
     int allocs = 0;
     for (const bool fresh : {true, false}) {  // the first call's allocations, those of a larger call
         const std::string title = std::string(name) + (fresh ? ", first call" : ", larger call");
@@ -222,13 +233,15 @@ static int check(const char* name, const se_options& opt, const Call& call) {
             fake::where = title + ", allocation " + std::to_string(i) + " of " + std::to_string(n);
             se_ctx* c = nullptr;
             se_create(&c, &opt);
+            if (prepare) prepare(c);
             if (!fresh && call(c, 0) != SE_OK) complain("the small call failed");
             const int before = fake::allocs;
             if (i > 0) fake::fail_at = before + i;
             const int rc = call(c, size);
             fake::fail_at = 0;
             if (i == 0) n = fake::allocs - before;
-            if (rc != (i == 0 ? SE_OK : SE_ERR_OOM)) complain("its failure is not reported");
+            if (rc != (i == 0 || copes ? SE_OK : SE_ERR_OOM))
+                complain(copes ? "the call failed or left outputs out" : "its failure is not reported");
             if (call(c, 0) != SE_OK) complain("the small call after it failed or left outputs out");
             if (call(c, 1) != SE_OK) complain("the middle call after it failed or left outputs out");
             if (call(c, 2) != SE_OK) complain("the large call after it failed or left outputs out");
@@ -257,6 +270,7 @@ int main(int argc, char** argv) {
         opt.learned = opt.learned_skip_seed = opt.learned_cell_scan = 1;
         allocs = check("learned", opt, queries);
     }
+    if (what == "foreign") allocs = check("foreign", opt, foreign, true, [](se_ctx* c) { return build(c, 100); });
     if (what == "model") allocs = check("model", opt, model);
     if (what == "batch lanes") allocs = check("batch lanes", opt, [](se_ctx* c, int s) { return batch(c, s, 2000); });
     if (allocs == 0) complain("no such scenario, or nothing allocated in it");

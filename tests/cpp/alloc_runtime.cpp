@@ -23,6 +23,8 @@ bool live(const void* p, int64_t bytes, const char* what) {
     if (!ok) complain(what);
     return ok;
 }
+Device::Device(const void* q, size_t bytes) : p(q) { g_blocks[(const char*)q] = bytes; }
+Device::~Device() { g_blocks.erase((const char*)p); }
 static cudaError_t take(void** p, size_t bytes) {
     *p = nullptr;
     if (++allocs == fail_at) return cudaErrorMemoryAllocation;

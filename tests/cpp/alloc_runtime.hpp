@@ -14,4 +14,10 @@ void complain(const char* what);
 size_t blocks();  // allocations not freed
 // Whether p points to at least `bytes` of one live block; complains if not.
 bool live(const void* p, int64_t bytes, const char* what);
+// A caller's device array, live as long as this object.
+struct Device {
+    const void* p;
+    Device(const void* p, size_t bytes);
+    ~Device();
+};
 }  // namespace fake

@@ -30,7 +30,8 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["train", "batch slices", "batch lanes", "queries", "learned", "model"])
+@pytest.mark.parametrize("scenario", ["train", "batch slices", "batch lanes", "queries", "learned", "model",
+                                      "foreign"])
 def test_a_failed_allocation_leaves_the_context_usable(harness, scenario):
     r = subprocess.run([harness, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
