@@ -992,8 +992,12 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
     const bool learned = a.learned_r2 != nullptr;
     const float cap0 = (learned && active) ? __ldg(a.learned_r2 + qo) : INFINITY;
     bool act = active;
+    // Nothing is near a query with a NaN coordinate: no distance passes its
+    // bound and none tightens it, so a search would scan the whole tree for it.
+    if (EXT) act = act && qx == qx && qy == qy && qz == qz;
     nn.init();
     for (int attempt = learned ? 0 : 1; attempt < 2; ++attempt) {
+        if (EXT && !__any_sync(FULL, act)) break;
         const float cap = attempt == 0 ? cap0 : INFINITY;
         const bool seed = attempt == 1 || !a.learned_skip_seed;
         const int64_t sw0 = seed && !lone ? w0 : 0, sw1 = seed && !lone ? w1 : 0;  // points offered by the seed
@@ -1071,8 +1075,7 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
     }
     if (!active) return;
 
-    // A query with a NaN coordinate is near nothing: it gets points of its
-    // window, at distance NaN.
+    // A query with a NaN coordinate gets points of its window, at distance NaN.
     const bool lost = q.n == 0;
     if (lost)
         for (; q.n < K && w0 + q.n < w1; ++q.n) {
