@@ -994,7 +994,14 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
     bool act = active;
     // Nothing is near a query with a NaN coordinate: no distance passes its
     // bound and none tightens it, so a search would scan the whole tree for it.
-    if (EXT) act = act && qx == qx && qy == qy && qz == qz;
+    // Nor is anything nearer than the rest to one whose every squared distance
+    // overflows: the lowest indices win the tie. The decoded points lie in the
+    // cube [lo, hi]^3, whose box distance is no larger than any of theirs.
+    auto out_of_range = [&]() {
+        const float lo = st->min_coord, hi = __fmaf_rn(1.0f, st->range, lo);
+        return box_dist2(qx, qy, qz, lo, lo, lo, hi, hi, hi) == INFINITY;
+    };
+    if (EXT) act = act && qx == qx && qy == qy && qz == qz && !out_of_range();
     nn.init();
     for (int attempt = learned ? 0 : 1; attempt < 2; ++attempt) {
         if (EXT && !__any_sync(FULL, act)) break;
@@ -1075,12 +1082,13 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
     }
     if (!active) return;
 
-    // A query with a NaN coordinate gets points of its window, at distance NaN.
-    const bool lost = q.n == 0;
-    if (lost)
-        for (; q.n < K && w0 + q.n < w1; ++q.n) {
+    // A query with a NaN coordinate gets points of its window, at distance NaN;
+    // one out of range the first points of the tree.
+    const bool lost = q.n == 0 && !(EXT && qx == qx && qy == qy && qz == qz);
+    if (q.n == 0)
+        for (const int64_t first = lost ? w0 : 0, end = lost ? w1 : u; q.n < K && first + q.n < end; ++q.n) {
             W.d[q.n][lane] = INFINITY;
-            W.idx[q.n][lane] = (int32_t)(w0 + q.n);
+            W.idx[q.n][lane] = (int32_t)(first + q.n);
         }
     // the k nearest in the lists' order: by distance, then by index
     unsigned long long key[K];
