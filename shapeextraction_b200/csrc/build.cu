@@ -120,14 +120,15 @@ __device__ __forceinline__ void load_bbox(const DevState* st, float& mn, float& 
 
 // Digit offsets, trivial-pass detection and ping-pong parity, by one block of
 // NT threads (kSortBins / NT adjacent digits each). With first < last only
-// passes [first, last) run, all of them; otherwise those of the first `passes`
-// whose digits are not all equal.
+// passes [first, last) run, all of them, or none where the keys are in order
+// and `last` - `first` is even (the result is in the same buffer then);
+// otherwise those of the first `passes` whose digits are not all equal.
 template <int NT>
 __device__ __forceinline__ void sort_prep(int64_t n, int passes, DevState* st, int first, int last) {
     constexpr int kPer = kSortBins / NT;
     __shared__ uint32_t s_w[NT / 32 + 1];
     __shared__ int s_triv[kSortPasses];
-    for (int p = 0; p < passes; ++p) {
+    for (int p = first; p < (first < last ? last : passes); ++p) {
         uint32_t h[kPer], sum = 0, tot;
 #pragma unroll
         for (int i = 0; i < kPer; ++i) {
@@ -147,8 +148,9 @@ __device__ __forceinline__ void sort_prep(int64_t n, int passes, DevState* st, i
     }
     if (threadIdx.x == 0) {
         int act = 0;
+        const bool sorted = !st->disorder && (last - first) % 2 == 0;
         for (int p = 0; p < kSortPasses; ++p) {
-            const bool run = first < last ? p >= first && p < last : p < passes && !s_triv[p];
+            const bool run = first < last ? p >= first && p < last && !sorted : p < passes && !s_triv[p];
             st->pass_active[p] = run;
             st->pass_parity[p] = act & 1;
             act += run;
@@ -1254,7 +1256,8 @@ __global__ void __launch_bounds__(256) k_copy_if_odd(const uint64_t* __restrict_
 }
 
 // Order keys of foreign queries (their places by binary search over the
-// tree's codes) and the digit histograms of the passes that sort them.
+// tree's codes), the digit histograms of the passes that sort them, and whether
+// they come out of order at all.
 __global__ void __launch_bounds__(256) k_query_keys(const float* __restrict__ q, int64_t n,
                                                     const uint64_t* __restrict__ codes, int64_t u, int code_bits,
                                                     int shift, int first, uint64_t* __restrict__ keys,
@@ -1264,17 +1267,72 @@ __global__ void __launch_bounds__(256) k_query_keys(const float* __restrict__ q,
     __syncthreads();
     const float mn = tree->min_coord, range = tree->range;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
+    auto place = [&](int64_t i) {
         const uint64_t code = query_to_code(q[3 * i], q[3 * i + 1], q[3 * i + 2], mn, range, code_bits);
-        const uint64_t k = ((uint64_t)code_position(codes, u, code) << (shift + kOrderShift)) | (uint64_t)i;
-        keys[i] = k;
-        for (int p = first; p < kSortPasses - 1; ++p) atomicAdd(&s_h[p][(k >> (kSortBits * p)) & (kSortBins - 1)], 1u);
+        return (uint64_t)code_position(codes, u, code) << (shift + kOrderShift);
+    };
+    for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += stride) {
+        const int lane = threadIdx.x & 31;
+        const int64_t i = i0 + lane;
+        const uint64_t at = i < n ? place(i) : ~0ull;
+        if (i < n) {
+            const uint64_t k = at | (uint64_t)i;
+            keys[i] = k;
+            for (int p = first; p < kSortPasses - 1; ++p)
+                atomicAdd(&s_h[p][(k >> (kSortBits * p)) & (kSortBins - 1)], 1u);
+        }
+        // in order by the digits that are sorted; the step from the query before
+        // the warp's first costs another search, made where all others are up
+        uint64_t before = __shfl_up_sync(0xffffffffu, at, 1);
+        if (lane == 0) before = 0;
+        bool down = before >> (kSortBits * first) > at >> (kSortBits * first);
+        if (!__any_sync(0xffffffffu, down) && lane == 0 && i0 > 0)
+            down = place(i0 - 1) >> (kSortBits * first) > at >> (kSortBits * first);
+        if (down) st->disorder = 1;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kSortPasses * kSortBins; i += blockDim.x) {
         const uint32_t v = (&s_h[0][0])[i];
         if (v) atomicAdd(&(&st->hist[0][0])[i], v);
     }
+}
+
+// Work items of sorted foreign queries, one thread per query: an aligned group
+// of `group` queries that spans kTogetherSpan places, else its aligned parts of
+// `per` queries that span kWindowSpan, else single ones. Queries far apart share
+// nothing, and one warp that took several of them ended last: 250k queries that
+// are tree points moved by 1e-5, a few of them far from the rest in the tree's
+// order, took 736 us in parts of 16, without the few 312 us.
+__global__ void __launch_bounds__(256) k_query_items(const uint64_t* __restrict__ keys, int64_t n, int shift, int per,
+                                                     int group, uint64_t* __restrict__ items, DevState* tree) {
+    constexpr unsigned kFull = 0xffffffffu;
+    __shared__ uint32_t s_at[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int lo = (int)(keys[min64(i, n - 1)] >> shift), hi = lo, size = 1;
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+        lo = min(lo, __shfl_xor_sync(kFull, lo, o));
+        hi = max(hi, __shfl_xor_sync(kFull, hi, o));
+        if (2 * o == per && hi - lo <= kWindowSpan) size = per;
+        if (2 * o == group && hi - lo <= kTogetherSpan) size = group;
+    }
+    const uint32_t firsts = __ballot_sync(kFull, i < n && (lane & (size - 1)) == 0);
+    if (lane == 0) s_at[warp] = __popc(firsts);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t total = 0;
+        for (int w = 0; w < 8; ++w) {
+            const uint32_t c = s_at[w];
+            s_at[w] = total;
+            total += c;
+        }
+        const uint32_t base = atomicAdd(&tree->items, total);
+        for (int w = 0; w < 8; ++w) s_at[w] += base;
+    }
+    __syncthreads();
+    if ((firsts >> lane) & 1u)
+        items[s_at[warp] + __popc(firsts & lanemask_lt())] = ((uint64_t)min64(size, n - i) << 32) | (uint64_t)i;
 }
 
 inline unsigned grid_for(int64_t work, int threads, int64_t cap_blocks) {
@@ -1316,8 +1374,8 @@ cudaError_t enqueue_sort_keys(uint64_t* keys, uint64_t* tmp, int64_t n, uint32_t
 }
 
 cudaError_t enqueue_query_order(const BuildBufs& b, const QueryOrder& o, const float* queries, int64_t n, int64_t u,
-                                int code_bits, const uint64_t** order, int* shift, cudaStream_t s, int num_sms,
-                                int* launches) {
+                                int code_bits, const uint64_t** order, const uint64_t** items, int* shift,
+                                cudaStream_t s, int num_sms, int* launches) {
     cudaError_t e = set_onesweep_attributes();
     if (e != cudaSuccess) return e;
     int bits = 1;  // places are in [0, u]
@@ -1337,7 +1395,11 @@ cudaError_t enqueue_query_order(const BuildBufs& b, const QueryOrder& o, const f
         k_onesweep<<<(unsigned)tiles, kSortThreads, sizeof(SortSmem), s>>>(
             o.keys0, o.keys1, n, pass, o.lookback + kSortBins * tiles * (pass - first), o.st, kSpinLimit, 0);
     *order = passes & 1 ? o.keys1 : o.keys0;
-    *launches += 2 + passes;
+    uint64_t* list = passes & 1 ? o.keys0 : o.keys1;
+    k_query_items<<<grid_for(n, 256, 0), 256, 0, s>>>(*order, n, *shift + kOrderShift, queries_per_warp(n, num_sms, true),
+                                                      queries_per_warp(n, num_sms, false), list, b.st);
+    *items = list;
+    *launches += 3 + passes;
     return cudaGetLastError();
 }
 

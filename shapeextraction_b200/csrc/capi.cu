@@ -204,13 +204,12 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
             q.ext_queries = ext;
         }
     }
-    // Foreign queries come in any order; a warp's 32 share a walk only if they
-    // lie close together, so they are taken in the order of their places in the
-    // tree. With one query per warp there is nothing to share. (250k queries
-    // near a 2M-point scene, k = 8, in random order: 21.0 ms as given, 0.93 ms
-    // with the sort, which takes about 70 us of it.) Where the sort's 24 bytes
-    // per query cannot be had they are taken as given, one to a warp.
-    bool sorted = ext && !q.compat && queries_per_warp(count, c->num_sms, true) > 1;
+    // Foreign queries come in any order; a warp's share a walk only if they lie
+    // close together, so many of them are taken in the order of their places in
+    // the tree. (250k queries near a 2M-point scene, k = 8, in random order: 21.0
+    // ms as given, 0.66 ms in order.) Where the order's 24 bytes per query cannot
+    // be had they are taken as given, one to a warp.
+    bool sorted = ext && !q.compat && order_foreign(count, k, c->num_sms);
     if (sorted) {
         QueryOrder& o = c->q_order;
         const int64_t lookback = 3 * ((count + kSortTile - 1) / kSortTile) * kSortBins;
@@ -267,7 +266,7 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
                 "launch radius prediction");
     int order_launches = 0;
     if (sorted)
-        SE_CUDA(c, enqueue_query_order(c->b, c->q_order, q.ext_queries, count, u, c->opt.code_bits, &q.order,
+        SE_CUDA(c, enqueue_query_order(c->b, c->q_order, q.ext_queries, count, u, c->opt.code_bits, &q.order, &q.items,
                                        &q.order_shift, c->stream, c->num_sms, &order_launches),
                 "order queries");
     SE_CUDA(c, enqueue_query(c->b, q, c->stream, c->num_sms), "launch query");

@@ -205,7 +205,10 @@ struct QArgs {
     int32_t* out_idx;
     float* out_d2;
     float* out_normals;
-    const float* learned_r2;
+    union {
+        const float* learned_r2;
+        const uint64_t* items;  // foreign queries with an order: the work items
+    };
     union {
         const uint32_t* cell_lut;  // learned cell scan: code-range table (null: tree walk with the cap)
         const uint64_t* order;     // foreign queries: their order (null: as given)
@@ -222,7 +225,10 @@ struct QArgs {
         int lut_shift;    // per-axis shift of the table's level (bits per axis - level)
         int order_shift;  // scale of the places in `order`
     };
-    int cell_pmax;     // cell scan: most points per warp before it falls back to the walk
+    union {
+        int cell_pmax;  // cell scan: most points per warp before it falls back to the walk
+        float close;    // foreign queries as given: extent, in ranges of the tree, of a group taken together (0: none)
+    };
     int cell_span;     // cell scan: most cells per axis covering one lane's ball (2..4)
     int warp_queries;  // queries per warp, 1..32
 };
@@ -930,21 +936,21 @@ __device__ __forceinline__ void search(Nearest<K, EXACT>& nn, Query& q, WS& W, i
     }
 }
 
-// The queries [q0, q0 + warp_queries) of one warp: search, then the outputs.
+// The queries [q0, q0 + nq) of one warp: search, then the outputs.
 // CELLS: the learned attempt may run the cell scan (a separate instantiation,
 // launched only when the caller turned the cell scan on: compiled into the
 // default kernels, its code alone slowed them by about 8%).
 template <int K, bool EXACT, bool EXT, bool NORMALS, bool CELLS>
 __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const SNode* __restrict__ snodes,
                                          const uint64_t* __restrict__ codes, const QArgs& a, DevState* st,
-                                         int64_t q0, WarpSmem<KnnCfg<K>::buf, CELLS>& W, int lane) {
+                                         int64_t q0, int nq, WarpSmem<KnnCfg<K>::buf, CELLS>& W, int lane) {
     constexpr int kBuf = KnnCfg<K>::buf;
     static_assert(K + 8 <= kBuf, "k candidates and room for hits");
     const int64_t u = a.device_count ? (int64_t)st->u : a.u;
     const int64_t count = a.device_count ? u : a.count;
     if (q0 >= count) return;  // whole warp
     const int64_t qo = q0 + lane;
-    const bool active = lane < a.warp_queries && qo < count;
+    const bool active = lane < nq && qo < count;
     float qx, qy, qz;
     int64_t center;   // tree index of the warp's first query; foreign queries: the lane's place among the codes
     int64_t row = qo;  // of the outputs
@@ -971,16 +977,18 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
         qz = p.z;
         center = a.start + q0;
     }
-    // the seed window: the warp's. Sorted foreign queries can lie far apart, so
-    // there each lane only fills its list around its own place; unsorted ones
-    // come one to a warp, with a window around that.
-    const bool lone = EXT && a.order != nullptr;
-    int64_t w0 = 0, w1 = u;
-    if (!lone) {
-        const int64_t from = EXT ? __shfl_sync(FULL, center, 0) - 16 : center;
-        w0 = max64(0, from - a.seed_halo);
-        w1 = min64(u, from + (EXT ? 32 : a.warp_queries) + a.seed_halo);
+    // the seed window: the warp's, around its queries' places. Foreign queries
+    // can lie far apart: each lane then only fills its list around its own place.
+    int64_t from = center, to = center + nq;
+    bool lone = false;
+    if (EXT) {
+        const int first = (int)__reduce_min_sync(FULL, active ? (unsigned)center : UINT_MAX);
+        const int last = (int)__reduce_max_sync(FULL, active ? (unsigned)center : 0u);
+        lone = last - first > kWindowSpan;
+        from = first - 16;
+        to = last + 16;
     }
+    const int64_t w0 = lone ? 0 : max64(0, from - a.seed_halo), w1 = lone ? u : min64(u, to + a.seed_halo);
 
     Nearest<K, EXACT> nn;
     Query q{qx, qy, qz, a.k, 0, 0};
@@ -989,7 +997,7 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
     // With a learned radius, attempt 0 searches with the predicted bound as a
     // cap; a lane whose k-th neighbour lies beyond its cap (the cap pruned
     // points that could belong to its k best) is searched again without it.
-    const bool learned = a.learned_r2 != nullptr;
+    const bool learned = !EXT && a.learned_r2 != nullptr;
     const float cap0 = (learned && active) ? __ldg(a.learned_r2 + qo) : INFINITY;
     bool act = active;
     // Nothing is near a query with a NaN coordinate: no distance passes its
@@ -1123,6 +1131,22 @@ __device__ __forceinline__ void knn_warp(const float4* __restrict__ pts, const S
     }
 }
 
+// How many of the foreign queries from q0 on, one to a warp as given, the warp
+// takes: its one, or, as the first of an aligned group of 32 within a box of
+// `close` tree ranges, all of the group (the others then take none), since
+// such share nodes, leaves and most candidates. 17,000 queries within a point
+// spacing of each other in a 2M-point scene took 138 us (k = 8) and 449 us
+// (k = 32) one to a warp, now 50 and 81 us.
+__device__ __forceinline__ int foreign_share(const QArgs& a, const DevState* st, int64_t q0, int lane) {
+    const int64_t g0 = q0 & ~(int64_t)31;
+    const float* q = a.ext + 3 * min64(g0 + lane, a.count - 1);
+    const float x = __ldg(q), y = __ldg(q + 1), z = __ldg(q + 2);
+    const float extent =
+        fmaxf(fmaxf(warp_max(x) - warp_min(x), warp_max(y) - warp_min(y)), warp_max(z) - warp_min(z));
+    if (!(extent <= a.close * st->range)) return 1;
+    return q0 == g0 ? 32 : 0;
+}
+
 // Persistent: the grid is the resident blocks and each warp takes its next
 // queries from a counter. With a block per four warps' queries a block kept its
 // registers and shared memory until its slowest warp ended, and 15 of 20
@@ -1139,10 +1163,20 @@ __global__ void __launch_bounds__(KnnCfg<K>::threads, KnnCfg<K>::min_blocks)
     if (lane < kQueryCounters) W.count[lane] = 0;
     __syncwarp();
     const int64_t n = a.device_count ? (int64_t)st->u : a.count;
-    const uint32_t items = (uint32_t)((n + a.warp_queries - 1) / a.warp_queries);
+    const bool listed = EXT && a.order;
+    const uint32_t items = listed ? __ldg(&st->items) : (uint32_t)((n + a.warp_queries - 1) / a.warp_queries);
     uint32_t item = blockIdx.x * KnnCfg<K>::warps + warp;
     while (item < items) {
-        knn_warp<K, EXACT, EXT, NORMALS, CELLS>(pts, snodes, codes, a, st, (int64_t)item * a.warp_queries, W, lane);
+        int64_t q0 = (int64_t)item * a.warp_queries;
+        int nq = a.warp_queries;
+        if (listed) {
+            const uint64_t e = __ldg(a.items + item);
+            q0 = (int64_t)(uint32_t)e;
+            nq = (int)(e >> 32);
+        } else if (EXT && a.close > 0.0f) {
+            nq = foreign_share(a, st, q0, lane);
+        }
+        if (!EXT || nq > 0) knn_warp<K, EXACT, EXT, NORMALS, CELLS>(pts, snodes, codes, a, st, q0, nq, W, lane);
         __syncwarp();
         if (lane == 0) item = gridDim.x * KnnCfg<K>::warps + atomicAdd(&st->work, 1u);
         item = __shfl_sync(FULL, item, 0);
@@ -1191,7 +1225,7 @@ __global__ void __launch_bounds__(BatchCfg<K, NW>::threads, BatchCfg<K, NW>::min
         ca.out_normals = d.out_normals;
         ca.start = 0;
         ca.device_count = 1;
-        knn_warp<K, EXACT, false, true, false>(d.pts, d.snodes, nullptr, ca, d.st, ((int64_t)item - d.item0) * 32,
+        knn_warp<K, EXACT, false, true, false>(d.pts, d.snodes, nullptr, ca, d.st, ((int64_t)item - d.item0) * 32, 32,
                                                W, lane);
         __syncwarp();
         if (lane < kQueryCounters && W.count[lane]) {
@@ -1342,13 +1376,20 @@ int queries_per_warp(int64_t count, int num_sms, bool foreign) {
     // warps per SM as the aim the wider spread costs more than it shortens
     // (10k points 141 us, 40k points 230 against 197 us); from 48k points on
     // every choice is 32.
-    // Foreign queries share less, and until they are two to a warp they need not
-    // be sorted: 60 warps per SM (10k queries in a 2M-point precision mix, k = 8
-    // and 32: 345 and 597 us at 10 per SM, 122 and 360 us at 60; 60k: 609 and
-    // 1072, 532 and 1115; at 120 k = 32 loses: 1314).
+    // Foreign queries in order share less: 40 warps per SM (near a 2M-point
+    // scene, k = 8, 4 / 8 / 16 / 32 to a warp: 30k of them 281, 341, 536, 790 us;
+    // 60k 429, 413, 554, 852; 100k 548, 472, 466, 1068; 250k 859, 763, 702, 656).
     int per = 32;
-    while (per > 1 && (count + per - 1) / per < (int64_t)(foreign ? 60 : 10) * num_sms) per /= 2;
+    while (per > 1 && (count + per - 1) / per < (int64_t)(foreign ? 40 : 10) * num_sms) per /= 2;
     return per;
+}
+
+bool order_foreign(int64_t count, int k, int num_sms) {
+    // The order takes about 60 us. Queries near a 2M-point scene, one to a warp as
+    // given and in order, k = 1, 8, 16, 32: 20k of them 145, 220, 320, 694 us and
+    // 200, 240, 317, 541 us; 30k 196, 294, 447, 978 and 211, 281, 377, 627; 40k
+    // 249, 383, 580, 1297 and 233, 322, 441, 775.
+    return count >= (int64_t)(k <= 16 ? 180 : 120) * num_sms;
 }
 
 cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t s, int num_sms) {
@@ -1370,19 +1411,23 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     a.gap = q.eigengap_fp64;
     a.code_bits = q.code_bits;
     a.seed_halo = q.seed_halo;
-    a.learned_r2 = q.learned_r2;
     a.learned_skip_seed = q.learned_skip_seed;
     a.device_count = q.device_count;
     a.step_limit = q.step_limit;
     if (q.ext_queries) {
         a.order = q.order;
         a.order_shift = q.order_shift;
+        a.items = q.items;
+        // queries as given: close ones gain once there are more than warps fit;
+        // a box of the tree's point spacing, were the points spread over its cube
+        a.close = q.count > 20 * num_sms ? 1.0f / cbrtf((float)q.u) : 0.0f;
     } else {
+        a.learned_r2 = q.learned_r2;
         a.cell_lut = q.learned_r2 ? q.cell_lut : nullptr;
         a.lut_shift = q.lut_shift;
+        a.cell_pmax = q.cell_pmax;
+        a.cell_span = q.cell_span < 2 ? 2 : (q.cell_span > 4 ? 4 : q.cell_span);
     }
-    a.cell_pmax = q.cell_pmax;
-    a.cell_span = q.cell_span < 2 ? 2 : (q.cell_span > 4 ? 4 : q.cell_span);
     if (a.seed_halo > kMaxHalo) a.seed_halo = kMaxHalo;
     if (a.seed_halo < 0) a.seed_halo = 0;
     a.warp_queries = q.ext_queries && !q.order ? 1 : queries_per_warp(q.count, num_sms, q.ext_queries != nullptr);

@@ -42,6 +42,8 @@ struct DevState {
     // what a query clears and the host reads after it
     uint32_t err;
     uint32_t work;  // next work item of a persistent search launch
+    uint32_t items;  // foreign queries: entries of its list of work items
+    uint32_t spare;
     unsigned long long counters[kQueryCounters];  // in the order of se_stats
     // what the host reads after a build
     unsigned long long u;      // unique codes
@@ -59,7 +61,8 @@ struct DevState {
     int32_t n_active;                       // non-trivial sort passes
     int32_t pass_active[kSortPasses];
     int32_t pass_parity[kSortPasses];
-    uint32_t tile_counter[16];              // dynamic tile ids: sort passes, dedup, octree scan, leaves; encode's blocks
+    uint32_t tile_counter[15];              // dynamic tile ids: sort passes, dedup, octree scan, leaves; encode's blocks
+    uint32_t disorder;                      // given keys were not in order
     uint32_t hist[kSortPasses][kSortBins];       // per-digit histograms of the codes
     uint32_t digit_off[kSortPasses][kSortBins];  // exclusive digit offsets
 };
@@ -214,13 +217,26 @@ struct QueryOrder {
     uint32_t* lookback;  // kSortBins words per 4096-key tile
     DevState* st;
 };
-// *order receives the sorted keys (keys0 or keys1), *shift the scale of the
-// places, *launches the number of kernels launched.
+// *order receives the sorted keys (keys0 or keys1), *items the search's work
+// items in the other buffer (their number goes into b.st->items), *shift the
+// scale of the places, *launches the number of kernels launched.
 cudaError_t enqueue_query_order(const BuildBufs& b, const QueryOrder& o, const float* queries, int64_t n, int64_t u,
-                                int code_bits, const uint64_t** order, int* shift, cudaStream_t s, int num_sms,
-                                int* launches);
-// Queries per warp of a search of `count` queries.
+                                int code_bits, const uint64_t** order, const uint64_t** items, int* shift,
+                                cudaStream_t s, int num_sms, int* launches);
+// Queries per warp of a search of `count` queries, and whether foreign ones are
+// put in order (those that are not come one to a warp).
 int queries_per_warp(int64_t count, int num_sms, bool foreign);
+bool order_foreign(int64_t count, int k, int num_sms);
+// A work item of sorted foreign queries: the first of them in the low half, how
+// many in the high half. Places that the queries of one warp may span: as many
+// as the foreign rule allows, and as many as of the tree's own points (which
+// share nearly everything). 250k queries near a 2M-point scene, k = 8: 1046 us
+// without seed windows for those that span less, 721 us with windows up to 256
+// places, 674 us up to 512 (4096 cost more than they save). The second bound at
+// 1024 makes 50k queries 694 us, at 64 every seventh tree point as a query (50k)
+// 373 us; as now 400 and 293 us.
+constexpr int kWindowSpan = 512;
+constexpr int kTogetherSpan = 256;
 
 struct QueryParams {
     int k;
@@ -229,6 +245,7 @@ struct QueryParams {
     int64_t u;          // tree points
     const float* ext_queries;  // AoS xyz external queries or nullptr (self queries)
     const uint64_t* order = nullptr;  // external queries: their order (enqueue_query_order), or nullptr: as given
+    const uint64_t* items = nullptr;  // with order: the work items
     int order_shift = 0;
     int32_t* out_idx;   // count*k or nullptr
     float* out_d2;      // count*k or nullptr

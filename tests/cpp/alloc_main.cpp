@@ -53,15 +53,17 @@ cudaError_t enqueue_build(const BuildBufs& b, const BuildParams& p, cudaStream_t
     return cudaSuccess;
 }
 cudaError_t enqueue_octree(const BuildBufs&, const BuildParams&, cudaStream_t, int*) { return cudaSuccess; }
-int queries_per_warp(int64_t count, int, bool) { return count > 5000 ? 32 : 1; }
+bool order_foreign(int64_t count, int, int) { return count > 5000; }
 cudaError_t enqueue_query_order(const BuildBufs&, const QueryOrder& o, const float* q, int64_t n, int64_t, int,
-                                const uint64_t** order, int* shift, cudaStream_t, int, int* launches) {
+                                const uint64_t** order, const uint64_t** items, int* shift, cudaStream_t, int,
+                                int* launches) {
     const int64_t tiles = (n + kSortTile - 1) / kSortTile;
     if (!(live(q, 12 * n, "order: queries") && live(o.keys0, 8 * n, "order: keys0") &&
           live(o.keys1, 8 * n, "order: keys1") && live(o.lookback, 3 * 4 * tiles * kSortBins, "order: lookback") &&
           live(o.st, sizeof(DevState), "order: st")))
         return cudaErrorInvalidValue;
     *order = o.keys0;
+    *items = o.keys1;
     *shift = 0;
     ++*launches;
     return cudaSuccess;
