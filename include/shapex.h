@@ -104,8 +104,10 @@ typedef struct se_options {
     int32_t batch_lanes;           /* streams the clouds' builds are spread over (1..16;
                                       default 16) */
     int32_t batch_lane_min_points; /* clouds of at least this many points are queried on
-                                      their stream right after their build, the others in
-                                      the shared persistent launches (default 262144) */
+                                      their stream right after their build (default
+                                      262144), and so are those that share their k with
+                                      none below that, or, from 65536 points, with one;
+                                      the others in the shared persistent launches */
     int32_t batch_blocks_per_sm;   /* resident blocks per SM of the persistent launches
                                       (default: as many as fit) */
     int32_t batch_warps_per_block; /* warps per block of the persistent launches: 2 or 4

@@ -24,7 +24,13 @@ namespace {
 // tail where a launch per cloud has one each: with clouds queried on their lane
 // from 65536 points on the 256 take 33.2 ms, from 262144 30.6 ms, never
 // 29.5 ms; but few large clouds are better off starting their queries before
-// the last of them is built (8 of 1M: 8.0 ms, 8.6 in one launch).
+// the last of them is built (8 of 1M: 8.0 ms, 8.6 in one launch). Shared by one or
+// two clouds a launch only waits for the others: 8 clouds of 8 different k, in
+// launches per k and on their lanes, take 801 and 337 us (1k points each), 1590
+// and 999 (20k), 2317 and 1696 (100k), 3355 and 2768 (200k); 8 of 4 different k
+// 453 and 354 us (1k), 940 and 1056 (20k), 1359 and 1242 (60k), 2804 and 2762
+// (200k); 16 of 4 different k 1089 and 1931 (20k), 2842 and 3145 (100k).
+constexpr int64_t kLaneQueryPair = 65536;
 int batch_lanes(const se_ctx* c) { return c->opt.batch_lanes > 0 ? c->opt.batch_lanes : 16; }
 int64_t batch_lane_min(const se_ctx* c) {
     return c->opt.batch_lane_min_points > 0 ? (int64_t)c->opt.batch_lane_min_points : 262144;
@@ -252,7 +258,9 @@ int se_normals_batch(se_ctx* c, const float* x, const float* y, const float* z, 
 
     // ---- plan ----
     // Clouds of at least kLaneQueryMin points are queried on their lane right
-    // after their build (a launch of their own fills enough of the GPU). The
+    // after their build (a launch of their own fills enough of the GPU), and so
+    // are those that would share their launch with none or, from kLaneQueryPair
+    // points on, one other: the shared launches run one after another. The
     // rest share one persistent launch per k, after their builds; their k
     // groups go largest k first, so the costliest queries start while the
     // lanes still build later groups. Lanes take the large clouds first, then
@@ -267,10 +275,15 @@ int se_normals_batch(se_ctx* c, const float* x, const float* y, const float* z, 
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         return offsets[a + 1] - offsets[a] > offsets[b + 1] - offsets[b];
     });
+    int sharing[33] = {};  // clouds below the cut-off, by k
+    for (int ci : order) {
+        const int64_t n = offsets[ci + 1] - offsets[ci];
+        if (n > 0 && n < kLaneQueryMin) ++sharing[ks[ci]];
+    }
     for (int ci : order) {
         const int64_t n = offsets[ci + 1] - offsets[ci];
         if (n == 0) continue;
-        if (n >= kLaneQueryMin) {
+        if (n >= kLaneQueryMin || sharing[ks[ci]] == 1 || (sharing[ks[ci]] == 2 && n >= kLaneQueryPair)) {
             plan.lane_query[ci] = 1;
             ++plan.n_lane_queries;
         } else if (std::find(plan.group_k.begin(), plan.group_k.end(), ks[ci]) == plan.group_k.end()) {
