@@ -100,7 +100,7 @@ typedef struct se_options {
     int32_t cell_max_points;   /* cell scan: a warp whose cells hold more points walks the
                                   tree instead (0: the default, 4096) */
     /* se_normals_batch scheduling (0: the default of each); se_tune_batch
-     * measures and sets them, with leaf_bucket and seed_halo. */
+     * measures and sets them, with seed_halo. */
     int32_t batch_lanes;           /* streams the clouds' builds are spread over (1..16;
                                       default 16) */
     int32_t batch_lane_min_points; /* clouds of at least this many points are queried on
@@ -240,17 +240,17 @@ typedef struct se_batch_tuning {
     int32_t lanes;
     int32_t lane_min_points;
     int32_t blocks_per_sm;   /* 0: as many as fit */
-    int32_t warps_per_block; /* 0: per k */
+    int32_t warps_per_block; /* 0: 2 */
 } se_batch_tuning;
 SE_API int se_get_batch_tuning(const se_ctx* ctx, se_batch_tuning* tuning);
 SE_API int se_set_batch_tuning(se_ctx* ctx, const se_batch_tuning* tuning);
 
 /* Autotuner for se_normals_batch: times the given batch (the same arguments
  * as se_normals_batch, outputs to internal memory) with CUDA events under
- * candidate tunings, one parameter at a time over two rounds (bucket 48..128,
- * halo, lanes 4..16, lane cut-off 2^15..2^18, resident blocks, 2- or 4-warp
- * blocks), `reps` timed calls each (median), and leaves the fastest set on
- * the context. best and best_ms (optional) receive it and its time. */
+ * candidate tunings, one parameter at a time over two rounds (halo, lanes
+ * 4..16, lane cut-off 2^15..2^18 or none, 2- or 4-warp blocks; values that
+ * come to the same schedule once), `reps` timed calls each (median), and
+ * leaves the fastest set on the context. best and best_ms (optional) receive it and its time. */
 SE_API int se_tune_batch(se_ctx* ctx, const float* x, const float* y, const float* z, const int64_t* offsets,
                   int n_clouds, const int32_t* ks, int mem, int reps, se_batch_tuning* best, float* best_ms);
 

@@ -1,11 +1,12 @@
 """Autotuner for the kNN kernel's tile parameters and the batch schedule.
 
-Two parameters shape the search kernel's work: `leaf_bucket` (subtrees of at
-most this many points are streamed as one tile) and `seed_halo` (Morton-window
+One parameter shapes the search kernel's work: `seed_halo` (Morton-window
 points offered on each side of a warp's 32 queries before the tree walk). The
+leaves of the search hierarchy hold 32 points, the most they can: smaller ones
+(`leaf_bucket`) searched a 1M-point scene more slowly at every size and k. The
 batched path adds its schedule: stream lanes, the size above which a cloud is
-queried on its lane, and the persistent launches' resident blocks per SM and
-warps per block. The best values depend on density, k and the batch's size
+queried on its lane, and the persistent launches' warps per block.
+The best values depend on density, k and the batch's size
 mix, so they are measured, not guessed, on the caller's own cloud or batch
 (single clouds here with CUDA events around the build and the fused kNN +
 normals kernel; batches in the library, se_tune_batch), and the winner is
@@ -22,7 +23,7 @@ import numpy as np
 
 from ._native import Context
 
-CANDIDATES = [(b, h) for b in (32, 64, 96) for h in (8, 16, 32)]
+CANDIDATES = [(32, h) for h in (8, 16, 32, 48)]  # (leaf_bucket, seed_halo)
 DEFAULT_CACHE = os.path.join(os.path.expanduser("~"), ".cache", "shapeextraction_b200", "autotune.json")
 
 
@@ -87,9 +88,9 @@ def batch_key(clouds, ks, code_bits=63) -> str:
 
 
 def tune_batch(clouds, ks, code_bits=63, device=0, cache_path=DEFAULT_CACHE, reps=2, force=False, ctx=None):
-    """Best se_normals_batch tuning for this batch's class: bucket size, seed
-    halo, stream lanes, the per-lane query cut-off, and the persistent
-    launches' resident blocks and block shape. The search runs in the library
+    """Best se_normals_batch tuning for this batch's class: seed halo, stream
+    lanes, the per-lane query cut-off, and the persistent launches' block
+    shape. The search runs in the library
     (se_tune_batch: CUDA events around whole batched calls, one parameter at
     a time over two rounds); the winner is cached per class and, when `ctx`
     is given, left set on it."""

@@ -358,7 +358,7 @@ int se_normals_batch(se_ctx* c, const float* x, const float* y, const float* z, 
     key.push_back((int64_t)(uintptr_t)out_normals);
     key.push_back((int64_t)c->batch_epoch);
     // the tuning changes the launches
-    key.push_back(c->opt.leaf_bucket);
+    key.push_back(std::min(c->opt.leaf_bucket, kLeafMax));
     key.push_back(c->opt.seed_halo);
     key.push_back(batch_lanes(c));
     key.push_back(kLaneQueryMin);
@@ -524,28 +524,38 @@ int se_tune_batch(se_ctx* c, const float* x, const float* y, const float* z, con
     };
     float cur_ms = 0.0f;
     rc = measure(cur, cur_ms);
-    // coordinate descent, two rounds: each parameter over its values, the others fixed
-    static const int kBucket[] = {48, 64, 96, 128};
+    // Coordinate descent, two rounds: each parameter over its values, the others
+    // fixed. Not tried: leaf sizes below 32 (a 1M scene's search is slower with
+    // every one of them; larger ones are 32) and fewer blocks per SM than fit (256
+    // clouds of 1k to 500k points: 30.5 ms with all, 31.1 to 65.9 ms with fewer).
     static const int kHalo[] = {-1, 8, 16, 32};
     static const int kLanes[] = {4, 8, 16};
-    static const int kLaneMin[] = {32768, 65536, 131072, 262144};
-    static const int kBlocks[] = {0, 2, 3, 4};
+    static const int kLaneMin[] = {32768, 65536, 131072, 262144, 1 << 30};
     static const int kWarps[] = {2, 4};
+    // what a value comes to: the clouds at or above a cut-off, the lanes in use,
+    // the default block shape
+    auto effect = [&](int dim, int v) -> int64_t {
+        if (dim == 1) return std::min(v, n_clouds);
+        if (dim == 2) {
+            int64_t above = 0;
+            for (int i = 0; i < n_clouds; ++i) above += offsets[i + 1] - offsets[i] >= v;
+            return above;
+        }
+        return dim == 3 && v == 0 ? 2 : v;
+    };
     for (int round = 0; round < 2 && rc == SE_OK; ++round) {
-        for (int dim = 0; dim < 6 && rc == SE_OK; ++dim) {
+        for (int dim = 0; dim < 4 && rc == SE_OK; ++dim) {
             const int* vals;
             int nv;
             int32_t se_batch_tuning::*field;
             switch (dim) {
-                case 0: vals = kBucket; nv = 4; field = &se_batch_tuning::leaf_bucket; break;
-                case 1: vals = kHalo; nv = 4; field = &se_batch_tuning::seed_halo; break;
-                case 2: vals = kLanes; nv = 3; field = &se_batch_tuning::lanes; break;
-                case 3: vals = kLaneMin; nv = 4; field = &se_batch_tuning::lane_min_points; break;
-                case 4: vals = kBlocks; nv = 4; field = &se_batch_tuning::blocks_per_sm; break;
+                case 0: vals = kHalo; nv = 4; field = &se_batch_tuning::seed_halo; break;
+                case 1: vals = kLanes; nv = 3; field = &se_batch_tuning::lanes; break;
+                case 2: vals = kLaneMin; nv = 5; field = &se_batch_tuning::lane_min_points; break;
                 default: vals = kWarps; nv = 2; field = &se_batch_tuning::warps_per_block; break;
             }
             for (int vi = 0; vi < nv && rc == SE_OK; ++vi) {
-                if (cur.*field == vals[vi]) continue;
+                if (effect(dim, cur.*field) == effect(dim, vals[vi])) continue;
                 se_batch_tuning t = cur;
                 t.*field = vals[vi];
                 float ms = 0.0f;

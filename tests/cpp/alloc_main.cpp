@@ -11,7 +11,9 @@
 // works all the same), and the three calls then work.
 #include <cstdio>
 #include <functional>
+#include <set>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "alloc_runtime.hpp"
@@ -23,6 +25,9 @@ using fake::complain;
 using fake::live;
 
 // ---- the kernel launchers ----------------------------------------------------
+static std::set<std::pair<int, int>> g_shapes;  // leaf sizes of the builds, blocks per SM of the shared launches
+static int g_batches = 0;                       // batched calls
+
 namespace shapex {
 static void fill(float* p, int64_t n) {
     for (int64_t i = 0; i < n; ++i) p[i] = 7.0f;
@@ -30,6 +35,7 @@ static void fill(float* p, int64_t n) {
 cudaError_t enqueue_build(const BuildBufs& b, const BuildParams& p, cudaStream_t, int, cudaEvent_t*, int* launches) {
     const int64_t n = p.n;
     if (launches) *launches = 1;
+    g_shapes.insert({p.bucket < kLeafMax ? p.bucket : kLeafMax, -1});
     if (!live(b.st, sizeof(DevState), "build: st")) return cudaErrorInvalidValue;
     *b.st = DevState{};
     if (n == 0) return cudaSuccess;
@@ -85,7 +91,8 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     return cudaSuccess;
 }
 cudaError_t enqueue_query_batch(const BatchCloud* clouds, int n_clouds, int64_t, unsigned long long* counter,
-                                const QueryParams&, cudaStream_t, int) {
+                                const QueryParams& q, cudaStream_t, int) {
+    g_shapes.insert({-1, q.batch_blocks_per_sm});
     if (!(live(clouds, sizeof(BatchCloud) * n_clouds, "batch: descriptors") && live(counter, 8, "batch: counter")))
         return cudaErrorInvalidValue;
     for (int i = 0; i < n_clouds; ++i) {
@@ -98,6 +105,7 @@ cudaError_t enqueue_query_batch(const BatchCloud* clouds, int n_clouds, int64_t,
     return cudaSuccess;
 }
 cudaError_t enqueue_batch_collect(const DevState* st, int n, unsigned long long* u, uint32_t* err, cudaStream_t) {
+    ++g_batches;
     for (int i = 0; i < n; ++i) {
         u[i] = st[i].u;
         err[i] = st[i].err;
@@ -256,12 +264,40 @@ static int check(const char* name, const se_options& opt, const Call& call, bool
     return allocs;
 }
 
+// The batch tuner times no schedule twice: no leaf sizes (all those it tried
+// were the same), no limits of the blocks per SM, no cut-offs with the same
+// clouds above them.
+static int tuner(const se_options& opt) {
+    fake::where = "tuner";
+    se_ctx* c = nullptr;
+    se_create(&c, &opt);
+    for (const int big : {1000, 40000}) {
+        const std::vector<int64_t> off{0, 500, 500 + big, 500 + 2 * big, 500 + 3 * big};
+        const std::vector<int32_t> ks{8, 8, 8, 16};
+        std::vector<float> x(off.back());
+        g_shapes.clear();
+        g_batches = 0;
+        se_batch_tuning best;
+        float ms = 0.0f;
+        if (se_tune_batch(c, x.data(), x.data(), x.data(), off.data(), 4, ks.data(), SE_MEM_HOST, 1, &best, &ms) != SE_OK)
+            complain("failed");
+        if (g_shapes.size() != 2) complain("tried leaf sizes or blocks per SM");
+        // two calls each: the present setting; per round 3 halos, the other block shape and,
+        // where clouds lie above 32768 points, that cut-off (4 clouds take 4 lanes at most)
+        if (g_batches != 2 * (1 + 2 * (3 + 1 + (big > 32768)))) complain("other schedules than expected");
+        std::printf("tuner: %d batches\n", g_batches);
+    }
+    se_destroy(c);
+    return fake::bad;
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     se_options opt;
     se_options_init(&opt);
     opt.batch_graph = 0;
     int allocs = 0;
+    if (what == "tuner") return tuner(opt) ? 1 : 0;
     if (what == "train") allocs = check("train", opt, train);
     if (what == "batch slices") {
         opt.batch_lanes = 1;  // one lane, never regrown: it holds 1024 points at least

@@ -35,3 +35,15 @@ def harness(tmp_path_factory):
 def test_a_failed_allocation_leaves_the_context_usable(harness, scenario):
     r = subprocess.run([harness, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_the_batch_tuner_times_no_schedule_twice(harness):
+    r = subprocess.run([harness, "tuner"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_the_cloud_tuner_times_no_setting_twice():
+    from shapeextraction_b200 import autotune
+
+    settings = [(min(bucket, 32), halo) for bucket, halo in autotune.CANDIDATES]
+    assert len(set(settings)) == len(settings)
