@@ -201,7 +201,10 @@ static_assert(24 + (kMaxLevels - 1) * 8 <= 64, "order keys fit behind the staged
 // registers instead of 142, one resident block per SM fewer.
 struct QArgs {
     int64_t start, count, u;
-    const float* ext;
+    union {
+        const float* ext;      // foreign queries
+        const uint64_t* parts;  // the tree's own points: work items (null: warp_queries each)
+    };
     int32_t* out_idx;
     float* out_d2;
     float* out_normals;
@@ -1174,14 +1177,14 @@ __global__ void __launch_bounds__(KnnCfg<K>::threads, KnnCfg<K>::min_blocks)
     if (lane < kQueryCounters) W.count[lane] = 0;
     __syncwarp();
     const int64_t n = a.device_count ? (int64_t)st->u : a.count;
-    const bool listed = EXT && a.order;
+    const bool listed = EXT ? a.order != nullptr : !CELLS && a.parts != nullptr;
     const uint32_t items = listed ? __ldg(&st->items) : (uint32_t)((n + a.warp_queries - 1) / a.warp_queries);
     uint32_t item = blockIdx.x * KnnCfg<K>::warps + warp;
     while (item < items) {
         int64_t q0 = (int64_t)item * a.warp_queries;
         int nq = a.warp_queries;
         if (listed) {
-            const uint64_t e = __ldg(a.items + item);
+            const uint64_t e = __ldg((EXT ? a.items : a.parts) + item);
             q0 = (int64_t)(uint32_t)e;
             nq = (int)(e >> 32);
         } else if (EXT && a.close > 0.0f) {
@@ -1247,6 +1250,59 @@ __global__ void __launch_bounds__(BatchCfg<K, NW>::threads, BatchCfg<K, NW>::min
     }
 }
 
+// Work items of the tree's own points [start, start + count) (all of them on the
+// device's count with device_count): 32 at a time, cut where the Morton order
+// jumps and then into `per`. The jumps are the lowest common prefixes of adjacent
+// codes, `jump` bits below the median of the 32 or lower, three at most. A warp
+// across a jump walks two regions and what lies between, and a call of a few
+// rounds of warps ends with its slowest: normals of 110k points of a scene, k = 8,
+// lasted 249 us for one warp of 3438 (99 of 100 end within 120 us, half within 66).
+// Over scenes, cubes, mixtures and precision mixes, against none cut (6, 7, 8, 9, 10
+// bits): 45k points, k = 8: 0.78, 0.82, 0.84, 0.88, 0.92; 110k, k = 16: 0.93, 0.90,
+// 0.88, 0.88, 0.89; k = 32: 0.98, 0.91, 0.89, 0.89, 0.89; 300k, k = 16: 1.10, 1.01,
+// 0.96, 0.94, 0.95; k = 32: 1.30, 1.14, 1.06, 1.01, 0.99.
+__global__ void __launch_bounds__(256) k_point_items(const uint64_t* __restrict__ codes, int64_t start, int64_t count,
+                                                     int device_count, int per, int jump,
+                                                     uint64_t* __restrict__ items, DevState* st) {
+    __shared__ uint32_t s_at[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t n = device_count ? (int64_t)st->u : count;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const uint64_t code = i < n ? __ldg(codes + start + i) : 0ull;
+    const uint64_t before = __shfl_up_sync(FULL, code, 1);
+    const int shared = lane > 0 && i < n ? __clzll((long long)(code ^ before)) : 64;  // leading bits, 64: no pair
+    int median = 0;  // the most leading bits that 16 adjacent pairs share
+#pragma unroll
+    for (int b = 32; b >= 1; b >>= 1)
+        if (__popc(__ballot_sync(FULL, shared >= median + b)) >= 17) median += b;
+    uint32_t cuts = 0;
+    for (int at = median - jump; at >= 0; --at) {
+        cuts = __ballot_sync(FULL, shared <= at);
+        if (__popc(cuts) <= 3) break;
+    }
+    cuts |= 1u;
+    const int from = 31 - __clz(cuts & (2u * (1u << lane) - 1u));  // where the lane's part begins
+    const uint32_t firsts = __ballot_sync(FULL, i < n && ((lane - from) & (per - 1)) == 0);
+    if (lane == 0) s_at[warp] = __popc(firsts);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t total = 0;
+        for (int w = 0; w < 8; ++w) {
+            const uint32_t c = s_at[w];
+            s_at[w] = total;
+            total += c;
+        }
+        const uint32_t base = atomicAdd(&st->items, total);
+        for (int w = 0; w < 8; ++w) s_at[w] += base;
+    }
+    __syncthreads();
+    if ((firsts >> lane) & 1u) {
+        const uint32_t later = lane < 31 ? firsts >> (lane + 1) : 0u;
+        const int64_t size = later ? __ffs(later) : min64(32, n - (i - lane)) - lane;
+        items[s_at[warp] + __popc(firsts & lanemask_lt())] = ((uint64_t)size << 32) | (uint64_t)i;
+    }
+}
+
 template <int K, bool EXACT, bool EXT, bool NORMALS, bool CELLS = false>
 cudaError_t launch_one(const BuildBufs& b, const QArgs& a, unsigned blocks, cudaStream_t s, int num_sms) {
     constexpr int smem = (int)sizeof(WarpSmem<KnnCfg<K>::buf, CELLS>) * KnnCfg<K>::warps;
@@ -1265,7 +1321,9 @@ cudaError_t launch_one(const BuildBufs& b, const QArgs& a, unsigned blocks, cuda
 
 template <int K, bool EXACT>
 cudaError_t launch_k(const BuildBufs& b, const QArgs& a, bool ext, bool normals, cudaStream_t s, int num_sms) {
-    const int64_t warps = (a.count + a.warp_queries - 1) / a.warp_queries;
+    // Cut items are more than this; while all warps fit at once none of them may
+    // wait for a warp to end (an item that did started 50 us late).
+    const int64_t warps = (a.count + a.warp_queries - 1) / a.warp_queries * (!ext && a.parts ? 2 : 1);
     const unsigned blocks = (unsigned)((warps + KnnCfg<K>::warps - 1) / KnnCfg<K>::warps);
     if (ext) return launch_one<K, EXACT, true, false>(b, a, blocks, s, num_sms);
     if (a.cell_lut) {
@@ -1385,14 +1443,20 @@ int queries_per_warp(int64_t count, int num_sms, bool foreign) {
     // as one warp: 2k points, k = 8, 74 us with 32 queries per warp and 39 us
     // with one; 10k points, k = 16, 162 and 115 us (eight per warp). With 20
     // warps per SM as the aim the wider spread costs more than it shortens
-    // (10k points 141 us, 40k points 230 against 197 us); from 48k points on
-    // every choice is 32.
+    // (10k points 141 us, 40k points 230 against 197 us).
     // Foreign queries in order share less: 40 warps per SM (near a 2M-point
     // scene, k = 8, 4 / 8 / 16 / 32 to a warp: 30k of them 281, 341, 536, 790 us;
     // 60k 429, 413, 554, 852; 100k 548, 472, 466, 1068; 250k 859, 763, 702, 656).
     int per = 32;
     while (per > 1 && (count + per - 1) / per < (int64_t)(foreign ? 40 : 10) * num_sms) per /= 2;
     return per;
+}
+
+bool list_points(int64_t count, int num_sms) {
+    // Of the time without the list: 12k points 0.87 to 0.93, 500k 0.93 (k = 4) to
+    // 1.01 (k = 32), 1M 0.99 to 1.05. At four and fewer per warp there is little to
+    // cut.
+    return queries_per_warp(count, num_sms, false) >= 8 && count <= (int64_t)3400 * num_sms;
 }
 
 bool order_foreign(int64_t count, int k, int num_sms) {
@@ -1412,7 +1476,6 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     a.start = q.start;
     a.count = q.count;
     a.u = q.u;
-    a.ext = q.ext_queries;
     a.out_idx = q.out_idx;
     a.out_d2 = q.out_d2;
     a.out_normals = q.out_normals;
@@ -1426,6 +1489,7 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     a.device_count = q.device_count;
     a.step_limit = q.step_limit;
     if (q.ext_queries) {
+        a.ext = q.ext_queries;
         a.order = q.order;
         a.order_shift = q.order_shift;
         a.items = q.items;
@@ -1433,6 +1497,7 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
         // a box of the tree's point spacing, were the points spread over its cube
         a.close = q.count > 20 * num_sms ? 1.0f / cbrtf((float)q.u) : 0.0f;
     } else {
+        a.parts = nullptr;
         a.learned_r2 = q.learned_r2;
         a.cell_lut = q.learned_r2 ? q.cell_lut : nullptr;
         a.lut_shift = q.lut_shift;
@@ -1443,6 +1508,13 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     if (a.seed_halo < 0) a.seed_halo = 0;
     a.warp_queries = q.ext_queries && !q.order ? 1 : queries_per_warp(q.count, num_sms, q.ext_queries != nullptr);
     const bool ext = q.ext_queries != nullptr;
+    if (!ext && !a.cell_lut && list_points(q.count, num_sms)) {
+        uint64_t* items = reinterpret_cast<uint64_t*>(b.scratch);  // the build is done with it
+        const int jump = q.count <= (int64_t)1600 * num_sms ? 8 : 9;
+        k_point_items<<<(unsigned)((q.count + 255) / 256), 256, 0, s>>>(b.codes, q.start, q.count, q.device_count,
+                                                                        a.warp_queries, jump, items, b.st);
+        a.parts = items;
+    }
     const bool nrm = q.out_normals != nullptr && !ext;
     switch (q.k) {
         case 8: return launch_k<8, true>(b, a, ext, nrm, s, num_sms);

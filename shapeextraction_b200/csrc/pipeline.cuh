@@ -42,7 +42,7 @@ struct DevState {
     // what a query clears and the host reads after it
     uint32_t err;
     uint32_t work;  // next work item of a persistent search launch
-    uint32_t items;  // foreign queries: entries of its list of work items
+    uint32_t items;  // entries of a search's list of work items
     uint32_t spare;
     unsigned long long counters[kQueryCounters];  // in the order of se_stats
     // what the host reads after a build
@@ -227,6 +227,9 @@ cudaError_t enqueue_query_order(const BuildBufs& b, const QueryOrder& o, const f
 // put in order (those that are not come one to a warp).
 int queries_per_warp(int64_t count, int num_sms, bool foreign);
 bool order_foreign(int64_t count, int k, int num_sms);
+// Whether a search of `count` of the tree's own points lists its work items
+// first (one more kernel; the list takes b.scratch).
+bool list_points(int64_t count, int num_sms);
 // A work item of sorted foreign queries: the first of them in the low half, how
 // many in the high half. Places that the queries of one warp may span: as many
 // as the foreign rule allows, and as many as of the tree's own points (which
