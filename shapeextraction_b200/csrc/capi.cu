@@ -284,7 +284,7 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
                     "copy normals");
     }
     c->query_launches = (use_learned ? 2 : 1) + (lut_launched ? 1 : 0) + order_launches +
-                        (!ext && !q.compat && !cells && list_points(count, c->num_sms) ? 1 : 0);
+                        (!ext && !q.compat && !cells && list_points(count, k, c->num_sms) ? 1 : 0);
     c->have_query_times = true;
     SE_CUDA(c, cudaMemcpyAsync(c->h_st, c->b.st, kQueryStateBytes, cudaMemcpyDeviceToHost, c->stream), "read state");
     c->h_st->n_active = 0;

@@ -188,6 +188,7 @@ struct WarpSmem {
     float d[B][32];
     int32_t idx[B][32];
     uint32_t count[kQueryCounters];  // the warp's work counters, added to the build state's when it ends
+    uint32_t whole, items;           // work items of the launch: those from the front of a list, all
     float4 box_lo, box_hi;           // the box of the warp's active queries
     __device__ __forceinline__ uint32_t* level_keys(int l) {  // l >= 1
         return reinterpret_cast<uint32_t*>(&pts[24]) + 32 * (l - 1);
@@ -213,8 +214,9 @@ struct QArgs {
         const uint64_t* items;  // foreign queries with an order: the work items
     };
     union {
-        const uint32_t* cell_lut;  // learned cell scan: code-range table (null: tree walk with the cap)
-        const uint64_t* order;     // foreign queries: their order (null: as given)
+        const uint32_t* cell_lut;   // learned cell scan: code-range table (null: tree walk with the cap)
+        const uint64_t* order;      // foreign queries: their order (null: as given)
+        const uint64_t* parts_end;  // with `parts` (and no cell scan)
     };
     float vx, vy, vz;
     float gap;
@@ -1178,13 +1180,17 @@ __global__ void __launch_bounds__(KnnCfg<K>::threads, KnnCfg<K>::min_blocks)
     __syncwarp();
     const int64_t n = a.device_count ? (int64_t)st->u : a.count;
     const bool listed = EXT ? a.order != nullptr : !CELLS && a.parts != nullptr;
-    const uint32_t items = listed ? __ldg(&st->items) : (uint32_t)((n + a.warp_queries - 1) / a.warp_queries);
+    if (lane == 0) {  // kept here: a register less across the search
+        W.whole = listed ? __ldg(&st->items) : (uint32_t)((n + a.warp_queries - 1) / a.warp_queries);
+        W.items = listed && !EXT ? W.whole + __ldg(&st->parts) : W.whole;
+    }
+    __syncwarp();
     uint32_t item = blockIdx.x * KnnCfg<K>::warps + warp;
-    while (item < items) {
+    while (item < W.items) {
         int64_t q0 = (int64_t)item * a.warp_queries;
         int nq = a.warp_queries;
         if (listed) {
-            const uint64_t e = __ldg((EXT ? a.items : a.parts) + item);
+            const uint64_t e = __ldg(EXT ? a.items + item : item < W.whole ? a.parts + item : a.parts_end - 1 - (item - W.whole));
             q0 = (int64_t)(uint32_t)e;
             nq = (int)(e >> 32);
         } else if (EXT && a.close > 0.0f) {
@@ -1250,23 +1256,25 @@ __global__ void __launch_bounds__(BatchCfg<K, NW>::threads, BatchCfg<K, NW>::min
     }
 }
 
-// Work items of the tree's own points [start, start + count) (all of them on the
-// device's count with device_count): 32 at a time, cut where the Morton order
-// jumps and then into `per`. The jumps are the lowest common prefixes of adjacent
-// codes, `jump` bits below the median of the 32 or lower, three at most. A warp
-// across a jump walks two regions and what lies between, and a call of a few
-// rounds of warps ends with its slowest: normals of 110k points of a scene, k = 8,
-// lasted 249 us for one warp of 3438 (99 of 100 end within 120 us, half within 66).
-// Over scenes, cubes, mixtures and precision mixes, against none cut (6, 7, 8, 9, 10
-// bits): 45k points, k = 8: 0.78, 0.82, 0.84, 0.88, 0.92; 110k, k = 16: 0.93, 0.90,
+// Work items of the tree's own points [start, start + count): 32 at a time, cut
+// where the Morton order jumps and then into `per`. The jumps are the lowest common
+// prefixes of adjacent codes, `jump` bits below the median of the 32 or lower, three
+// at most. A warp across a jump walks two regions and what lies between, and a call
+// of a few rounds of warps ends with its slowest: normals of 110k points of a scene,
+// k = 8, lasted 249 us for one warp of 3438 (99 of 100 end within 120 us, half within
+// 66). Over scenes, cubes, mixtures and precision mixes, against none cut (6, 7, 8, 9,
+// 10 bits): 45k points, k = 8: 0.78, 0.82, 0.84, 0.88, 0.92; 110k, k = 16: 0.93, 0.90,
 // 0.88, 0.88, 0.89; k = 32: 0.98, 0.91, 0.89, 0.89, 0.89; 300k, k = 16: 1.10, 1.01,
 // 0.96, 0.94, 0.95; k = 32: 1.30, 1.14, 1.06, 1.01, 0.99.
-__global__ void __launch_bounds__(256) k_point_items(const uint64_t* __restrict__ codes, int64_t start, int64_t count,
-                                                     int device_count, int per, int jump,
-                                                     uint64_t* __restrict__ items, DevState* st) {
-    __shared__ uint32_t s_at[8];
+// Whole items fill the list from its front and parts, which end sooner, from its
+// back (room entries on), so that parts are what starts late when not all fit at
+// once.
+constexpr int kItemBytes = 2;  // of the list, per point: 4 + 32 / 8 - 1 parts of 8 bytes in 32 points
+__global__ void __launch_bounds__(256) k_point_items(const uint64_t* __restrict__ codes, int64_t start, int64_t n,
+                                                     int per, int jump, uint64_t* __restrict__ items, int64_t room,
+                                                     DevState* st) {
+    __shared__ uint32_t s_at[2][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t n = device_count ? (int64_t)st->u : count;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const uint64_t code = i < n ? __ldg(codes + start + i) : 0ull;
     const uint64_t before = __shfl_up_sync(FULL, code, 1);
@@ -1283,23 +1291,32 @@ __global__ void __launch_bounds__(256) k_point_items(const uint64_t* __restrict_
     cuts |= 1u;
     const int from = 31 - __clz(cuts & (2u * (1u << lane) - 1u));  // where the lane's part begins
     const uint32_t firsts = __ballot_sync(FULL, i < n && ((lane - from) & (per - 1)) == 0);
-    if (lane == 0) s_at[warp] = __popc(firsts);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t total = 0;
-        for (int w = 0; w < 8; ++w) {
-            const uint32_t c = s_at[w];
-            s_at[w] = total;
-            total += c;
-        }
-        const uint32_t base = atomicAdd(&st->items, total);
-        for (int w = 0; w < 8; ++w) s_at[w] += base;
+    const uint32_t later = lane < 31 ? firsts >> (lane + 1) : 0u;
+    const int64_t size = later ? __ffs(later) : min64(32, n - (i - lane)) - lane;
+    const bool first = (firsts >> lane) & 1u;
+    const uint32_t whole = __ballot_sync(FULL, first && size == per), part = firsts & ~whole;
+    if (lane == 0) {
+        s_at[0][warp] = __popc(whole);
+        s_at[1][warp] = __popc(part);
     }
     __syncthreads();
-    if ((firsts >> lane) & 1u) {
-        const uint32_t later = lane < 31 ? firsts >> (lane + 1) : 0u;
-        const int64_t size = later ? __ffs(later) : min64(32, n - (i - lane)) - lane;
-        items[s_at[warp] + __popc(firsts & lanemask_lt())] = ((uint64_t)size << 32) | (uint64_t)i;
+    if (threadIdx.x < 2) {
+        uint32_t* at = s_at[threadIdx.x];
+        uint32_t total = 0;
+        for (int w = 0; w < 8; ++w) {
+            const uint32_t c = at[w];
+            at[w] = total;
+            total += c;
+        }
+        const uint32_t base = atomicAdd(threadIdx.x == 0 ? &st->items : &st->parts, total);
+        for (int w = 0; w < 8; ++w) at[w] += base;
+    }
+    __syncthreads();
+    if (first) {
+        const bool w = (whole >> lane) & 1u;
+        const int64_t at = w ? s_at[0][warp] + __popc(whole & lanemask_lt())
+                             : room - 1 - (s_at[1][warp] + __popc(part & lanemask_lt()));
+        items[at] = ((uint64_t)size << 32) | (uint64_t)i;
     }
 }
 
@@ -1326,7 +1343,7 @@ cudaError_t launch_k(const BuildBufs& b, const QArgs& a, bool ext, bool normals,
     const int64_t warps = (a.count + a.warp_queries - 1) / a.warp_queries * (!ext && a.parts ? 2 : 1);
     const unsigned blocks = (unsigned)((warps + KnnCfg<K>::warps - 1) / KnnCfg<K>::warps);
     if (ext) return launch_one<K, EXACT, true, false>(b, a, blocks, s, num_sms);
-    if (a.cell_lut) {
+    if (a.cell_lut && !a.parts) {
         if (normals) return launch_one<K, EXACT, false, true, true>(b, a, blocks, s, num_sms);
         return launch_one<K, EXACT, false, false, true>(b, a, blocks, s, num_sms);
     }
@@ -1452,11 +1469,14 @@ int queries_per_warp(int64_t count, int num_sms, bool foreign) {
     return per;
 }
 
-bool list_points(int64_t count, int num_sms) {
-    // Of the time without the list: 12k points 0.87 to 0.93, 500k 0.93 (k = 4) to
-    // 1.01 (k = 32), 1M 0.99 to 1.05. At four and fewer per warp there is little to
-    // cut.
-    return queries_per_warp(count, num_sms, false) >= 8 && count <= (int64_t)3400 * num_sms;
+bool list_points(int64_t count, int k, int num_sms) {
+    // At four and fewer per warp there is little to cut; many rounds of warps hide
+    // their slowest, and the parts' work adds up, the more so the longer the lists
+    // (normals of precision mixes, of the time without the list, k = 4, 8, 16, 32:
+    // 130k points 0.76, 0.76, 0.76, 0.79; 220k 0.78, 0.83, 0.91, 1.00; 300k 0.93, 1.00,
+    // 1.05, 1.12; scenes 300k 0.88, 0.87, 0.89, 0.94; a scene of 207k, k = 31: 1.09).
+    const int most = k <= 8 ? 2600 : (k <= 16 ? 1500 : 750);
+    return queries_per_warp(count, num_sms, false) >= 8 && count <= (int64_t)most * num_sms;
 }
 
 bool order_foreign(int64_t count, int k, int num_sms) {
@@ -1508,12 +1528,13 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     if (a.seed_halo < 0) a.seed_halo = 0;
     a.warp_queries = q.ext_queries && !q.order ? 1 : queries_per_warp(q.count, num_sms, q.ext_queries != nullptr);
     const bool ext = q.ext_queries != nullptr;
-    if (!ext && !a.cell_lut && list_points(q.count, num_sms)) {
+    if (!ext && !a.cell_lut && !q.device_count && list_points(q.count, q.k, num_sms)) {
         uint64_t* items = reinterpret_cast<uint64_t*>(b.scratch);  // the build is done with it
-        const int jump = q.count <= (int64_t)1600 * num_sms ? 8 : 9;
-        k_point_items<<<(unsigned)((q.count + 255) / 256), 256, 0, s>>>(b.codes, q.start, q.count, q.device_count,
-                                                                        a.warp_queries, jump, items, b.st);
+        const int64_t room = q.count * kItemBytes / (int64_t)sizeof(uint64_t);
+        k_point_items<<<(unsigned)((q.count + 255) / 256), 256, 0, s>>>(
+            b.codes, q.start, q.count, a.warp_queries, q.count <= (int64_t)1600 * num_sms ? 8 : 9, items, room, b.st);
         a.parts = items;
+        a.parts_end = items + room;
     }
     const bool nrm = q.out_normals != nullptr && !ext;
     switch (q.k) {

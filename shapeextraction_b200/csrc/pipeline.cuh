@@ -42,8 +42,8 @@ struct DevState {
     // what a query clears and the host reads after it
     uint32_t err;
     uint32_t work;  // next work item of a persistent search launch
-    uint32_t items;  // entries of a search's list of work items
-    uint32_t spare;
+    uint32_t items;  // entries of a search's list of work items, from its front
+    uint32_t parts;  // and from its back
     unsigned long long counters[kQueryCounters];  // in the order of se_stats
     // what the host reads after a build
     unsigned long long u;      // unique codes
@@ -228,8 +228,9 @@ cudaError_t enqueue_query_order(const BuildBufs& b, const QueryOrder& o, const f
 int queries_per_warp(int64_t count, int num_sms, bool foreign);
 bool order_foreign(int64_t count, int k, int num_sms);
 // Whether a search of `count` of the tree's own points lists its work items
-// first (one more kernel; the list takes b.scratch).
-bool list_points(int64_t count, int num_sms);
+// first (one more kernel; the list takes b.scratch). Not where other clouds fill
+// the GPU beside it (device_count).
+bool list_points(int64_t count, int k, int num_sms);
 // A work item of sorted foreign queries: the first of them in the low half, how
 // many in the high half. Places that the queries of one warp may span: as many
 // as the foreign rule allows, and as many as of the tree's own points (which

@@ -57,11 +57,11 @@ def test_both_sides_of_the_rules(native, oracle):
     rng = np.random.default_rng(32)
     sms = _sms()
     with native.Context(build_octree=False) as c, native.Context(code_bits=30, build_octree=False) as c30:
-        x, y, z = (np.ascontiguousarray(v, np.float32) for v in rng.random((3, 3400 * sms + 4_000)))
+        x, y, z = (np.ascontiguousarray(v, np.float32) for v in rng.random((3, 2600 * sms + 4_000)))
         u = c.build(x, y, z)["n_points"]
-        for k in (8, 12):
-            for count, launches in ((40 * sms, 1), (80 * sms - 8, 1), (80 * sms, 2), (1600 * sms, 2),
-                                    (1600 * sms + 1, 2), (3400 * sms, 2), (3400 * sms + 1, 1)):
+        for k, most in ((8, 2600), (12, 1500), (24, 750)):
+            for count, launches in ((40 * sms, 1), (80 * sms - 8, 1), (80 * sms, 2), (min(most, 1600) * sms, 2),
+                                    (most * sms, 2), (most * sms + 1, 1)):
                 assert _check(c, oracle, k, rng, int(rng.integers(0, u - count)), count) == launches, count
         c30.build(x[:100_000], y[:100_000], z[:100_000])
         assert _check(c30, oracle, 16, rng) == 2
