@@ -38,7 +38,7 @@
 // written once; one loop climbs minimum and maximum levels alike. 200k points,
 // k = 16: 53.2 ms with one query per thread in lockstep over the eight child
 // numbers, 31.7 ms with the carried items and each thread's own next child,
-// 18.9 ms now; warp instructions 12.3 G -> 8.9 G -> 6.4 G.
+// 18.9 ms now (of 100k points: 3.6 G warp instructions, 8 of 32 threads in each).
 
 #include <cstdint>
 

@@ -26,10 +26,10 @@
 // Before, the lists held (distance, index) keys and took one insertion per
 // buffered candidate. Distances alone merge eight at a time through min/max
 // networks in half the registers, and nothing is gathered twice: 2M scene,
-// k = 16, ALU instructions 0.81 G -> 0.52 G, search 2.69 -> 2.29 ms; 20M
-// precision mix 18.0 -> 15.5 ms; 1M lists of 32 3.14 -> 2.05 ms. What holds it
-// now is latency: issue slots 54% busy, fixed-latency waits 2.4 per issue,
-// shared and global loads 0.9 each.
+// k = 16, search 2.69 -> 2.29 ms; 20M precision mix 18.0 -> 15.5 ms; 1M lists of
+// 32 3.14 -> 2.05 ms. What holds it now is latency and issue: of the 4M precision
+// mix 64% of the issue slots are busy, fixed-latency waits 2.6 per issue, waits
+// for global loads 1.35, for shared ones 0.9.
 
 #include <cfloat>
 #include <climits>
@@ -799,8 +799,7 @@ __device__ __forceinline__ float warp_max(float v) {
 // its own query and bound. The first test is one pass for 32 nodes where the
 // binary tree before it took a visit for every two (2M scene, k = 16: 43 tree
 // visits and 12 buckets of about 60 points per warp became 19 visits of 32
-// nodes and 21 leaves of about 20 points; warp instructions 2.10 G -> 1.71 G,
-// search 3.08 -> 2.69 ms; 20M precision mix 20.8 -> 18.0 ms, both with the
+// nodes and 21 leaves of about 20 points; search 3.08 -> 2.69 ms; 20M precision mix 20.8 -> 18.0 ms, both with the
 // earlier lists). The second keeps warps whose queries lie far apart (their
 // box covers what is between) from descending everywhere. Fetching the next
 // sibling's box one step ahead was slower (3.01 ms): its registers and moves

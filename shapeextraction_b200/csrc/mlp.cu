@@ -25,7 +25,7 @@ __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__floa
 // ---------------------------------------------------------------------------
 // Features of query qi (a tree point), all scale-free:
 //   0..11  log2(d2 to the Morton neighbours at +-1, 2, 4, 8, 16, 32) - log2(range^2), / 16
-//   12..27 for the leaf's first 8 ancestors in the search hierarchy (parent
+//   12..27 for the leaf's first 8 ancestors in the radix tree (parent
 //          first): log2(points under the node) / 21, then its code-prefix
 //          length / 63; past the root the root's values repeat. A node of s
 //          points with a p-bit prefix spans a cube of side range * 2^(-p/3),
