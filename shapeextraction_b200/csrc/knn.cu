@@ -1270,36 +1270,42 @@ __global__ void __launch_bounds__(BatchCfg<K, NW>::threads, BatchCfg<K, NW>::min
 }
 
 // Work items of the tree's own points [start, start + count): 32 at a time, cut
-// where the Morton order jumps and then into `per`. The jumps are the lowest common
-// prefixes of adjacent codes, `jump` bits below the median of the 32 or lower, three
-// at most. A warp across a jump walks two regions and what lies between, and a call
-// of a few rounds of warps ends with its slowest: normals of 110k points of a scene,
-// k = 8, lasted 249 us for one warp of 3438 (99 of 100 end within 120 us, half within
-// 66). Over scenes, cubes, mixtures and precision mixes, against none cut (6, 7, 8, 9,
-// 10 bits): 45k points, k = 8: 0.78, 0.82, 0.84, 0.88, 0.92; 110k, k = 16: 0.93, 0.90,
-// 0.88, 0.88, 0.89; k = 32: 0.98, 0.91, 0.89, 0.89, 0.89; 300k, k = 16: 1.10, 1.01,
-// 0.96, 0.94, 0.95; k = 32: 1.30, 1.14, 1.06, 1.01, 0.99.
+// where the Morton order jumps and then into `per`. A jump is a gap between adjacent
+// points of more than `jump` times the median gap of the 32; the three widest count.
+// A warp across a jump walks two regions and what lies between, and a call of a few
+// rounds of warps ends with its slowest: normals of 110k points of a scene, k = 8,
+// lasted 249 us for one warp of 3438 (99 of 100 end within 120 us, half within 66).
+// Over scenes, cubes, mixtures and precision mixes, against none cut (gaps of 5, 6, 8,
+// 10, 12, 16 medians): 45k points, k = 8: 0.77, 0.79, 0.84, 0.86, 0.87, 0.92; 110k, k =
+// 16: 0.92, 0.92, 0.82, 0.85, 0.87, 0.92; 300k, k = 16: 1.06, 1.01, 0.98, 0.95, 0.96,
+// 0.95. A plane or a line has few: 110k points, k = 16, 131 and 66 us uncut, 172 and 86
+// at 5, 134 and 72 at 10. (Judged by the codes' common prefixes, 8 bits below the
+// median, a line of 200k points was cut everywhere: 158 -> 306 us.)
 // Whole items fill the list from its front and parts, which end sooner, from its
 // back (room entries on), so that parts are what starts late when not all fit at
 // once.
 constexpr int kItemBytes = 2;  // of the list, per point: 4 + 32 / 8 - 1 parts of 8 bytes in 32 points
-__global__ void __launch_bounds__(256) k_point_items(const uint64_t* __restrict__ codes, int64_t start, int64_t n,
-                                                     int per, int jump, uint64_t* __restrict__ items, int64_t room,
+__global__ void __launch_bounds__(256) k_point_items(const float4* __restrict__ pts, int64_t start, int64_t n,
+                                                     int per, float jump, uint64_t* __restrict__ items, int64_t room,
                                                      DevState* st) {
     __shared__ uint32_t s_at[2][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const uint64_t code = i < n ? __ldg(codes + start + i) : 0ull;
-    const uint64_t before = __shfl_up_sync(FULL, code, 1);
-    const int shared = lane > 0 && i < n ? __clzll((long long)(code ^ before)) : 64;  // leading bits, 64: no pair
-    int median = 0;  // the most leading bits that 16 adjacent pairs share
+    const float4 p = __ldg(pts + start + min64(i, n - 1));
+    float gap = fmaxf(fmaxf(fabsf(p.x - __shfl_up_sync(FULL, p.x, 1)), fabsf(p.y - __shfl_up_sync(FULL, p.y, 1))),
+                      fabsf(p.z - __shfl_up_sync(FULL, p.z, 1)));
+    if (lane == 0 || i >= n) gap = 0.0f;
+    uint32_t median = 0;  // 16 gaps are at least this, to an eighth (0: fewer, or of equal points)
 #pragma unroll
-    for (int b = 32; b >= 1; b >>= 1)
-        if (__popc(__ballot_sync(FULL, shared >= median + b)) >= 17) median += b;
+    for (uint32_t b = 1u << 30; b >= 1u << 20; b >>= 1)
+        if (__popc(__ballot_sync(FULL, __float_as_uint(gap) >= (median | b))) >= 16) median |= b;
     uint32_t cuts = 0;
-    for (int at = median - jump; at >= 0; --at) {
-        cuts = __ballot_sync(FULL, shared <= at);
-        if (__popc(cuts) <= 3) break;
+    if (median > 0) {
+        float most = jump * __uint_as_float(median);
+        do {
+            cuts = __ballot_sync(FULL, gap > most);
+            most *= 2.0f;
+        } while (__popc(cuts) > 3);
     }
     cuts |= 1u;
     const int from = 31 - __clz(cuts & (2u * (1u << lane) - 1u));  // where the lane's part begins
@@ -1545,7 +1551,8 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
         uint64_t* items = reinterpret_cast<uint64_t*>(b.scratch);  // the build is done with it
         const int64_t room = q.count * kItemBytes / (int64_t)sizeof(uint64_t);
         k_point_items<<<(unsigned)((q.count + 255) / 256), 256, 0, s>>>(
-            b.codes, q.start, q.count, a.warp_queries, q.count <= (int64_t)1600 * num_sms ? 8 : 9, items, room, b.st);
+            b.pts4, q.start, q.count, a.warp_queries, q.count <= (int64_t)750 * num_sms ? 8.0f : 10.0f, items, room,
+            b.st);
         a.parts = items;
         a.parts_end = items + room;
     }

@@ -24,6 +24,8 @@ def _cloud(kind, n, rng):
     if kind == "line":
         t = rng.random(n)
         return np.stack([t, t, t])
+    if kind == "plane":
+        return np.stack([rng.random(n), rng.random(n), np.full(n, 0.5)])
     g = rng.integers(0, 70, (n, 3))  # equal distances, equal prefixes, equal points
     return g.T / 64.0
 
@@ -41,7 +43,7 @@ def _check(c, oracle, k, rng, start=0, count=None):
     return launches
 
 
-@pytest.mark.parametrize("kind", ["scene", "jumps", "line", "grid"])
+@pytest.mark.parametrize("kind", ["scene", "jumps", "line", "plane", "grid"])
 @pytest.mark.parametrize("k", [1, 8, 10, 16, 24, 32])
 def test_listed_searches_are_exact(native, oracle, kind, k):
     rng = np.random.default_rng(31)
@@ -65,6 +67,24 @@ def test_both_sides_of_the_rules(native, oracle):
                 assert _check(c, oracle, k, rng, int(rng.integers(0, u - count)), count) == launches, count
         c30.build(x[:100_000], y[:100_000], z[:100_000])
         assert _check(c30, oracle, 16, rng) == 2
+
+
+@pytest.mark.parametrize("kind,more", [("line", 1.5), ("plane", 1.5)])
+def test_few_cuts_without_jumps(native, kind, more):
+    """Along a line and on a plane most neighbours in the Morton order are
+    neighbours: the cuts add few node visits to those of whole warps. (Judged by
+    the codes alone a line is cut into four times as many parts.)"""
+    rng = np.random.default_rng(33)
+    most = 750 * _sms()  # points of a listed search with k > 16
+    with native.Context(build_octree=False) as c:
+        u = c.build(*(np.ascontiguousarray(v, np.float32) for v in _cloud(kind, most + 9_000, rng)))["n_points"]
+        assert u > most
+        nodes = []
+        for count, launches in ((most, 2), (most + 1, 1)):
+            c.knn_self(24, 0, count)
+            assert c.profile()["query_launches"] == launches
+            nodes.append(c.stats()["nodes_visited"])
+    assert nodes[0] < more * nodes[1], nodes
 
 
 def test_listed_searches_leave_the_tree_as_it_was(native):
