@@ -209,7 +209,7 @@ int run_query(se_ctx* c, int k, int64_t start, int64_t count, const float* ext, 
     // the tree. (250k queries near a 2M-point scene, k = 8, in random order: 21.0
     // ms as given, 0.66 ms in order.) Where the order's 24 bytes per query cannot
     // be had they are taken as given, one to a warp.
-    bool sorted = ext && !q.compat && order_foreign(count, k, c->num_sms);
+    bool sorted = ext && !q.compat && order_foreign(count, u, k, c->num_sms);
     if (sorted) {
         QueryOrder& o = c->q_order;
         const int64_t lookback = 3 * ((count + kSortTile - 1) / kSortTile) * kSortBins;

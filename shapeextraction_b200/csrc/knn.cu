@@ -1498,12 +1498,12 @@ bool list_points(int64_t count, int k, int num_sms) {
     return queries_per_warp(count, num_sms, false) >= 8 && count <= (int64_t)most * num_sms;
 }
 
-bool order_foreign(int64_t count, int k, int num_sms) {
+bool order_foreign(int64_t count, int64_t u, int k, int num_sms) {
     // The order takes about 60 us. Queries near a 2M-point scene, one to a warp as
     // given and in order, k = 1, 8, 16, 32: 20k of them 145, 220, 320, 694 us and
     // 200, 240, 317, 541 us; 30k 196, 294, 447, 978 and 211, 281, 377, 627; 40k
     // 249, 383, 580, 1297 and 233, 322, 441, 775.
-    return count >= (int64_t)(k <= 16 ? 180 : 120) * num_sms;
+    return u > kTinyTree && count >= (int64_t)(k <= 16 ? 180 : 120) * num_sms;
 }
 
 cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t s, int num_sms) {
@@ -1534,7 +1534,7 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
         a.items = q.items;
         // queries as given: close ones gain once there are more than warps fit;
         // a box of the tree's point spacing, were the points spread over its cube
-        a.close = q.count > 20 * num_sms ? 1.0f / cbrtf((float)q.u) : 0.0f;
+        a.close = q.count > 20 * num_sms && q.u > kTinyTree ? 1.0f / cbrtf((float)q.u) : 0.0f;
     } else {
         a.parts = nullptr;
         a.learned_r2 = q.learned_r2;
@@ -1545,7 +1545,8 @@ cudaError_t enqueue_query(const BuildBufs& b, const QueryParams& q, cudaStream_t
     }
     if (a.seed_halo > kMaxHalo) a.seed_halo = kMaxHalo;
     if (a.seed_halo < 0) a.seed_halo = 0;
-    a.warp_queries = q.ext_queries && !q.order ? 1 : queries_per_warp(q.count, num_sms, q.ext_queries != nullptr);
+    const bool foreign = q.ext_queries && q.u > kTinyTree;
+    a.warp_queries = foreign && !q.order ? 1 : queries_per_warp(q.count, num_sms, foreign);
     const bool ext = q.ext_queries != nullptr;
     if (!ext && !a.cell_lut && !q.device_count && list_points(q.count, q.k, num_sms)) {
         uint64_t* items = reinterpret_cast<uint64_t*>(b.scratch);  // the build is done with it

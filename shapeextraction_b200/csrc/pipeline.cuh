@@ -226,7 +226,12 @@ cudaError_t enqueue_query_order(const BuildBufs& b, const QueryOrder& o, const f
 // Queries per warp of a search of `count` queries, and whether foreign ones are
 // put in order (those that are not come one to a warp).
 int queries_per_warp(int64_t count, int num_sms, bool foreign);
-bool order_foreign(int64_t count, int k, int num_sms);
+bool order_foreign(int64_t count, int64_t u, int k, int num_sms);
+// Trees of at most this many points: foreign queries are taken as given, as many
+// to a warp as the tree's own points (every warp reads all of the tree anyway).
+// 100k queries, k = 1: of a tree of 5 points 103 us in order, 56 as given; of 100
+// points 118 and 64 us.
+constexpr int64_t kTinyTree = 256;
 // Whether a search of `count` of the tree's own points lists its work items
 // first (one more kernel; the list takes b.scratch). Not where other clouds fill
 // the GPU beside it (device_count).

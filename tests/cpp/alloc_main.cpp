@@ -59,7 +59,7 @@ cudaError_t enqueue_build(const BuildBufs& b, const BuildParams& p, cudaStream_t
     return cudaSuccess;
 }
 cudaError_t enqueue_octree(const BuildBufs&, const BuildParams&, cudaStream_t, int*) { return cudaSuccess; }
-bool order_foreign(int64_t count, int, int) { return count > 5000; }
+bool order_foreign(int64_t count, int64_t, int, int) { return count > 5000; }
 bool list_points(int64_t, int, int) { return false; }
 cudaError_t enqueue_query_order(const BuildBufs&, const QueryOrder& o, const float* q, int64_t n, int64_t, int,
                                 const uint64_t** order, const uint64_t** items, int* shift, cudaStream_t, int,

@@ -159,3 +159,30 @@ def test_queries_close_together_and_in_order(native, oracle, n, k):
             assert np.array_equal(d2[s[ok[s]]], ed), name
             assert np.array_equal(idx[s[ok[s]]], ei), name
             assert np.isnan(d2[~ok]).all() and idx.min() >= 0 and idx.max() < len(p), name
+
+
+@pytest.mark.parametrize("k", [1, 8, 31])
+def test_trees_of_few_points(native, oracle, k):
+    """Both sides of the size up to which queries share warps as given."""
+    with native.Context() as c:
+        for u in (1, 2, 7, 33, 100, 255, 256, 257):
+            p, rng = _tree(c, u, 10)
+            assert len(p) == u
+            for n in (1, 100, 5_000, 70_001):
+                q = (rng.random((n, 3)) * 3 - 1).astype(np.float32)
+                q[::17] = np.nan
+                q[5::17] = np.inf
+                idx, d2 = c.knn(q, k, with_d2=True)
+                ok = ~np.isnan(q).any(1)
+                ei, ed = oracle.knn_exact(p, q[ok], k, brute=True)
+                assert np.array_equal(d2[ok], ed) and np.array_equal(idx[ok], ei), (u, n)
+                assert np.isnan(d2[~ok]).all() and idx.min() >= 0 and idx.max() < u
+
+
+def test_trees_of_few_points_share_warps(native):
+    """100 points are four buckets, and two of 5000 queries or more share a warp
+    (one to a warp scanned 20,000 buckets)."""
+    with native.Context() as c:
+        _, rng = _tree(c, 100, 10)
+        c.knn(rng.random((5_000, 3)).astype(np.float32), 32)
+        assert 0 < c.stats()["buckets_scanned"] <= 2_500 * 4
